@@ -7,6 +7,7 @@
 #include <vector>
 #include <cublas_v2.h>
 #include <cusolverDn.h>
+#include "fx64.h"
 #include "handle.h"
 
 namespace cbx {
@@ -58,26 +59,14 @@ inline std::vector<T> d2h(cbx_handle* h, const T* d, size_t n) {
   return v;
 }
 
-// Cholesky of a column-major SPD matrix in place; returns false if not PD.
-inline bool potrf(cbx_handle* h, double* A, int64_t n) {
-  Libs& L = libs(h);
-  int lw = 0;
-  CBX_SOLVER(cusolverDnDpotrf_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, A, (int)n, &lw));
-  DevBuf<double> work;
-  work.resize(std::max(lw, 1));
-  DevBuf<int> info;
-  info.resize(1);
-  CBX_SOLVER(cusolverDnDpotrf(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, A, (int)n, work.p, lw, info.p));
-  int hi = 0;
-  CBX_CUDA(cudaMemcpyAsync(&hi, info.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  CBX_CUDA(cudaStreamSynchronize(h->stream));
-  return hi == 0;
-}
-inline void potrs(cbx_handle* h, const double* Lf, int64_t n, double* B, int64_t nrhs) {
+// Cholesky of a column-major SPD matrix (its lower triangle is read) in place: the
+// upper factor U = L', zeros below.  Returns false if not PD (A is then unchanged).
+inline bool potrf(cbx_handle* h, double* A, int64_t n) { return fx64_cholesky(h, A, n, false, A, nullptr); }
+inline void potrs(cbx_handle* h, const double* Uf, int64_t n, double* B, int64_t nrhs) {
   Libs& L = libs(h);
   DevBuf<int> info;
   info.resize(1);
-  CBX_SOLVER(cusolverDnDpotrs(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, (int)nrhs, Lf, (int)n, B, (int)n, info.p));
+  CBX_SOLVER(cusolverDnDpotrs(L.sol, CUBLAS_FILL_MODE_UPPER, (int)n, (int)nrhs, Uf, (int)n, B, (int)n, info.p));
 }
 // Eigen-bending inverse (invert_psd_matrix) and Cholesky inverse on the device.
 void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double ridge, double* out_dev);

@@ -1,0 +1,762 @@
+// FP64-accurate dense algebra on the tensor cores: C = A B', Cholesky factors and
+// SPD inverses, for the set-up (G^-1, A22^-1, H^-1) and the dense AI-REML steps
+// (reference: matrix_io.cpp:488-501, vce.cpp:2859-3195, relationship_builder.cpp:
+// 573-584).  GB300 runs FP64 at 1/64 of its FP32 rate (1.2 TFLOP/s), so these
+// were bound by cuSOLVER's FP64 GEMMs.
+//
+// Products.  Row i of an operand is scaled by 2^(61 - e_i), 2^e_i above its largest
+// magnitude, and rounded to an integer |F| < 2^61 (below 2^-62 of the row maximum, the
+// rounding of a double itself is 2^-54).  F is cut into eight balanced base-256
+// digits (-128 .. 127, exact in f16).  The 36 digit pairs with s + t <= 7 are multiplied
+// by kind::f16 MMAs; pairs of one weight s + t share an FP32 accumulator ("class"), whose
+// partial sums are integers of at most 8 * 128 * 2^14 = 2^24, hence exact, over chunks
+// of 128 K elements.  Each chunk is flushed into two int64 totals per output and the
+// product is rounded to FP64 once.  The dropped pairs weigh below 2^-58 of the product
+// of the two row maxima per term, less than an FP64 multiply-add's rounding.
+//
+// Factorization.  Right-looking in blocks of 32 inside outer panels of 128 to 512
+// columns, in a row-major lower triangle W.  Step k (k_panel) factors the 32 x 32
+// pivot block by FP64 elimination, giving X = L_kk^-1, and forms L_ik = S_ik X' for the
+// rows below; for the inverse also row k of M = L^-1, M_kj = X R_kj for j < k, where
+// R_ij = -sum_l L_il M_lj is kept in the slot of W that L_ij has left.  Digit MMAs then
+// apply S_ij -= L_ik L_jk' and R_ij -= L_ik M_kj, within the panel after each step
+// (K = 32) and to the rest once per panel (K = the panel's width).  A^-1 = M'M is one
+// triangular product at the end.
+//
+// Bound: below n = 3,000 the chain of 32-wide steps (a pivot factor and a K = 32 update,
+// about 60 us); above it the digit MMAs (36 per FP64 multiply-add, N <= 256 from shared
+// memory) and the FP64 conversions of their epilogue.  Measured, inverse with its
+// factor, against cuSOLVER potrf + potri: n = 500 0.98 ms (4.2), 2,000 4.0 (31), 8,000 38
+// (1,194), 20,000 337 (about 11,000).  The product at n = 2,000: 0.62 ms (15.3 by
+// cuBLAS DGEMM).  128 x 64 tiles: eight classes of 64 columns fill the 512 TMEM columns,
+// and a narrower tile would read the A digits from L2 faster than L2 delivers them.
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include "fx64.h"
+#include "tma.cuh"
+
+namespace cbx {
+namespace fx {
+
+constexpr int NPL = 8;                         // digit planes
+constexpr int PLANE_A = 128 * 32 * 2;          // one plane of a 128-row, 32-wide block
+constexpr int BLK = NPL * PLANE_A;             // 64 KB: one (row tile, K step) block
+constexpr int PLANE_B = 64 * 32 * 2;
+constexpr int STAGE = BLK + NPL * PLANE_B;     // 96 KB
+constexpr int NSTAGE = 2;
+constexpr int OFF_BAR = NSTAGE * STAGE;
+constexpr int SMEM = OFF_BAR + 256 + 1024;
+constexpr int THREADS = 320;
+constexpr int CHUNK = 4;                       // K steps per exact FP32 chunk
+constexpr int EX_MIN = -900, EX_BAD = 1 << 20; // exponent of a zero row; of a row with NaN / Inf
+constexpr unsigned long long BIAS = 0x8080808080808080ull;  // 128 in each digit byte
+static_assert(SMEM <= 232448, "shared memory budget");
+
+// canonical K-major no-swizzle offset of (row, k) in a 32-wide f16 plane
+__device__ __forceinline__ uint32_t cm_off(int r, int k) {
+  return (uint32_t)((r >> 3) * 512 + (r & 7) * 16 + (k >> 3) * 128 + (k & 7) * 2);
+}
+// digit byte j of two elements as an f16 pair: byte - 128, exact
+__device__ __forceinline__ uint32_t digit_pair(uint32_t ga, uint32_t gb, uint32_t j) {
+  const uint32_t u = __byte_perm(ga, gb, j | ((j + 4) << 4));
+  const uint32_t v = __byte_perm(u, 0x64646464u, 0x4140);  // f16 1024 + byte
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0xE480E480u));  // - 1152
+  return d;
+}
+__device__ __forceinline__ double pow2d(int n) { return __longlong_as_double((long long)(n + 1023) << 52); }
+// smallest e with |v| < 2^e (v finite, not zero), from the bits of |v|
+__device__ __forceinline__ int expo(double v) {
+  const int e = (int)((__double_as_longlong(v) >> 52) & 0x7FF);
+  return e == 0x7FF ? EX_BAD : max(EX_MIN, e - 1022);
+}
+// digit planes of eight consecutive K elements of one row
+__device__ __forceinline__ void put_digits(const double (&v)[8], int ex, uint8_t* blk, int row, int kg) {
+  const double sc = pow2d(61 - (ex == EX_BAD ? 0 : ex));
+  uint32_t lo[8], hi[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const unsigned long long G =
+        BIAS + (ex == EX_BAD ? 0ull : (unsigned long long)__double2ll_rn(v[e] * sc));
+    lo[e] = (uint32_t)G;
+    hi[e] = (uint32_t)(G >> 32);
+  }
+#pragma unroll
+  for (int pl = 0; pl < NPL; ++pl) {
+    const int j = 7 - pl;
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      w[e] = j < 4 ? digit_pair(lo[2 * e], lo[2 * e + 1], j) : digit_pair(hi[2 * e], hi[2 * e + 1], j - 4);
+    *reinterpret_cast<uint4*>(blk + pl * PLANE_A + cm_off(row, kg * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// ---- products --------------------------------------------------------------
+// Output tiles of 128 x 64.  A segment holds row tiles [ra, rb) with column tiles
+// [ca, cb), or [ca, 2 rt + 2) (the lower triangle) when tri.
+struct Seg {
+  int ra, rb, ca, cb, tri, cmin;
+  __host__ __device__ int count() const {
+    return rb <= ra ? 0 : tri ? (rb - ra) * (rb + ra + 1 - ca) : cb <= ca ? 0 : (rb - ra) * (cb - ca);
+  }
+};
+struct Job {
+  const uint8_t *A, *B;
+  const int32_t *ea, *eb;
+  int ka, kb;        // K steps per row tile in storage
+  int ks0, ks1;      // K steps summed
+  int ktri;          // storage and sum start at the row tile's own K step (4 rt)
+  Seg seg[2];
+  int tiles;
+  int mode;          // 0: C -= T; 1: C = T; 2: C = C' = T (lower triangle computed)
+  int rmin;          // rows below rmin, columns below the segment's cmin are left alone (mode 0)
+  int m, n;          // output bounds (modes 1, 2)
+  double* C;
+  int64_t ldc;
+};
+struct Bars {
+  uint64_t full[NSTAGE], empty[NSTAGE], acc_full, acc_empty, drain;
+  uint32_t tmem;
+  int abort;
+};
+
+__device__ __forceinline__ void tile_of(const Job& J, int t, int& rt, int& ct, int& cmin) {
+  const int c0 = J.seg[0].count();
+  const Seg& s = t < c0 ? J.seg[0] : J.seg[1];
+  if (t >= c0) t -= c0;
+  cmin = s.cmin;
+  if (s.tri) {
+    // f(x) = (x - ra)(x + ra + 1 - ca) <= t < f(x + 1)
+    const float b = 1.0f - s.ca;
+    int x = (int)(0.5f * (-b + sqrtf(b * b + 4.0f * ((float)t + (float)s.ra * (s.ra + 1 - s.ca)))));
+    x = max(s.ra, min(x, s.rb - 1));
+    while (x > s.ra && (x - s.ra) * (x + s.ra + 1 - s.ca) > t) --x;
+    while ((x + 1 - s.ra) * (x + s.ra + 2 - s.ca) <= t) ++x;
+    rt = x;
+    ct = s.ca + t - (x - s.ra) * (x + s.ra + 1 - s.ca);
+  } else {
+    const int w = s.cb - s.ca;
+    rt = s.ra + t / w;
+    ct = s.ca + t % w;
+  }
+}
+// first block of a row tile in a panel's storage (triangular panels keep K steps >= 4 rt)
+__device__ __forceinline__ size_t blk_of(int rt, int ks, int stride, int tri) {
+  return tri ? (size_t)rt * stride - 2 * (size_t)rt * (rt - 1) + (ks - 4 * rt) : (size_t)rt * stride + ks;
+}
+
+// Warp roles: 0 bulk loads, 1 TMEM owner and MMA issuer, 2-9 epilogue (two warps
+// per TMEM lane quadrant, 32 columns each).
+__global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job J, int* status) {
+  extern __shared__ uint8_t dsm_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
+  Bars* bars = reinterpret_cast<Bars*>(smem + OFF_BAR);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < NSTAGE; ++i) {
+      mbar_init(&bars->full[i], 1);
+      mbar_init(&bars->empty[i], 1);
+    }
+    mbar_init(&bars->acc_full, 1);
+    mbar_init(&bars->acc_empty, 8);
+    mbar_init(&bars->drain, 1);
+    bars->abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars->tmem, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = bars->tmem;
+  volatile int* abort_flag = &bars->abort;
+  auto fail = [&]() {
+    bars->abort = 1;
+    atomicExch(status, DEV_TIMEOUT);
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t g = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
+        int rt, ct, cmin;
+        tile_of(J, t, rt, ct, cmin);
+        for (int k = J.ktri ? 4 * rt : J.ks0; k < J.ks1; ++k, ++g) {
+          const uint32_t s = g % NSTAGE;
+          if (!mbar_wait(&bars->empty[s], ((g / NSTAGE) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(&bars->full[s], STAGE);
+          const uint32_t dst = smem_addr(smem + s * STAGE);
+          bulk_load(dst, J.A + blk_of(rt, k, J.ka, J.ktri) * BLK, BLK, &bars->full[s]);
+          const uint8_t* b = J.B + blk_of(ct >> 1, k, J.kb, J.ktri) * BLK + (ct & 1) * PLANE_B;
+#pragma unroll
+          for (int pl = 0; pl < NPL; ++pl)
+            bulk_load(dst + BLK + pl * PLANE_B, b + pl * PLANE_A, PLANE_B, &bars->full[s]);
+        }
+      }
+      if (!ok) fail();
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      uint32_t g = 0, c = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
+        int rt, ct, cmin;
+        tile_of(J, t, rt, ct, cmin);
+        const int k0 = J.ktri ? 4 * rt : J.ks0;
+        for (int k = k0; k < J.ks1; ++k, ++g) {
+          const int ci = (k - k0) % CHUNK;
+          if (ci == 0) {
+            if (!mbar_wait(&bars->acc_empty, (c & 1) ^ 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+          }
+          const uint32_t s = g % NSTAGE;
+          if (!mbar_wait(&bars->full[s], (g / NSTAGE) & 1, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t op = smem_addr(smem + s * STAGE);
+#pragma unroll
+          for (int kh = 0; kh < 2; ++kh) {
+            const uint32_t acc0 = (ci == 0 && kh == 0) ? 0u : 1u;
+            const uint32_t bb = op + BLK + kh * 256;
+#pragma unroll
+            for (int pl = 0; pl < NPL; ++pl) {
+              // digit plane pl of A against planes 0 .. 7 - pl of B: classes pl .. 7
+              const uint64_t dA = sdesc_noswizzle(op + pl * PLANE_A + kh * 256, 128, 512);
+              const int n1 = (NPL - pl) * 64;
+              umma_f16(tmem + pl * 64, dA, sdesc_noswizzle(bb, 128, 512), idesc_f16_f32(128, n1 > 256 ? 256 : n1),
+                       pl == 0 ? acc0 : 1u);
+              if (n1 > 256)
+                umma_f16(tmem + pl * 64 + 256, dA, sdesc_noswizzle(bb + 4 * PLANE_B, 128, 512),
+                         idesc_f16_f32(128, n1 - 256), pl == 0 ? acc0 : 1u);
+            }
+          }
+          umma_commit(&bars->empty[s]);
+          if (ci == CHUNK - 1 || k == J.ks1 - 1) {
+            umma_commit(&bars->acc_full);
+            ++c;
+          }
+        }
+      }
+      if (!ok) fail();
+      umma_commit(&bars->drain);
+      const uint64_t t0 = global_ns();
+      while (!mbar_try(&bars->drain, 0) && global_ns() - t0 < kWaitLimitNs) {}
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, j0 = ((warp - 2) >> 2) * 32;
+    uint32_t c = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
+      int rt, ct, cmin;
+      tile_of(J, t, rt, ct, cmin);
+      const int steps = J.ks1 - (J.ktri ? 4 * rt : J.ks0);
+      const int nch = (steps + CHUNK - 1) / CHUNK;
+      long long hi[32], lo[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
+      for (int ch = 0; ch < nch; ++ch, ++c) {
+        if (!mbar_wait_idle(&bars->acc_full, c & 1, abort_flag, 20)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + j0;
+#pragma unroll
+        for (int ci = 0; ci < NPL; ++ci) {
+          const int mul = 1 << ((3 - (ci & 3)) * 8);
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t r[16];
+            tmem_ld16(ta + ci * 64 + hh * 16, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const long long v = (long long)__float2int_rn(__uint_as_float(r[j])) * mul;
+              if (ci < 4) hi[hh * 16 + j] += v;
+              else lo[hh * 16 + j] += v;
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->acc_empty);
+      }
+      if (!ok) break;
+      const int row = rt * 128 + q * 32 + lane, col0 = ct * 64 + j0;
+      const int ea = J.ea[row] - 66;  // 56 - 2 * 61
+      auto val = [&](int j) -> double {
+        const int n = ea + J.eb[col0 + j];
+        const double x = fma((double)hi[j], 0x1p32, (double)lo[j]);
+        if (n > -1000 && n < 900) return x * pow2d(n);
+        return n > EX_BAD / 2 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(x, n);
+      };
+      if (J.mode == 0) {
+        if (row >= J.rmin && col0 + 31 >= cmin) {
+          double* p = J.C + (int64_t)row * J.ldc + col0;
+          if (col0 >= cmin) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              double2 o = *reinterpret_cast<double2*>(p + j);
+              o.x -= val(j);
+              o.y -= val(j + 1);
+              *reinterpret_cast<double2*>(p + j) = o;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (col0 + j >= cmin) p[j] -= val(j);
+          }
+        }
+      } else {
+        if (row < J.m) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int cc = col0 + j;
+            if (cc < J.n && (J.mode == 1 || cc <= row)) {
+              const double x = val(j);
+              J.C[(int64_t)row * J.ldc + cc] = x;
+              if (J.mode == 2) J.C[(int64_t)cc * J.ldc + row] = x;
+            }
+          }
+        }
+      }
+    }
+    if (!ok) fail();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// ---- digits of a matrix ------------------------------------------------------
+// ex[r]: exponent of the largest magnitude of row r (rows past `rows` are zero).
+// One warp per row; trans: one thread per row, K over blockDim.y.
+__global__ void __launch_bounds__(256) k_rowexp(const double* __restrict__ src, int64_t ld, int64_t rows, int64_t k,
+                                                int32_t* __restrict__ ex) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  int e = EX_MIN;
+  if (r < rows)
+    for (int64_t j = threadIdx.x & 31; j < k; j += 32) {
+      const double v = src[r * ld + j];
+      if (v != 0.0) e = max(e, expo(v));
+    }
+  for (int o = 16; o; o >>= 1) e = max(e, __shfl_xor_sync(~0u, e, o));
+  if ((threadIdx.x & 31) == 0) ex[r] = e;
+}
+__global__ void __launch_bounds__(256) k_rowexp_t(const double* __restrict__ src, int64_t ld, int64_t rows, int64_t k,
+                                                  int32_t* __restrict__ ex) {
+  __shared__ int red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t r = (int64_t)blockIdx.x * 32 + lane;
+  int e = EX_MIN;
+  if (r < rows)
+    for (int64_t j = w; j < k; j += 8) {
+      const double v = src[j * ld + r];
+      if (v != 0.0) e = max(e, expo(v));
+    }
+  red[w][lane] = e;
+  __syncthreads();
+  if (w == 0) {
+    for (int i = 1; i < 8; ++i) e = max(e, red[i][lane]);
+    ex[r] = e;
+  }
+}
+// blocks (row tile, K step): thread = row, 8 K elements at a time
+__global__ void __launch_bounds__(128) k_digits(const double* __restrict__ src, int64_t ld, int64_t rows, int64_t k,
+                                                int trans, int ks, const int32_t* __restrict__ ex,
+                                                uint8_t* __restrict__ dig) {
+  const int64_t r = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int64_t k0 = (int64_t)blockIdx.y * 32;
+  uint8_t* blk = dig + ((size_t)blockIdx.x * ks + blockIdx.y) * BLK;
+  const int e = ex[r];
+#pragma unroll
+  for (int kg = 0; kg < 4; ++kg) {
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int64_t kk = k0 + kg * 8 + i;
+      v[i] = (r < rows && kk < k) ? (trans ? src[kk * ld + r] : src[r * ld + kk]) : 0.0;
+    }
+    put_digits(v, e, blk, threadIdx.x, kg);
+  }
+}
+
+// ---- Cholesky ------------------------------------------------------------------
+// W (np x np row-major) = lower triangle of A (column-major), identity on the padding
+__global__ void __launch_bounds__(256) k_load_lower(const double* __restrict__ A, int64_t n, int64_t np,
+                                                    double* __restrict__ W) {
+  __shared__ double t[32][33];
+  const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
+  if (j0 > i0) return;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int c = y; c < 32; c += 8) {
+    const int64_t i = i0 + x, j = j0 + c;
+    t[c][x] = (i < n && j < n) ? A[j * n + i] : (i == j ? 1.0 : 0.0);
+  }
+  __syncthreads();
+  for (int r = y; r < 32; r += 8) W[(i0 + r) * np + j0 + x] = t[x][r];
+}
+
+struct Panel {
+  double* W;
+  int64_t np;
+  int k0, K0, K1, B;
+  int inverse;
+  uint8_t* dig;       // inner digits (K = 32)
+  int32_t* ex;        // their exponents
+  int32_t* exo;       // exponents of the outer panel's rows, so far
+  int32_t* exm;       // exponents of the columns of M, so far
+  double* P;          // L of the outer panel (np x B)
+  double* D;          // diagonal blocks of M (or L), np x 32: other CTAs still read the pivot block in W
+  double* piv;
+  int* bad;
+};
+
+// One 32-wide step.  Every CTA factors the pivot block (it is small, and a separate
+// launch would cost more than the repeat), then takes 32-row groups: out = v X' with v
+// the row's 32 entries in the pivot columns (rows below the pivot), the column's
+// entries in the pivot rows (columns left of it), or a unit vector (the pivot rows).
+// FP64 issue bounds both parts.
+__global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) {
+  __shared__ double X[32][33], V[32][33], Lm[32][33], prow[2][32], pv[32];
+  __shared__ int mx[4][32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t np = a.np;
+  double* Wk = a.W + (int64_t)a.k0 * np + a.k0;
+  // lane = column, registers = rows w + 4 t
+  double d[8];
+  for (int r = w; r < 32; r += 4) V[r][lane] = lane <= r ? Wk[r * np + lane] : 0.0;
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int r = w + 4 * t;
+    d[t] = lane <= r ? V[r][lane] : V[lane][r];
+  }
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    for (int ww = 0; ww < 4; ++ww) {
+      const int k = 4 * kk + ww, b = k & 1;
+      if (w == ww) {
+        const double p = __shfl_sync(~0u, d[kk], k);
+        const double inv = 1.0 / p;
+        prow[b][lane] = lane == k ? inv : d[kk] * inv;
+        if (lane == k) {
+          pv[k] = p;
+          d[kk] = 1.0;
+        }
+      }
+      __syncthreads();
+      const double qv = prow[b][lane];
+#pragma unroll
+      for (int t = kk; t < 8; ++t) {
+        if (t > kk || w > ww) {
+          const double f = __shfl_sync(~0u, d[t], k);
+          if (lane == k) Lm[w + 4 * t][k] = f;
+          d[t] = fma(-f, qv, lane == k ? 0.0 : d[t]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int r = w + 4 * t;
+    X[r][lane] = lane <= r ? d[t] / sqrt(pv[r]) : 0.0;
+  }
+  if (blockIdx.x == 0 && tid < 32) {
+    const double p = pv[tid];
+    a.piv[a.k0 + tid] = p;
+    if (!(p > 0.0) || !isfinite(p)) atomicExch(a.bad, 1);
+  }
+  __syncthreads();
+  const int gk = a.k0 / 32, ng = (int)(np / 32), g0 = a.inverse ? 0 : gk;
+  for (int g = g0 + blockIdx.x; g < ng; g += gridDim.x) {
+    const int r0 = g * 32, r = r0 + lane;
+    // V[l][row]
+    if (g > gk) {
+      for (int i = w; i < 32; i += 4) V[lane][i] = a.W[(int64_t)(r0 + i) * np + a.k0 + lane];
+    } else if (g < gk) {
+      for (int l = w; l < 32; l += 4) V[l][lane] = a.W[(int64_t)(a.k0 + l) * np + r];
+    } else {
+      for (int l = w; l < 32; l += 4) V[l][lane] = l == lane ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    double acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.0;
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+      const double v = V[l][lane];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (l <= 4 * j + 3) acc[j] = fma(v, X[w + 4 * j][l], acc[j]);
+    }
+    __syncthreads();
+    int e = EX_MIN;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      V[w + 4 * j][lane] = acc[j];
+      if (acc[j] != 0.0) e = max(e, expo(acc[j]));
+    }
+    mx[w][lane] = e;
+    __syncthreads();
+    e = max(max(mx[0][lane], mx[1][lane]), max(mx[2][lane], mx[3][lane]));
+    if (w == 0) {
+      a.ex[r] = e;
+      a.exo[r] = (a.k0 == a.K0 || g == gk) ? e : max(e, a.exo[r]);
+      if (a.inverse && g <= gk) a.exm[r] = g == gk ? e : max(e, a.exm[r]);
+    }
+    double v8[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v8[i] = V[w * 8 + i][lane];
+    put_digits(v8, e, a.dig + (size_t)(r0 / 128) * BLK, r & 127, w);
+    if (g > gk) {
+      for (int i = w; i < 32; i += 4) {
+        const double l = V[lane][i];
+        a.P[(int64_t)(r0 + i) * a.B + (a.k0 - a.K0) + lane] = l;
+        a.W[(int64_t)(r0 + i) * np + a.k0 + lane] = a.inverse ? 0.0 : l;
+      }
+    } else if (g < gk) {
+      for (int l = w; l < 32; l += 4) a.W[(int64_t)(a.k0 + l) * np + r] = V[l][lane];
+    } else {
+      for (int l = w; l < 32; l += 4) {
+        const double x = a.inverse ? X[l][lane] : lane < l ? Lm[l][lane] / sqrt(pv[lane]) : sqrt(pv[l]);
+        a.D[(a.k0 + l) * 32 + lane] = lane <= l ? x : 0.0;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// element (i, j), i >= j, of the finished triangle
+__device__ __forceinline__ double lower(const double* W, const double* D, int64_t np, int64_t i, int64_t j) {
+  return (i >> 5) == (j >> 5) ? D[i * 32 + (j & 31)] : W[i * np + j];
+}
+
+// Digits of the outer panel: rows below it from P, columns left of its end (rows of
+// M') from W.  Blocks (row tile, K step of the panel).
+__global__ void __launch_bounds__(128) k_panel_digits(const __grid_constant__ Panel a, uint8_t* __restrict__ dig,
+                                                      int rt0) {
+  const int rt = rt0 + blockIdx.x, r = rt * 128 + threadIdx.x, kb = blockIdx.y * 32;
+  uint8_t* blk = dig + ((size_t)rt * (a.B / 32) + blockIdx.y) * BLK;
+  const int e = a.exo[r];
+#pragma unroll
+  for (int kg = 0; kg < 4; ++kg) {
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = kb + kg * 8 + i;
+      if (r >= a.K1) v[i] = a.K0 + k < a.K1 ? a.P[(int64_t)r * a.B + k] : 0.0;
+      else v[i] = a.K0 + k < r ? 0.0 : lower(a.W, a.D, a.np, a.K0 + k, r);
+    }
+    put_digits(v, e, blk, threadIdx.x, kg);
+  }
+}
+// Digits of M' (row j = column j of M = L^-1, K steps from the row tile's own on)
+__global__ void __launch_bounds__(128) k_minv_digits(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int n, int ks,
+                                                     const int32_t* __restrict__ ex, uint8_t* __restrict__ dig) {
+  const int rt = blockIdx.x, k0 = blockIdx.y;
+  if (k0 < 4 * rt) return;
+  const int r = rt * 128 + threadIdx.x;
+  uint8_t* blk = dig + blk_of(rt, k0, ks, 1) * BLK;
+  const int e = r < n ? ex[r] : EX_MIN;
+#pragma unroll
+  for (int kg = 0; kg < 4; ++kg) {
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 * 32 + kg * 8 + i;
+      v[i] = (k >= r && k < n && r < n) ? lower(W, D, np, k, r) : 0.0;
+    }
+    put_digits(v, e, blk, threadIdx.x, kg);
+  }
+}
+// sum of log pivots, in a fixed order
+__global__ void __launch_bounds__(256) k_logsum(const double* __restrict__ piv, int n, double* __restrict__ out) {
+  __shared__ double red[256];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 256) s += log(piv[i]);
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[0] = red[0];
+}
+// U = L' (column-major upper = row-major lower), zeros elsewhere
+__global__ void k_store_factor(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int64_t n, double* __restrict__ out) {
+  const int64_t total = n * n;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / n, c = i % n;
+    out[i] = c <= r ? lower(W, D, np, r, c) : 0.0;
+  }
+}
+
+// Scratch of the factorizations, kept by the handle between calls of up to
+// kKeepBytes (a GBLUP of a few thousand animals); larger ones are freed on return,
+// where an allocation costs little beside the work.
+constexpr size_t kKeepBytes = (size_t)1 << 30;
+struct Scratch {
+  DevBuf<double> W, P, D, piv;
+  DevBuf<uint8_t> din, dout, dm;
+  DevBuf<int32_t> ex, exo, exm;
+  DevBuf<int> bad;
+  size_t bytes() const { return W.n * 8 + P.n * 8 + din.n + dout.n + dm.n; }
+};
+template <typename T>
+static void at_least(DevBuf<T>& b, size_t n) {
+  if (b.n < n) b.resize(n);
+}
+static Scratch& scratch(cbx_handle* h) {
+  if (!h->fx_slot) h->fx_slot = std::make_shared<Scratch>();
+  return *static_cast<Scratch*>(h->fx_slot.get());
+}
+
+static void launch(cbx_handle* h, Job& J) {
+  J.tiles = J.seg[0].count() + J.seg[1].count();
+  if (J.tiles <= 0 || J.ks1 <= 0) return;
+  ensure_smem((const void*)k_fx64, SMEM, h->device);
+  k_fx64<<<std::min(J.tiles, h->num_sms), THREADS, SMEM, h->stream>>>(J, h->status.p);
+  h->launched("k_fx64");
+}
+
+}  // namespace fx
+
+void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans) {
+  CBX_REQUIRE(rows > 0 && k > 0 && rows < (1 << 24) && k < (1 << 24), CBX_ERR_ARG, "bad operand shape");
+  P.rt = (int)((rows + 127) / 128);
+  P.ks = (int)((k + 31) / 32);
+  fx::at_least(P.dig, (size_t)P.rt * P.ks * fx::BLK);
+  fx::at_least(P.ex, (size_t)P.rt * 128);
+  cudaStream_t s = h->stream;
+  if (trans) fx::k_rowexp_t<<<P.rt * 4, 256, 0, s>>>(src, ld, rows, k, P.ex.p);
+  else fx::k_rowexp<<<P.rt * 16, 256, 0, s>>>(src, ld, rows, k, P.ex.p);
+  h->launched("k_rowexp");
+  for (int y = 0; y < P.ks; y += 65535) {  // grid.y limit
+    const int cnt = std::min(65535, P.ks - y);
+    fx::k_digits<<<dim3(P.rt, cnt), 128, 0, s>>>(src + (trans ? (int64_t)y * 32 * ld : (int64_t)y * 32), ld, rows,
+                                                 k - (int64_t)y * 32, trans, P.ks, P.ex.p,
+                                                 P.dig.p + (size_t)y * fx::BLK);
+    h->launched("k_digits");
+  }
+}
+
+void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int64_t n, double* C, int64_t ldc) {
+  CBX_REQUIRE(A.ks == B.ks && m <= (int64_t)A.rt * 128 && n <= (int64_t)B.rt * 128, CBX_ERR_ARG, "operand shapes differ");
+  fx::Job J{};
+  J.A = A.dig.p;
+  J.B = B.dig.p;
+  J.ea = A.ex.p;
+  J.eb = B.ex.p;
+  J.ka = J.kb = J.ks1 = A.ks;
+  J.seg[0] = {0, A.rt, 0, (int)((n + 63) / 64), 0, 0};
+  J.mode = 1;
+  J.m = (int)m;
+  J.n = (int)n;
+  J.C = C;
+  J.ldc = ldc;
+  fx::launch(h, J);
+}
+
+bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet) {
+  CBX_REQUIRE(n > 0 && n <= 130000, CBX_ERR_ARG, "matrix order out of range");
+  cudaStream_t s = h->stream;
+  fx::Scratch& S = fx::scratch(h);
+  const int64_t np = (n + 127) / 128 * 128;
+  const int rt = (int)(np / 128), B0 = n < 3000 ? 128 : n < 10000 ? 256 : 512;
+  const int B = (int)std::min<int64_t>(B0, np);
+  fx::at_least(S.W, (size_t)np * np);
+  fx::at_least(S.P, (size_t)np * B);
+  fx::at_least(S.D, (size_t)np * 32);
+  fx::at_least(S.piv, (size_t)np + 1);
+  fx::at_least(S.din, (size_t)rt * fx::BLK);
+  fx::at_least(S.dout, (size_t)rt * (B / 32) * fx::BLK);
+  fx::at_least(S.ex, (size_t)np);
+  fx::at_least(S.exo, (size_t)np);
+  fx::at_least(S.exm, (size_t)np);
+  fx::at_least(S.bad, 1);
+  CBX_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), s));
+  fx::k_load_lower<<<dim3((unsigned)(np / 32), (unsigned)(np / 32)), 256, 0, s>>>(A, n, np, S.W.p);
+  h->launched("k_load_lower");
+  fx::Panel a{S.W.p, np, 0, 0, 0, B, inverse ? 1 : 0, S.din.p, S.ex.p, S.exo.p, S.exm.p, S.P.p, S.D.p, S.piv.p,
+              S.bad.p};
+  fx::Job J{};
+  J.C = S.W.p;
+  J.ldc = np;
+  for (int64_t K0 = 0; K0 < n; K0 += B) {
+    a.K0 = (int)K0;
+    a.K1 = (int)std::min<int64_t>(K0 + B, np);
+    const int tp = a.K1 / 128;
+    for (int k0 = a.K0; k0 < a.K1 && k0 < n; k0 += 32) {
+      a.k0 = k0;
+      const int groups = (int)(np / 32) - (inverse ? 0 : k0 / 32);
+      fx::k_panel<<<std::min(groups, h->num_sms), 128, 0, s>>>(a);
+      h->launched("k_panel");
+      const int next = k0 + 32;
+      if (next >= a.K1 || next >= n) continue;
+      // within the panel: its remaining columns below, and its remaining rows of R
+      J.A = J.B = S.din.p;
+      J.ea = J.eb = S.ex.p;
+      J.ka = J.kb = J.ks1 = 1;
+      J.rmin = next;
+      J.seg[0] = {next / 128, tp, inverse ? 0 : next / 64, 0, 1, inverse ? 0 : next};
+      J.seg[1] = {tp, rt, next / 64, 2 * tp, 0, next};
+      fx::launch(h, J);
+    }
+    if (a.K1 >= n) break;
+    const int first = inverse ? 0 : tp;
+    fx::k_panel_digits<<<dim3(rt - first, B / 32), 128, 0, s>>>(a, S.dout.p, first);
+    h->launched("k_panel_digits");
+    J.A = J.B = S.dout.p;
+    J.ea = J.eb = S.exo.p;
+    J.ka = J.kb = J.ks1 = B / 32;
+    J.rmin = a.K1;
+    J.seg[0] = {tp, rt, inverse ? 0 : 2 * tp, 0, 1, 0};
+    J.seg[1] = {0, 0, 0, 0, 0, 0};
+    fx::launch(h, J);
+  }
+  double ld = 0.0;
+  int bad = 0;
+  if (logdet) {
+    fx::k_logsum<<<1, 256, 0, s>>>(S.piv.p, (int)n, S.piv.p + np);
+    h->launched("k_logsum");
+    CBX_CUDA(cudaMemcpyAsync(&ld, S.piv.p + np, sizeof(double), cudaMemcpyDeviceToHost, s));
+  }
+  CBX_CUDA(cudaMemcpyAsync(&bad, S.bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CBX_CUDA(cudaStreamSynchronize(s));
+  h->check_status("FP64 factorization");
+  if (!bad && inverse) {
+    const int ks = (int)(np / 32);
+    fx::at_least(S.dm, ((size_t)rt * ks - 2 * (size_t)rt * (rt - 1)) * fx::BLK);
+    fx::k_minv_digits<<<dim3(rt, ks), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, S.exm.p, S.dm.p);
+    h->launched("k_minv_digits");
+    fx::Job M{};
+    M.A = M.B = S.dm.p;
+    M.ea = M.eb = S.exm.p;
+    M.ka = M.kb = M.ks1 = ks;
+    M.ktri = 1;
+    M.seg[0] = {0, rt, 0, 0, 1, 0};
+    M.mode = 2;
+    M.m = M.n = (int)n;
+    M.C = out;
+    M.ldc = n;
+    fx::launch(h, M);
+  } else if (!bad && out) {
+    fx::k_store_factor<<<(unsigned)std::min<int64_t>((n * n + 255) / 256, 8 * h->num_sms), 256, 0, s>>>(S.W.p, S.D.p, np, n,
+                                                                                                      out);
+    h->launched("k_store_factor");
+  }
+  if (logdet) *logdet = ld;
+  if (S.bytes() > fx::kKeepBytes) {
+    CBX_CUDA(cudaStreamSynchronize(s));
+    h->fx_slot.reset();
+  }
+  return bad == 0;
+}
+
+}  // namespace cbx

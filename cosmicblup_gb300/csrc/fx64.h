@@ -1,0 +1,30 @@
+// FP64-accurate dense algebra on the tensor cores by exact fixed-point digits
+// (fx64.cu): products, Cholesky factors and SPD inverses of the set-up and
+// dense-AI paths.
+#pragma once
+#include <cstdint>
+#include "handle.h"
+
+namespace cbx {
+
+// Digits of an operand: rows (padded to 128) x k (padded to 32), 16 bytes an entry.
+struct FxPanel {
+  DevBuf<uint8_t> dig;
+  DevBuf<int32_t> ex;
+  int rt = 0, ks = 0;  // row tiles of 128, K steps of 32
+};
+
+// Rows of P from src: element (r, k) is src[r * ld + k], or src[k * ld + r] when
+// trans.
+void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans);
+// C[i * ldc + j] = sum_k A(i, k) B(j, k) for i < m, j < n.
+void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int64_t n, double* C, int64_t ldc);
+
+// Cholesky of the symmetric n x n matrix A (column-major, its lower triangle is
+// read).  Returns false when a pivot is not positive.  logdet (may be null) gets
+// log det A.  With inverse, out (may be A) receives the full symmetric A^-1;
+// otherwise, when out is given, out gets the factor U = L' (column-major upper
+// triangle, zeros below).
+bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet);
+
+}  // namespace cbx

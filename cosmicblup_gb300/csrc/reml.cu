@@ -88,60 +88,6 @@ __global__ void k_build_P_ci(int64_t n_rec, int64_t p, int64_t q, int64_t dim, c
     P[idx] = ((i == j ? 1.0 : 0.0) - hsum) / ve;
   }
 }
-// C = A B for n x n column-major FP64 matrices: 64 x 64 output tiles per
-// block, 4 x 4 per thread, K in steps of 16 staged in shared memory; every
-// output sums its K terms in index order.  FP64 multiply-add issue bounds it
-// (GB300 runs FP64 at 1/64 of the FP32 rate).
-__global__ void __launch_bounds__(256) k_dgemm_nn(int64_t n, const double* __restrict__ A,
-                                                  const double* __restrict__ B, double* __restrict__ C) {
-  __shared__ double As[16][65];
-  __shared__ double Bs[16][65];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t row0 = (int64_t)blockIdx.x * 64, col0 = (int64_t)blockIdx.y * 64;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (int64_t k0 = 0; k0 < n; k0 += 16) {
-    for (int t = threadIdx.x; t < 1024; t += 256) {
-      const int r = t & 63, kk = t >> 6;
-      As[kk][r] = (row0 + r < n && k0 + kk < n) ? A[(k0 + kk) * n + row0 + r] : 0.0;
-      const int kb = t & 15, c = t >> 4;
-      Bs[kb][c] = (col0 + c < n && k0 + kb < n) ? B[(col0 + c) * n + k0 + kb] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t r = row0 + ty * 4 + i, c = col0 + tx * 4 + j;
-      if (r < n && c < n) C[c * n + r] = acc[i][j];
-    }
-}
-// y = A x for an n x n column-major FP64 matrix (one thread per row, K in order)
-__global__ void k_dgemv_n(int64_t n, const double* __restrict__ A, const double* __restrict__ x,
-                          double* __restrict__ y) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (int64_t k = 0; k < n; ++k) t = fma(A[k * n + r], x[k], t);
-    y[r] = t;
-  }
-}
 // ZAZt[i, j] = A[aid_i - 1, aid_j - 1] (0 for records without an animal)
 __global__ void k_build_zazt(int64_t n_rec, int64_t q, const int32_t* __restrict__ aid, const double* __restrict__ A,
                              double* __restrict__ Z) {
@@ -151,15 +97,6 @@ __global__ void k_build_zazt(int64_t n_rec, int64_t q, const int32_t* __restrict
     const int64_t i = idx % n_rec, j = idx / n_rec;
     const int32_t a = aid[i], b = aid[j];
     Z[idx] = (a > 0 && a <= q && b > 0 && b <= q) ? A[(int64_t)(b - 1) * q + (a - 1)] : 0.0;
-  }
-}
-// fill the strict upper triangle from the lower one (column-major)
-__global__ void k_symmetrize_lower(double* __restrict__ A, int64_t n) {
-  const int64_t total = n * n;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx % n, c = idx / n;
-    if (r < c) A[idx] = A[r * n + c];
   }
 }
 // partial sums of: sum M_ij M_ji, sum M_ij P_ij, sum P_ij^2, tr M, tr P
@@ -845,7 +782,22 @@ struct DenseExact {
   bool init = false;
   int64_t n = 0, dim = 0;
   DevBuf<double> ZAZt;
+  FxPanel Vdig, Pdig;
+  // kept between steps up to order kKeepDense (0.5 GB each), where allocating them costs
+  // as much as the step: LHS, its inverse, P, P V
+  DevBuf<double> C, Ci, P, Mu;
   double log_det_A = 0;
+  static constexpr int64_t kKeepDense = 8192;
+  struct Trim {
+    DenseExact& d;
+    ~Trim() {
+      if (d.n <= kKeepDense && d.dim <= kKeepDense) return;
+      d.C.release();
+      d.Ci.release();
+      d.P.release();
+      d.Mu.release();
+    }
+  };
 };
 static DenseExact& dense_state(cbx_handle* h) {
   if (!h->dense_slot) h->dense_slot = std::make_shared<DenseExact>();
@@ -863,31 +815,21 @@ static void dense_init(cbx_handle* h, DenseExact& D) {
   A.resize((size_t)q * q);
   CBX_CUDA(cudaMemcpy2DAsync(A.p, q * sizeof(double), m.Qd64.p, m.ld * sizeof(double), q * sizeof(double), q,
                              cudaMemcpyDeviceToDevice, s));
-  CBX_REQUIRE(potrf(h, A.p, q), CBX_ERR_FACTOR, "Qinv is not positive definite");
-  D.log_det_A = -2.0 * log_diag(h, A.p, q);
-  {
-    Libs& L = libs(h);
-    int lw = 0;
-    CBX_SOLVER(cusolverDnDpotri_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)q, A.p, (int)q, &lw));
-    DevBuf<double> work;
-    work.resize(std::max(lw, 1));
-    DevBuf<int> info;
-    info.resize(1);
-    CBX_SOLVER(cusolverDnDpotri(L.sol, CUBLAS_FILL_MODE_LOWER, (int)q, A.p, (int)q, work.p, lw, info.p));
-    k_symmetrize_lower<<<gridn(q * q, 256, 8 * h->num_sms), 256, 0, s>>>(A.p, q);
-    h->launched("k_symmetrize_lower");
-  }
+  CBX_REQUIRE(fx64_cholesky(h, A.p, q, true, A.p, &D.log_det_A), CBX_ERR_FACTOR, "Qinv is not positive definite");
+  D.log_det_A = -D.log_det_A;
   D.ZAZt.resize((size_t)n * n);
   k_build_zazt<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(n, q, m.aid.p, A.p, D.ZAZt.p);
   h->launched("k_build_zazt");
+  // V = Z A Z' is the second factor of every step's product P V: its digits are kept
+  fx64_digits(h, D.Vdig, D.ZAZt.p, n, n, n, false);
   CBX_CUDA(cudaStreamSynchronize(s));
   D.n = n;
   D.dim = dim;
   D.init = true;
 }
 
-// Factor C(lambda) in C (dim x dim); returns false if not PD.
-static bool factor_lhs(cbx_handle* h, double lam, DevBuf<double>& C) {
+// C(lambda) in C (dim x dim)
+static void build_lhs(cbx_handle* h, double lam, DevBuf<double>& C) {
   Mme& m = *h->mme;
   cudaStream_t s = h->stream;
   const int64_t dim = m.dim;
@@ -897,26 +839,63 @@ static bool factor_lhs(cbx_handle* h, double lam, DevBuf<double>& C) {
   h->launched("k_build_lhs");
   k_scatter_csr<<<gridn(dim, 256, 4 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, C.p);
   h->launched("k_scatter_csr");
-  return potrf(h, C.p, dim);
+}
+// y = A x (+ y0 when given, minus A x when neg) for a symmetric n x n matrix: one warp
+// per row, 32 partial sums in a fixed order.  Bound by the read of A (HBM, or L2 below
+// n = 4,000).
+__global__ void __launch_bounds__(256) k_symv(int64_t n, const double* __restrict__ A, const double* __restrict__ x,
+                                              const double* __restrict__ y0, int neg, double* __restrict__ y) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= n) return;
+  const double* a = A + r * n;
+  double t[4] = {0.0, 0.0, 0.0, 0.0};
+  int64_t k = threadIdx.x & 31;
+  for (; k + 96 < n; k += 128)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) t[u] = fma(a[k + 32 * u], x[k + 32 * u], t[u]);
+  for (; k < n; k += 32) t[0] = fma(a[k], x[k], t[0]);
+  double v = (t[0] + t[1]) + (t[2] + t[3]);
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+  if ((threadIdx.x & 31) == 0) y[r] = (y0 ? y0[r] : 0.0) + (neg ? -v : v);
+}
+static void symv(cbx_handle* h, const double* A, int64_t n, const double* x, const double* y0, bool neg, double* y) {
+  k_symv<<<(unsigned)((n + 7) / 8), 256, 0, h->stream>>>(n, A, x, y0, neg ? 1 : 0, y);
+  h->launched("k_symv");
+}
+// sol = C^-1 b from the explicit inverse, with one step of refinement on C (the
+// residual removes the product's error, which the condition of C amplifies)
+static void solve_by_inverse(cbx_handle* h, const double* C, const double* Ci, int64_t n, const double* b,
+                             DevBuf<double>& sol) {
+  DevBuf<double> r;
+  r.resize(n);
+  sol.resize(n);
+  symv(h, Ci, n, b, nullptr, false, sol.p);
+  symv(h, C, n, sol.p, b, true, r.p);
+  symv(h, Ci, n, r.p, sol.p, false, sol.p);
 }
 
-// compute_logL of run_dense_exact_step (vce.cpp:2974-3007); -1e18 if C is not PD
-static double dense_logL(cbx_handle* h, DenseExact& D, double vu, double ve, DevBuf<double>& C, DevBuf<double>& sol,
-                         double* ld_out = nullptr) {
+// compute_logL of run_dense_exact_step (vce.cpp:2974-3007); -1e18 if C is not PD.  D.C
+// keeps the LHS (its factor when inverse is false), D.Ci its inverse.
+static double dense_logL(cbx_handle* h, DenseExact& D, double vu, double ve, bool inverse, DevBuf<double>& sol) {
   Mme& m = *h->mme;
   const int64_t n = m.n_rec, p = m.p, q = m.q, dim = m.dim;
-  if (!factor_lhs(h, ve / vu, C)) return -1e18;
-  const double ld_C = 2.0 * log_diag(h, C.p, dim);
+  build_lhs(h, ve / vu, D.C);
+  if (inverse) D.Ci.resize((size_t)dim * dim);
+  double ld_C = 0.0;
+  if (!fx64_cholesky(h, D.C.p, dim, inverse, inverse ? D.Ci.p : D.C.p, &ld_C)) return -1e18;
   if (!std::isfinite(ld_C)) return -1e18;
-  sol.resize(dim);
-  CBX_CUDA(cudaMemcpyAsync(sol.p, m.rhs.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  potrs(h, C.p, dim, sol.p, 1);
+  if (inverse) {
+    solve_by_inverse(h, D.C.p, D.Ci.p, dim, m.rhs.p, sol);
+  } else {
+    sol.resize(dim);
+    CBX_CUDA(cudaMemcpyAsync(sol.p, m.rhs.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    potrs(h, D.C.p, dim, sol.p, 1);
+  }
   DevBuf<double> e;
   e.resize(n);
   record_residual(h, sol.p, e.p);
   const auto eh = d2h(h, e.p, n);
   const double yPy = dot_h(m.y_host, eh) / ve;
-  if (ld_out) *ld_out = ld_C;
   const double m2 = ld_C + (double)(n - p - q) * std::log(ve) + (double)q * std::log(vu) + yPy + D.log_det_A;
   return -0.5 * m2;
 }
@@ -956,34 +935,20 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   Libs& L = libs(h);
   const int64_t n = m.n_rec, dim = m.dim;
   const double vu = vu_io, ve = ve_io;
-  DevBuf<double> C, sol;
-  const double cur0 = dense_logL(h, D, vu, ve, C, sol);
+  DenseExact::Trim trim{D};
+  DevBuf<double> sol;
+  const double cur0 = dense_logL(h, D, vu, ve, true, sol);
   if (cur0 <= -1e18) return false;
   double cur = cur0;
-  // P = (I - W C^-1 W^T) / ve from the explicit C^-1 (inverse of the factor),
-  // then M_u = P ZAZ^T: the FP64 products on this library's kernels
-  DevBuf<double> Ci;
-  Ci.resize((size_t)dim * dim);
-  CBX_CUDA(cudaMemcpyAsync(Ci.p, C.p, (size_t)dim * dim * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  {
-    int lw = 0;
-    CBX_SOLVER(cusolverDnDpotri_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)dim, Ci.p, (int)dim, &lw));
-    DevBuf<double> work;
-    work.resize(std::max(lw, 1));
-    DevBuf<int> info;
-    info.resize(1);
-    CBX_SOLVER(cusolverDnDpotri(L.sol, CUBLAS_FILL_MODE_LOWER, (int)dim, Ci.p, (int)dim, work.p, lw, info.p));
-    k_symmetrize_lower<<<gridn(dim * dim, 256, 8 * h->num_sms), 256, 0, s>>>(Ci.p, dim);
-    h->launched("k_symmetrize_lower");
-  }
-  DevBuf<double> P, Mu;
+  // P = (I - W C^-1 W^T) / ve from the explicit C^-1, then M_u = P ZAZ^T by digits
+  DevBuf<double>&P = D.P, &Mu = D.Mu;
   P.resize((size_t)n * n);
   Mu.resize((size_t)n * n);
   k_build_P_ci<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(n, m.p, m.q, dim, m.aid.p, m.x_ptr.p, m.x_col.p,
-                                                                  m.x_val.p, Ci.p, ve, P.p);
+                                                                  m.x_val.p, D.Ci.p, ve, P.p);
   h->launched("k_build_P_ci");
-  k_dgemm_nn<<<dim3((unsigned)((n + 63) / 64), (unsigned)((n + 63) / 64)), 256, 0, s>>>(n, P.p, D.ZAZt.p, Mu.p);
-  h->launched("k_dgemm_nn");
+  fx64_digits(h, D.Pdig, P.p, n, n, n, false);
+  fx64_gemm(h, D.Pdig, D.Vdig, n, n, Mu.p, n);
   const unsigned g = gridn(n * n, 256, 4 * h->num_sms);
   DevBuf<double> part;
   part.resize((size_t)g * 5);
@@ -1003,8 +968,7 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   DevBuf<double> dPy;
   dPy.resize(n);
   CBX_CUDA(cudaMemcpyAsync(dPy.p, Py.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
-  k_dgemv_n<<<gridn(n, 256, 4 * h->num_sms), 256, 0, s>>>(n, D.ZAZt.p, dPy.p, ZPy.p);
-  h->launched("k_dgemv_n");
+  symv(h, D.ZAZt.p, n, dPy.p, nullptr, false, ZPy.p);
   const auto ZPyh = d2h(h, ZPy.p, n);
   const double score_u = dot_h(Py, ZPyh), score_e = dot_h(Py, Py);
   const double grad_u = -0.5 * sums[3] + 0.5 * score_u;
@@ -1034,8 +998,8 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   for (int k = 0; k < max_halving; ++k) {
     const double vu_n = vu + delta[0], ve_n = ve + delta[1];
     if (vu_n > 0 && ve_n > 0) {
-      DevBuf<double> C2, s2;
-      const double nl = dense_logL(h, D, vu_n, ve_n, C2, s2);
+      DevBuf<double> s2;
+      const double nl = dense_logL(h, D, vu_n, ve_n, false, s2);
       if (nl > cur || k == max_halving - 1) {
         cur = nl;
         vu_io = vu_n;
@@ -1467,14 +1431,14 @@ __global__ void k_add_lowrank(double* __restrict__ A, int64_t n, const double* _
 // eps = max(1e-12 lambda_max, 1e-6) to eps and returns U diag(1 / lambda) U^T.
 // The same matrix is formed without the full eigendecomposition:
 //  * lambda_max <= ||M||_inf, so eps = 1e-6 whenever 1e-12 ||M||_inf <= 1e-6;
-//  * if M - eps I has a Cholesky factor, no eigenvalue is raised and the result
-//    is M^-1 (Cholesky inverse);
+//  * if every eigenvalue is above eps (M^-1 bounds them from below, or M - eps I has a
+//    Cholesky factor) none is raised and the result is M^-1 (Cholesky inverse);
 //  * otherwise only the eigenpairs below eps are computed (syevdx), M is raised
 //    to M + sum (eps - lambda_i) u_i u_i^T, whose eigenvalues are all >= eps,
 //    and that is inverted by Cholesky.
 //  * when the all-ones direction is (nearly) null -- every VanRaden G, whose
-//    centred columns sum to zero -- the one eigenpair below eps is found by
-//    inverse iteration instead (deflate_ones below), without syevdx.
+//    centred columns sum to zero -- the one eigenpair below eps and the inverse off it
+//    come from one inverse of M plus a rank-1 term (deflate_ones below).
 // The full eigendecomposition (syevd, scaled columns, GEMM) remains for the
 // other cases.  The four forms are the same matrix in exact arithmetic.
 static int env_int_reml(const char* name, int def) {
@@ -1524,56 +1488,89 @@ static void invert_psd_full(cbx_handle* h, const double* M_dev, int64_t n, doubl
                        &zero, out_dev, (int)n));
 }
 
+// R = N - u w' - w u' + g u u' + beta a a'
+__global__ void k_deflated(const double* __restrict__ N, int64_t n, const double* __restrict__ u,
+                           const double* __restrict__ w, double uw, double g, double beta, double* __restrict__ R) {
+  const int64_t total = n * n;
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = idx % n, c = idx / n;
+    const double ur = u[r], uc = u[c], wr = w[r], wc = w[c];
+    // the two rank-1 terms are added first and a a' is symmetric, so R is too
+    R[idx] = (N[idx] - (ur * wc + wr * uc)) + (g * (ur * uc) + beta * ((wr - uw * ur) * (wc - uw * uc)));
+  }
+}
+
 // One eigenvalue of Mr (M + ridge I, in out_dev) below eps, along a direction
-// close to v = 1/sqrt(n) (v'Mr v < eps):
-//  1. u from eight steps of inverse iteration with the Cholesky factor of
-//     Mr + eps I (each step shrinks the other eigenvectors' share by
-//     (lambda_1 + eps) / (lambda_i + eps));
-//  2. check: Mr + c u u^T - 100 eps I (c = ||Mr||_inf + 1) has a Cholesky factor,
-//     so every eigenvalue off u is above 100 eps and u is the only one raised;
-//     the gap also bounds u's error after step 1 by (0.1 * 2 / 101)^8;
-//  3. Mr + (eps - u'Mr u) u u^T, the raised matrix, inverted by Cholesky.
-// Returns false, with out_dev untouched, when step 1 or 2 fails.
-static bool deflate_ones(cbx_handle* h, const double* M_dev, int64_t n, double ridge, double eps, double rinf,
-                         double* out_dev) {
+// close to v = 1/sqrt(n) (v'Mr v < eps), from one inverse N = (Mr + c v v')^-1:
+//  1. check: every eigenvalue of Mr + c v v' is above 100 eps -- 1 / ||N||_inf is a
+//     lower bound of them, and where that is too low a Cholesky factor of
+//     Mr + c v v' - 100 eps I decides.  A rank-1 term moves no eigenvalue past the next,
+//     so Mr's second smallest is above 100 eps too, and the smallest is the only one
+//     raised;
+//  2. its eigenvector u from (Mr + c v v') u = rho u + c (v'u) v: each step
+//     u <- N (rho u + c (v'u) v) shrinks the error by rho / lambda_2 < 1e-2;
+//  3. with P = I - u u', w = N u, a = P w: P N P + rho / (1 - rho u'w) a a' is the inverse
+//     of Mr on the complement of u, and u u' / eps is added.
+// Returns false, with out_dev untouched, when step 1 or 2 fails.  N's condition is that of
+// Mr off its null direction, so the result keeps the digits that inverting the raised
+// matrix (condition 1e6 and more) would lose.
+static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double* out_dev) {
   cudaStream_t s = h->stream;
   Libs& L = libs(h);
   const int ni = (int)n;
-  DevBuf<double> T, u, y, w;
+  const unsigned grid = gridn(n * n, 256, 8 * h->num_sms);
+  DevBuf<double> T, N, u, v, y, w1;
   T.resize((size_t)n * n);
+  N.resize((size_t)n * n);
   u.resize(n);
+  v.resize(n);
   y.resize(n);
-  w.resize(1);
-  k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, eps, T.p);
-  h->launched("k_add_ridge_copy");
-  if (!potrf(h, T.p, n)) return false;
+  w1.resize(1);
   std::vector<double> x(n, 1.0 / std::sqrt((double)n));
-  CBX_CUDA(cudaMemcpyAsync(u.p, x.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
+  CBX_CUDA(cudaMemcpyAsync(v.p, x.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
+  CBX_CUDA(cudaMemcpyAsync(w1.p, &c, sizeof(double), cudaMemcpyHostToDevice, s));
+  CBX_CUDA(cudaMemcpyAsync(T.p, out_dev, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  k_add_lowrank<<<grid, 256, 0, s>>>(T.p, n, v.p, w1.p, 1);
+  h->launched("k_add_lowrank");
+  if (!fx64_cholesky(h, T.p, n, true, N.p, nullptr)) return false;
+  double ninf = 0.0;
+  k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(N.p, n, y.p);
+  h->launched("k_col_abs_sum");
+  for (double t : d2h(h, y.p, n)) ninf = std::isfinite(t) ? std::max(ninf, t) : HUGE_VAL;
+  if (!(ninf < 0.99 / (100.0 * eps))) {
+    k_add_ridge_copy<<<grid, 256, 0, s>>>(T.p, n, -100.0 * eps, T.p);
+    h->launched("k_add_ridge_copy");
+    if (!fx64_cholesky(h, T.p, n, false, nullptr, nullptr)) return false;
+  }
+  auto dot = [&](const double* a, const double* b) {
+    double t = 0.0;
+    CBX_BLAS(cublasDdot(L.blas, ni, a, 1, b, 1, &t));
+    return t;
+  };
+  // u <- N v normalised (exact when rho = 0), then the steps of 2.
+  CBX_CUDA(cudaMemcpyAsync(u.p, v.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  double rho = 0.0;
   for (int it = 0; it < 8; ++it) {
-    potrs(h, T.p, n, u.p, 1);
-    double nrm = 0.0;
-    CBX_BLAS(cublasDnrm2(L.blas, ni, u.p, 1, &nrm));
+    const double vu = dot(v.p, u.p) * c;
+    CBX_BLAS(cublasDscal(L.blas, ni, &rho, u.p, 1));
+    CBX_BLAS(cublasDaxpy(L.blas, ni, &vu, v.p, 1, u.p, 1));
+    symv(h, N.p, n, u.p, nullptr, false, y.p);
+    const double nrm = std::sqrt(dot(y.p, y.p));
     if (!(nrm > 0.0) || !std::isfinite(nrm)) return false;
     const double sc = 1.0 / nrm;
-    CBX_BLAS(cublasDscal(L.blas, ni, &sc, u.p, 1));
+    CBX_BLAS(cublasDscal(L.blas, ni, &sc, y.p, 1));
+    std::swap(u.p, y.p);
+    symv(h, out_dev, n, u.p, nullptr, false, y.p);
+    rho = dot(u.p, y.p);
+    if (std::abs(rho) < 1e-12 && it > 0) break;  // the next step would move u by less than 1e-8 of its error
   }
-  const double one = 1.0, zero = 0.0;
-  CBX_BLAS(cublasDgemv(L.blas, CUBLAS_OP_N, ni, ni, &one, out_dev, ni, u.p, 1, &zero, y.p, 1));
-  double rho = 0.0;
-  CBX_BLAS(cublasDdot(L.blas, ni, u.p, 1, y.p, 1, &rho));
   if (!(rho < eps)) return false;
-  const double c = rinf + 1.0;
-  k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, -100.0 * eps, T.p);
-  h->launched("k_add_ridge_copy");
-  CBX_CUDA(cudaMemcpyAsync(w.p, &c, sizeof(double), cudaMemcpyHostToDevice, s));
-  k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(T.p, n, u.p, w.p, 1);
-  h->launched("k_add_lowrank");
-  if (!potrf(h, T.p, n)) return false;
-  const double raise = eps - rho;
-  CBX_CUDA(cudaMemcpyAsync(w.p, &raise, sizeof(double), cudaMemcpyHostToDevice, s));
-  k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, u.p, w.p, 1);
-  h->launched("k_add_lowrank");
-  if (!chol_inverse_device(h, out_dev, n)) invert_psd_full(h, M_dev, n, ridge, out_dev);
+  symv(h, N.p, n, u.p, nullptr, false, y.p);
+  const double uw = dot(u.p, y.p), beta = rho / (1.0 - rho * uw);
+  k_deflated<<<grid, 256, 0, s>>>(N.p, n, u.p, y.p, uw, uw + 1.0 / eps, beta, out_dev);
+  h->launched("k_deflated");
+  CBX_CUDA(cudaStreamSynchronize(s));  // N and T go out of scope
   return true;
 }
 
@@ -1609,17 +1606,32 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
     CBX_BLAS(cublasDgemv(L.blas, CUBLAS_OP_N, ni, ni, &one, out_dev, ni, v.p, 1, &zero, y.p, 1));
     double rho0 = 0.0;
     CBX_BLAS(cublasDdot(L.blas, ni, v.p, 1, y.p, 1, &rho0));
-    if (rho0 < eps && deflate_ones(h, M_dev, n, ridge, eps, rinf, out_dev)) return;
+    if (rho0 < eps && deflate_ones(h, n, eps, rinf > 0.0 ? rinf : 1.0, out_dev)) return;
   }
   DevBuf<double> T;
   T.resize((size_t)n * n);
-  // no eigenvalue below eps: M - eps I is positive definite
-  k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, -eps, T.p);
-  h->launched("k_add_ridge_copy");
-  if (potrf(h, T.p, n)) {
-    if (chol_inverse_device(h, out_dev, n)) return;
-    invert_psd_full(h, M_dev, n, ridge, out_dev);
-    return;
+  // no eigenvalue below eps: 1 / ||M^-1||_inf, a lower bound of a positive definite M's
+  // eigenvalues, is above it, or M - eps I is positive definite
+  if (fx64_cholesky(h, out_dev, n, true, T.p, nullptr)) {
+    DevBuf<double> cs;
+    cs.resize(n);
+    k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(T.p, n, cs.p);
+    h->launched("k_col_abs_sum");
+    double ninf = 0.0;
+    for (double v : d2h(h, cs.p, n)) ninf = std::isfinite(v) ? std::max(ninf, v) : HUGE_VAL;
+    bool all_above = ninf < 0.99 / eps;
+    if (!all_above) {
+      DevBuf<double> U;
+      U.resize((size_t)n * n);
+      k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, -eps, U.p);
+      h->launched("k_add_ridge_copy");
+      all_above = fx64_cholesky(h, U.p, n, false, nullptr, nullptr);
+    }
+    if (all_above) {
+      CBX_CUDA(cudaMemcpyAsync(out_dev, T.p, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      CBX_CUDA(cudaStreamSynchronize(s));  // T goes out of scope
+      return;
+    }
   }
   // the eigenpairs below eps: lambda in (-||M||_inf - 1, eps)
   Libs& L = libs(h);
@@ -1656,21 +1668,8 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
   if (!chol_inverse_device(h, out_dev, n)) invert_psd_full(h, M_dev, n, ridge, out_dev);
 }
 
-// In-place inverse of an SPD device matrix by Cholesky; false if not PD.
-bool chol_inverse_device(cbx_handle* h, double* A, int64_t n) {
-  if (!potrf(h, A, n)) return false;
-  Libs& L = libs(h);
-  int lw = 0;
-  CBX_SOLVER(cusolverDnDpotri_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, A, (int)n, &lw));
-  DevBuf<double> work;
-  work.resize(std::max(lw, 1));
-  DevBuf<int> info;
-  info.resize(1);
-  CBX_SOLVER(cusolverDnDpotri(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, A, (int)n, work.p, lw, info.p));
-  k_symmetrize_lower<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, h->stream>>>(A, n);
-  h->launched("k_symmetrize_lower");
-  return true;
-}
+// In-place inverse of an SPD device matrix by Cholesky; false if not PD (A unchanged).
+bool chol_inverse_device(cbx_handle* h, double* A, int64_t n) { return fx64_cholesky(h, A, n, true, A, nullptr); }
 
 }  // namespace cbx
 
@@ -1695,8 +1694,9 @@ extern "C" int cbx_reml_logl_dense(cbx_handle* h, double var_u, double var_e, do
     if (m.has_dense && !m.has_sparse && m.ng == m.q) {
       cbx::DenseExact& D = cbx::dense_state(h);
       if (!D.init || D.n != m.n_rec || D.dim != m.dim) cbx::dense_init(h, D);
-      cbx::DevBuf<double> C, sol;
-      *logL = cbx::dense_logL(h, D, var_u, var_e, C, sol);
+      cbx::DenseExact::Trim trim{D};
+      cbx::DevBuf<double> sol;
+      *logL = cbx::dense_logL(h, D, var_u, var_e, false, sol);
     } else {
       // a split Qinv: calc_logL_internal, without the constant log|A|
       CBX_REQUIRE(m.dim <= cbx::kAiDenseMax, CBX_ERR_UNSUPPORTED, "LHS too large for a dense factorization");
@@ -1732,20 +1732,16 @@ extern "C" int cbx_final_solve(cbx_handle* h, double var_u, double var_e, int32_
     x.resize(dim);
     std::vector<double> Ci((size_t)p * p, 0.0);
     if (dense) {
-      cbx::DevBuf<double> C;
-      CBX_REQUIRE(cbx::factor_lhs(h, lam, C), CBX_ERR_FACTOR, "Direct Solver Decomposition Failed");
-      CBX_CUDA(cudaMemcpyAsync(x.p, m.rhs.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      cbx::potrs(h, C.p, dim, x.p, 1);
+      cbx::DevBuf<double> C, Cinv;
+      cbx::build_lhs(h, lam, C);
+      Cinv.resize((size_t)dim * dim);
+      CBX_REQUIRE(cbx::fx64_cholesky(h, C.p, dim, true, Cinv.p, nullptr), CBX_ERR_FACTOR,
+                  "Direct Solver Decomposition Failed");
+      cbx::solve_by_inverse(h, C.p, Cinv.p, dim, m.rhs.p, x);
       if (calc_se && p > 0) {
-        std::vector<double> E((size_t)dim * p, 0.0);
-        for (int64_t i = 0; i < p; ++i) E[(size_t)i * dim + i] = 1.0;
-        cbx::DevBuf<double> Ed;
-        Ed.resize(E.size());
-        CBX_CUDA(cudaMemcpyAsync(Ed.p, E.data(), E.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        cbx::potrs(h, C.p, dim, Ed.p, p);
-        std::vector<double> Eh = cbx::d2h(h, Ed.p, E.size());
-        for (int64_t i = 0; i < p; ++i)
-          for (int64_t j = 0; j < p; ++j) Ci[(size_t)i * p + j] = Eh[(size_t)i * dim + j];
+        CBX_CUDA(cudaMemcpy2DAsync(Ci.data(), p * sizeof(double), Cinv.p, dim * sizeof(double), p * sizeof(double), p,
+                                   cudaMemcpyDeviceToHost, s));
+        CBX_CUDA(cudaStreamSynchronize(s));
       }
     } else {
       const bool abs_mode = solver == 2;

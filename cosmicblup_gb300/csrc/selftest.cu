@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <vector>
 #include "dense_tc.h"
+#include "fx64.h"
 #include "handle.h"
 #include "solver.cuh"
 
@@ -316,6 +317,70 @@ extern "C" int cbx_selftest_dense_fx(cbx_handle* h, const double* Q, int64_t ng,
       h->check_status("cbx_selftest_dense_fx");
     }
     CBX_CUDA(cudaMemcpyAsync(Y, dY.p, (size_t)ng * S * 8, cudaMemcpyDeviceToHost, h->stream));
+    CBX_CUDA(cudaStreamSynchronize(h->stream));
+  });
+}
+
+// Mean device time of `reps` runs of fn on the handle's stream (ms).
+template <typename F>
+static double time_runs(cbx_handle* h, int reps, F&& fn) {
+  cudaEvent_t a, b;
+  CBX_CUDA(cudaEventCreate(&a));
+  CBX_CUDA(cudaEventCreate(&b));
+  CBX_CUDA(cudaEventRecord(a, h->stream));
+  for (int i = 0; i < reps; ++i) fn();
+  CBX_CUDA(cudaEventRecord(b, h->stream));
+  CBX_CUDA(cudaEventSynchronize(b));
+  float ms = 0;
+  CBX_CUDA(cudaEventElapsedTime(&ms, a, b));
+  cudaEventDestroy(a);
+  cudaEventDestroy(b);
+  return ms / reps;
+}
+
+// C (m x n, row-major) = A B' by exact digits: A m x k row-major, B n x k row-major,
+// or k x n when trans_b.  reps > 0 times the product (digits included).
+extern "C" int cbx_selftest_fx64_gemm(cbx_handle* h, const double* A, const double* B, int64_t m, int64_t n, int64_t k,
+                                      int32_t trans_b, int32_t reps, double* Cout, double* ms_out) {
+  return cbx_guard(h, [&] {
+    CBX_REQUIRE(m > 0 && n > 0 && k > 0, CBX_ERR_ARG, "bad shape");
+    CBX_CUDA(cudaSetDevice(h->device));
+    cbx::DevBuf<double> dA, dB, dC;
+    dA.resize((size_t)m * k);
+    dB.resize((size_t)n * k);
+    dC.resize((size_t)m * n);
+    CBX_CUDA(cudaMemcpyAsync(dA.p, A, (size_t)m * k * 8, cudaMemcpyHostToDevice, h->stream));
+    CBX_CUDA(cudaMemcpyAsync(dB.p, B, (size_t)n * k * 8, cudaMemcpyHostToDevice, h->stream));
+    cbx::FxPanel pa, pb;
+    auto run = [&] {
+      cbx::fx64_digits(h, pa, dA.p, k, m, k, false);
+      cbx::fx64_digits(h, pb, dB.p, trans_b ? n : k, n, k, trans_b != 0);
+      cbx::fx64_gemm(h, pa, pb, m, n, dC.p, n);
+    };
+    run();
+    h->check_status("cbx_selftest_fx64_gemm");
+    if (reps > 0 && ms_out) *ms_out = time_runs(h, reps, run);
+    CBX_CUDA(cudaMemcpyAsync(Cout, dC.p, (size_t)m * n * 8, cudaMemcpyDeviceToHost, h->stream));
+    CBX_CUDA(cudaStreamSynchronize(h->stream));
+  });
+}
+
+// The digit Cholesky of a symmetric n x n matrix: out = A^-1 (inverse != 0) or the
+// column-major upper factor; *ok = 0 when a pivot is not positive (out untouched).
+extern "C" int cbx_selftest_fx64_chol(cbx_handle* h, const double* A, int64_t n, int32_t inverse, int32_t reps,
+                                      double* out, double* logdet, int32_t* ok, double* ms_out) {
+  return cbx_guard(h, [&] {
+    CBX_REQUIRE(n > 0, CBX_ERR_ARG, "bad shape");
+    CBX_CUDA(cudaSetDevice(h->device));
+    cbx::DevBuf<double> dA, dO;
+    dA.resize((size_t)n * n);
+    dO.resize((size_t)n * n);
+    CBX_CUDA(cudaMemcpyAsync(dA.p, A, (size_t)n * n * 8, cudaMemcpyHostToDevice, h->stream));
+    auto run = [&] { return cbx::fx64_cholesky(h, dA.p, n, inverse != 0, dO.p, logdet); };
+    *ok = run() ? 1 : 0;
+    h->check_status("cbx_selftest_fx64_chol");
+    if (reps > 0 && ms_out) *ms_out = time_runs(h, reps, [&] { (void)run(); });
+    if (*ok) CBX_CUDA(cudaMemcpyAsync(out, dO.p, (size_t)n * n * 8, cudaMemcpyDeviceToHost, h->stream));
     CBX_CUDA(cudaStreamSynchronize(h->stream));
   });
 }
