@@ -24,12 +24,12 @@
 // triangular product at the end.
 //
 // Bound: below n = 3,000 the chain of 32-wide steps (a pivot factor and a K = 32 update,
-// about 60 us); above it the digit MMAs (36 per FP64 multiply-add, N <= 256 from shared
-// memory) and the FP64 conversions of their epilogue.  Measured, inverse with its
-// factor, against cuSOLVER potrf + potri: n = 500 0.98 ms (4.2), 2,000 4.0 (31), 8,000 38
-// (1,194), 20,000 337 (about 11,000).  The product at n = 2,000: 0.62 ms (15.3 by
-// cuBLAS DGEMM).  128 x 64 tiles: eight classes of 64 columns fill the 512 TMEM columns,
-// and a narrower tile would read the A digits from L2 faster than L2 delivers them.
+// 26 us); above it the digit MMAs (36 per FP64 multiply-add) and the L2 reads that feed
+// them (96 KB a step of 2,304 tensor clocks).  Measured, inverse with its factor, against
+// cuSOLVER potrf + potri: n = 500 0.63 ms (4.2), 2,000 2.8 (31), 8,000 34 (1,194), 20,000
+// 322 (about 11,000).  The product at n = 2,000: 0.60 ms (15.3 by cuBLAS DGEMM).  128 x 64
+// tiles: eight classes of 64 columns fill the 512 TMEM columns, and a narrower tile reads
+// the A digits more often.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -42,16 +42,20 @@ namespace fx {
 constexpr int NPL = 8;                         // digit planes
 constexpr int PLANE_A = 128 * 32 * 2;          // one plane of a 128-row, 32-wide block
 constexpr int BLK = NPL * PLANE_A;             // 64 KB: one (row tile, K step) block
-constexpr int PLANE_B = 64 * 32 * 2;
-constexpr int STAGE = BLK + NPL * PLANE_B;     // 96 KB
 constexpr int NSTAGE = 2;
-constexpr int OFF_BAR = NSTAGE * STAGE;
-constexpr int SMEM = OFF_BAR + 256 + 1024;
-constexpr int THREADS = 320;
+// Output tiles are 128 x NT, NT = 64 or 32: eight classes of NT TMEM columns.
+template <int NT> struct Tile {
+  static constexpr int PLANE_B = NT * 32 * 2;
+  static constexpr int STAGE = BLK + NPL * PLANE_B;  // 96 or 80 KB
+  static constexpr int EW = NT / 4;                  // epilogue warps: 16 columns of a TMEM lane quadrant each
+  static constexpr int THREADS = 128 + 32 * EW;
+  static constexpr int OFF_OUT = NSTAGE * STAGE;     // 2 KB per epilogue warp
+  static constexpr int OFF_BAR = OFF_OUT + EW * 2048;
+  static constexpr int SMEM = OFF_BAR + 256 + 1024;
+  };
 constexpr int CHUNK = 4;                       // K steps per exact FP32 chunk
 constexpr int EX_MIN = -900, EX_BAD = 1 << 20; // exponent of a zero row; of a row with NaN / Inf
 constexpr unsigned long long BIAS = 0x8080808080808080ull;  // 128 in each digit byte
-static_assert(SMEM <= 232448, "shared memory budget");
 
 // canonical K-major no-swizzle offset of (row, k) in a 32-wide f16 plane
 __device__ __forceinline__ uint32_t cm_off(int r, int k) {
@@ -71,6 +75,50 @@ __device__ __forceinline__ int expo(double v) {
   const int e = (int)((__double_as_longlong(v) >> 52) & 0x7FF);
   return e == 0x7FF ? EX_BAD : max(EX_MIN, e - 1022);
 }
+// (hi 2^32 + lo) 2^n, rounded to nearest, for -900 < n < 900, in about 30 integer
+// instructions without a branch: on GB300 each FP64 instruction or int64 conversion of a
+// warp holds its quarter of the SM's FP64 pipe for 64 clocks.
+__host__ __device__ __forceinline__ unsigned long long from_totals(long long hi, long long lo, int n) {
+  const long long h = hi + (lo >> 32);
+  const uint32_t m = (uint32_t)(h >> 63);
+  const unsigned long long l = (unsigned long long)((uint32_t)lo ^ m) + (m & 1u);
+  const unsigned long long t = ((unsigned long long)h ^ ((unsigned long long)m << 32 | m)) + (l >> 32);
+  uint32_t w2 = (uint32_t)(t >> 32), w1 = (uint32_t)t, w0 = (uint32_t)l;  // |x| in 96 bits
+  int e = 1023 + 32 + 62 + n;  // biased exponent, less the leading bit the mantissa adds
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int i = 0; i < 2; ++i) {
+    const bool z = w2 == 0;
+    w2 = z ? w1 : w2;
+    w1 = z ? w0 : w1;
+    w0 = z ? 0u : w0;
+    e -= z ? 32 : 0;
+  }
+#ifdef __CUDA_ARCH__
+  const int c = __clz((int)w2);
+  const uint32_t b1 = __funnelshift_l(w1, w2, c), b0 = __funnelshift_l(w0, w1, c);
+#else
+  const int c = w2 ? __builtin_clz(w2) : 32;
+  const uint32_t b1 = c ? (c < 32 ? (w2 << c) | (w1 >> (32 - c)) : 0u) : w2;
+  const uint32_t b0 = c ? (c < 32 ? (w1 << c) | (w0 >> (32 - c)) : 0u) : w1;
+#endif
+  const unsigned long long b = ((unsigned long long)b1 << 32) | b0;
+  const unsigned long long v = ((unsigned long long)(uint32_t)(e - c) << 52) + (b >> 11) + ((b >> 10) & 1);
+  return w2 ? v | ((unsigned long long)(m & 1u) << 63) : 0ull;
+}
+// the same for any exponent (EX_BAD: a row with NaN or Inf)
+__device__ __noinline__ double from_totals_any(long long hi, long long lo, int n) {
+  if (n > EX_BAD / 2) return __longlong_as_double(0x7FF8000000000000ll);
+  return ldexp(fma((double)hi, 0x1p32, (double)lo), n);
+}
+// Programmatic dependent launch: k_fx64's set-up overlaps the end of k_panel, whose writes
+// are visible after the wait.  Not the other way round: blocks of k_panel that arrive
+// early settle two on one SM while others idle, and share its FP64 pipe (15.7 ms became
+// 23 at n = 5,000).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // digit planes of eight consecutive K elements of one row
 __device__ __forceinline__ void put_digits(const double (&v)[8], int ex, uint8_t* blk, int row, int kg) {
   const double sc = pow2d(61 - (ex == EX_BAD ? 0 : ex));
@@ -94,13 +142,14 @@ __device__ __forceinline__ void put_digits(const double (&v)[8], int ex, uint8_t
 }
 
 // ---- products --------------------------------------------------------------
-// Output tiles of 128 x 64.  A segment holds row tiles [ra, rb) with column tiles
-// [ca, cb), or [ca, 2 rt + 2) (the lower triangle) when tri.
+// A segment of output tiles: row tiles [ra, rb) with column tiles [ca, cb), or
+// [ca, CPT (rt + 1)) (the lower triangle, CPT = 128 / NT) when tri.
 struct Seg {
   int ra, rb, ca, cb, tri, cmin;
-  __host__ __device__ int count() const {
-    return rb <= ra ? 0 : tri ? (rb - ra) * (rb + ra + 1 - ca) : cb <= ca ? 0 : (rb - ra) * (cb - ca);
+  __host__ __device__ int upto(int cpt, int x) const {  // tiles in the row tiles [ra, x)
+    return tri ? cpt * (x - ra) * (x + ra + 1) / 2 - ca * (x - ra) : (x - ra) * (cb - ca);
   }
+  __host__ __device__ int count(int cpt) const { return rb <= ra || (!tri && cb <= ca) ? 0 : upto(cpt, rb); }
 };
 struct Job {
   const uint8_t *A, *B;
@@ -122,37 +171,44 @@ struct Bars {
   int abort;
 };
 
+template <int NT>
 __device__ __forceinline__ void tile_of(const Job& J, int t, int& rt, int& ct, int& cmin) {
-  const int c0 = J.seg[0].count();
+  constexpr int CPT = 128 / NT;
+  const int c0 = J.seg[0].count(CPT);
   const Seg& s = t < c0 ? J.seg[0] : J.seg[1];
   if (t >= c0) t -= c0;
   cmin = s.cmin;
+  int x;
   if (s.tri) {
-    // f(x) = (x - ra)(x + ra + 1 - ca) <= t < f(x + 1)
-    const float b = 1.0f - s.ca;
-    int x = (int)(0.5f * (-b + sqrtf(b * b + 4.0f * ((float)t + (float)s.ra * (s.ra + 1 - s.ca)))));
+    // the root of upto(x) = t, then the exact row tile beside it
+    const float h = 0.5f * CPT, b = h - s.ca;
+    x = (int)((sqrtf(b * b + 4.0f * h * ((float)t + (float)s.ra * (h * (s.ra + 1) - s.ca))) - b) / (2.0f * h));
     x = max(s.ra, min(x, s.rb - 1));
-    while (x > s.ra && (x - s.ra) * (x + s.ra + 1 - s.ca) > t) --x;
-    while ((x + 1 - s.ra) * (x + s.ra + 2 - s.ca) <= t) ++x;
-    rt = x;
-    ct = s.ca + t - (x - s.ra) * (x + s.ra + 1 - s.ca);
+    while (x > s.ra && s.upto(CPT, x) > t) --x;
+    while (s.upto(CPT, x + 1) <= t) ++x;
   } else {
-    const int w = s.cb - s.ca;
-    rt = s.ra + t / w;
-    ct = s.ca + t % w;
+    x = s.ra + t / (s.cb - s.ca);
   }
+  rt = x;
+  ct = s.ca + t - s.upto(CPT, x);
 }
 // first block of a row tile in a panel's storage (triangular panels keep K steps >= 4 rt)
 __device__ __forceinline__ size_t blk_of(int rt, int ks, int stride, int tri) {
   return tri ? (size_t)rt * stride - 2 * (size_t)rt * (rt - 1) + (ks - 4 * rt) : (size_t)rt * stride + ks;
 }
 
-// Warp roles: 0 bulk loads, 1 TMEM owner and MMA issuer, 2-9 epilogue (two warps
-// per TMEM lane quadrant, 32 columns each).
-__global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job J, int* status) {
+// Warp roles: 0 bulk loads, 1 TMEM owner and MMA issuer, 4 and up epilogue (NT / 16 warps
+// per TMEM lane quadrant, 16 columns each: wider shares unroll to more code than the
+// instruction cache holds, and every launch starts cold).  The epilogue is kept off the two slow
+// pipes: totals are read from the floats' bits (an F2I takes four times an add) and become
+// doubles in integer instructions; C is read and written in whole sectors through a
+// swizzled 32 x 8 staging block per warp.
+template <int NT>
+__global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_constant__ Job J, int* status) {
+  using T = Tile<NT>;
   extern __shared__ uint8_t dsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
-  Bars* bars = reinterpret_cast<Bars*>(smem + OFF_BAR);
+  Bars* bars = reinterpret_cast<Bars*>(smem + T::OFF_BAR);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NSTAGE; ++i) {
@@ -160,13 +216,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
       mbar_init(&bars->empty[i], 1);
     }
     mbar_init(&bars->acc_full, 1);
-    mbar_init(&bars->acc_empty, 8);
+    mbar_init(&bars->acc_empty, T::EW);
     mbar_init(&bars->drain, 1);
     bars->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem, 512);
+    tmem_alloc(&bars->tmem, 8 * NT);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -178,6 +234,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
     bars->abort = 1;
     atomicExch(status, DEV_TIMEOUT);
   };
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -185,17 +242,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
       bool ok = true;
       for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
         int rt, ct, cmin;
-        tile_of(J, t, rt, ct, cmin);
+        tile_of<NT>(J, t, rt, ct, cmin);
         for (int k = J.ktri ? 4 * rt : J.ks0; k < J.ks1; ++k, ++g) {
           const uint32_t s = g % NSTAGE;
           if (!mbar_wait(&bars->empty[s], ((g / NSTAGE) & 1) ^ 1, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(&bars->full[s], STAGE);
-          const uint32_t dst = smem_addr(smem + s * STAGE);
+          mbar_expect_tx(&bars->full[s], T::STAGE);
+          const uint32_t dst = smem_addr(smem + s * T::STAGE);
           bulk_load(dst, J.A + blk_of(rt, k, J.ka, J.ktri) * BLK, BLK, &bars->full[s]);
-          const uint8_t* b = J.B + blk_of(ct >> 1, k, J.kb, J.ktri) * BLK + (ct & 1) * PLANE_B;
+          const uint8_t* b = J.B + blk_of(ct / (128 / NT), k, J.kb, J.ktri) * BLK + (ct % (128 / NT)) * T::PLANE_B;
 #pragma unroll
           for (int pl = 0; pl < NPL; ++pl)
-            bulk_load(dst + BLK + pl * PLANE_B, b + pl * PLANE_A, PLANE_B, &bars->full[s]);
+            bulk_load(dst + BLK + pl * T::PLANE_B, b + pl * PLANE_A, T::PLANE_B, &bars->full[s]);
         }
       }
       if (!ok) fail();
@@ -207,7 +264,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
       bool ok = true;
       for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
         int rt, ct, cmin;
-        tile_of(J, t, rt, ct, cmin);
+        tile_of<NT>(J, t, rt, ct, cmin);
         const int k0 = J.ktri ? 4 * rt : J.ks0;
         for (int k = k0; k < J.ks1; ++k, ++g) {
           const int ci = (k - k0) % CHUNK;
@@ -218,7 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
           const uint32_t s = g % NSTAGE;
           if (!mbar_wait(&bars->full[s], (g / NSTAGE) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t op = smem_addr(smem + s * STAGE);
+          const uint32_t op = smem_addr(smem + s * T::STAGE);
 #pragma unroll
           for (int kh = 0; kh < 2; ++kh) {
             const uint32_t acc0 = (ci == 0 && kh == 0) ? 0u : 1u;
@@ -227,11 +284,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
             for (int pl = 0; pl < NPL; ++pl) {
               // digit plane pl of A against planes 0 .. 7 - pl of B: classes pl .. 7
               const uint64_t dA = sdesc_noswizzle(op + pl * PLANE_A + kh * 256, 128, 512);
-              const int n1 = (NPL - pl) * 64;
-              umma_f16(tmem + pl * 64, dA, sdesc_noswizzle(bb, 128, 512), idesc_f16_f32(128, n1 > 256 ? 256 : n1),
+              const int n1 = (NPL - pl) * NT;
+              umma_f16(tmem + pl * NT, dA, sdesc_noswizzle(bb, 128, 512), idesc_f16_f32(128, n1 > 256 ? 256 : n1),
                        pl == 0 ? acc0 : 1u);
               if (n1 > 256)
-                umma_f16(tmem + pl * 64 + 256, dA, sdesc_noswizzle(bb + 4 * PLANE_B, 128, 512),
+                umma_f16(tmem + pl * NT + 256, dA, sdesc_noswizzle(bb + (256 / NT) * T::PLANE_B, 128, 512),
                          idesc_f16_f32(128, n1 - 256), pl == 0 ? acc0 : 1u);
             }
           }
@@ -248,35 +305,59 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
       while (!mbar_try(&bars->drain, 0) && global_ns() - t0 < kWaitLimitNs) {}
     }
     __syncwarp();
-  } else {
-    const int q = warp & 3, j0 = ((warp - 2) >> 2) * 32;
+  } else if (warp >= 4) {
+    constexpr int MAGIC = 0x4B400000;  // bits of 1.5 2^23: those of 1.5 2^23 + v are MAGIC + v, |v| <= 2^22
+    const int q = warp & 3, j0 = ((warp - 4) >> 2) * 16;
+    uint8_t* out = smem + T::OFF_OUT + (warp - 4) * 2048;
     uint32_t c = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
       int rt, ct, cmin;
-      tile_of(J, t, rt, ct, cmin);
+      tile_of<NT>(J, t, rt, ct, cmin);
       const int steps = J.ks1 - (J.ktri ? 4 * rt : J.ks0);
       const int nch = (steps + CHUNK - 1) / CHUNK;
-      long long hi[32], lo[32];
+      const int rb = rt * 128 + q * 32, row = rb + lane, col0 = ct * NT + j0;
+      const int ea = J.ea[row] - 66;  // 56 - 2 * 61
+      const int el = J.eb[col0 + (lane & 15)];
+      long long hi[16], lo[16];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
+      for (int j = 0; j < 16; ++j) hi[j] = lo[j] = -(long long)MAGIC * 0x01010101ll * nch;
       for (int ch = 0; ch < nch; ++ch, ++c) {
         if (!mbar_wait_idle(&bars->acc_full, c & 1, abort_flag, 20)) { ok = false; break; }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + j0;
+        float big = 0.0f;
 #pragma unroll
-        for (int ci = 0; ci < NPL; ++ci) {
-          const int mul = 1 << ((3 - (ci & 3)) * 8);
+        for (int u = 0; u < NPL; ++u) {
+          uint32_t r[16];
+          tmem_ld16(ta + u * NT, r);
+          tmem_ld_wait();
+          const int mul = 1 << ((3 - (u & 3)) * 8);
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
+          for (int j = 0; j < 16; ++j) {
+            const float f = __uint_as_float(r[j]);
+            big = fmaxf(big, fabsf(f));
+            const long long v = (long long)__float_as_int(__fadd_rn(f, 12582912.0f)) * mul;
+            if (u < 4) hi[j] += v;
+            else lo[j] += v;
+          }
+        }
+        // sums past 2^22 (possible over more than 32 K elements, and rare) do not fit the bits
+        // trick: replace its value by the F2I's
+        if (__any_sync(~0u, big > 4194304.0f)) {
+#pragma unroll
+          for (int u = 0; u < NPL; ++u) {
             uint32_t r[16];
-            tmem_ld16(ta + ci * 64 + hh * 16, r);
+            tmem_ld16(ta + u * NT, r);
             tmem_ld_wait();
+            const int mul = 1 << ((3 - (u & 3)) * 8);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const long long v = (long long)__float2int_rn(__uint_as_float(r[j])) * mul;
-              if (ci < 4) hi[hh * 16 + j] += v;
-              else lo[hh * 16 + j] += v;
+              const float f = __uint_as_float(r[j]);
+              const long long v =
+                  (long long)(__float2int_rn(f) + MAGIC - __float_as_int(__fadd_rn(f, 12582912.0f))) * mul;
+              if (u < 4) hi[j] += v;
+              else lo[j] += v;
             }
           }
         }
@@ -285,41 +366,57 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
         if (lane == 0) mbar_arrive(&bars->acc_empty);
       }
       if (!ok) break;
-      const int row = rt * 128 + q * 32 + lane, col0 = ct * 64 + j0;
-      const int ea = J.ea[row] - 66;  // 56 - 2 * 61
-      auto val = [&](int j) -> double {
-        const int n = ea + J.eb[col0 + j];
-        const double x = fma((double)hi[j], 0x1p32, (double)lo[j]);
-        if (n > -1000 && n < 900) return x * pow2d(n);
-        return n > EX_BAD / 2 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(x, n);
-      };
-      if (J.mode == 0) {
-        if (row >= J.rmin && col0 + 31 >= cmin) {
-          double* p = J.C + (int64_t)row * J.ldc + col0;
-          if (col0 >= cmin) {
+      // usual exponents take the branch-free conversion
+      const bool usual = !__any_sync(~0u, ea + 66 < -400 || ea + 66 > 400 || el < -400 || el > 400);
+      const int chunk = lane & 3;
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              double2 o = *reinterpret_cast<double2*>(p + j);
-              o.x -= val(j);
-              o.y -= val(j + 1);
-              *reinterpret_cast<double2*>(p + j) = o;
-            }
+      for (int h = 0; h < 16; h += 8) {
+        const int cb = col0 + h;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          double2 x;
+          const int e0 = ea + __shfl_sync(~0u, el, h + j), e1 = ea + __shfl_sync(~0u, el, h + j + 1);
+          if (usual) {
+            x.x = __longlong_as_double((long long)from_totals(hi[h + j], lo[h + j], e0));
+            x.y = __longlong_as_double((long long)from_totals(hi[h + j + 1], lo[h + j + 1], e1));
           } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col0 + j >= cmin) p[j] -= val(j);
+            x.x = from_totals_any(hi[h + j], lo[h + j], e0);
+            x.y = from_totals_any(hi[h + j + 1], lo[h + j + 1], e1);
+          }
+          *reinterpret_cast<double2*>(out + lane * 64 + (((j >> 1) ^ ((lane >> 1) & 3)) << 4)) = x;
+          if (J.mode == 2 && row < J.m) {
+            if (cb + j <= row) J.C[(int64_t)(cb + j) * J.ldc + row] = x.x;
+            if (cb + j + 1 <= row) J.C[(int64_t)(cb + j + 1) * J.ldc + row] = x.y;
           }
         }
-      } else {
-        if (row < J.m) {
+        __syncwarp();
+        if (J.mode == 0) {
+          double2 o[4];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int cc = col0 + j;
-            if (cc < J.n && (J.mode == 1 || cc <= row)) {
-              const double x = val(j);
-              J.C[(int64_t)row * J.ldc + cc] = x;
-              if (J.mode == 2) J.C[(int64_t)cc * J.ldc + row] = x;
+          for (int i = 0; i < 4; ++i) {
+            const int r = rb + 8 * i + (lane >> 2);
+            if (r >= J.rmin && cb >= cmin)
+              o[i] = *reinterpret_cast<const double2*>(J.C + (int64_t)r * J.ldc + cb + 2 * chunk);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rl = 8 * i + (lane >> 2);
+            const double2 x = *reinterpret_cast<const double2*>(out + rl * 64 + ((chunk ^ ((rl >> 1) & 3)) << 4));
+            if (rb + rl >= J.rmin && cb >= cmin) {
+              o[i].x -= x.x;
+              o[i].y -= x.y;
+              *reinterpret_cast<double2*>(J.C + (int64_t)(rb + rl) * J.ldc + cb + 2 * chunk) = o[i];
             }
+          }
+        } else {
+          const int col = lane & 7, cc = cb + col;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rl = 4 * i + (lane >> 3), r = rb + rl;
+            const double x =
+                *reinterpret_cast<const double*>(out + rl * 64 + (((col >> 1) ^ ((rl >> 1) & 3)) << 4) + (col & 1) * 8);
+            if (r < J.m && cc < J.n && (J.mode == 1 || cc <= r)) J.C[(int64_t)r * J.ldc + cc] = x;
           }
         }
       }
@@ -329,7 +426,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx64(const __grid_constant__ Job
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) tmem_dealloc(tmem, 8 * NT);
 }
 
 // ---- digits of a matrix ------------------------------------------------------
@@ -386,16 +483,24 @@ __global__ void __launch_bounds__(128) k_digits(const double* __restrict__ src, 
 }
 
 // ---- Cholesky ------------------------------------------------------------------
-// W (np x np row-major) = lower triangle of A (column-major), identity on the padding
+// The factorization runs on D A D, D_ii = 2^-k_i with 4^k_i <= A_ii < 4^(k_i + 1): its entries
+// are below 4, so that no 2 x 2 determinant over- or underflows, and the scaling is exact.
+__global__ void k_scales(const double* __restrict__ A, int64_t n, int64_t np, int32_t* __restrict__ sc) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= np) return;
+  const double v = i < n ? A[i * n + i] : 1.0;
+  sc[i] = v > 0.0 && isfinite(v) ? ilogb(v) >> 1 : 0;
+}
+// W (np x np row-major) = lower triangle of D A D (A column-major), identity on the padding
 __global__ void __launch_bounds__(256) k_load_lower(const double* __restrict__ A, int64_t n, int64_t np,
-                                                    double* __restrict__ W) {
+                                                    const int32_t* __restrict__ sc, double* __restrict__ W) {
   __shared__ double t[32][33];
   const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
   if (j0 > i0) return;
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   for (int c = y; c < 32; c += 8) {
     const int64_t i = i0 + x, j = j0 + c;
-    t[c][x] = (i < n && j < n) ? A[j * n + i] : (i == j ? 1.0 : 0.0);
+    t[c][x] = (i < n && j < n) ? A[j * n + i] * pow2d(max(-1022, min(1023, -sc[i] - sc[j]))) : (i == j ? 1.0 : 0.0);
   }
   __syncthreads();
   for (int r = y; r < 32; r += 8) W[(i0 + r) * np + j0 + x] = t[x][r];
@@ -416,115 +521,188 @@ struct Panel {
   int* bad;
 };
 
+// 1 / d from the hardware's 20-bit approximation by one third-order (Householder) step:
+// with e = 1 - d r, 1 / d = r (1 + e + e^2 + ...)
+__device__ __forceinline__ double reciprocal(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // One 32-wide step.  Every CTA factors the pivot block (it is small, and a separate
-// launch would cost more than the repeat), then takes 32-row groups: out = v X' with v
+// launch would cost more than the repeat), then takes 16-row groups: out = v X' with v
 // the row's 32 entries in the pivot columns (rows below the pivot), the column's
 // entries in the pivot rows (columns left of it), or a unit vector (the pivot rows).
-// FP64 issue bounds both parts.
+//
+// A chain of FP64 latencies bounds it: a dependent multiply-add takes 68 clocks, a reciprocal
+// 230, a publish and barrier 120, and one warp-wide FP64 instruction holds its
+// quarter of the SM's FP64 pipe for 64.  Hence 2 x 2 pivots (one reciprocal and one
+// barrier for two columns), the next pivot's rows and its publication ahead of the other
+// rows of a step, no square root inside the chain, and groups of 16 rows, which put a
+// problem of 2,000 rows on 128 SMs.  Measured at n = 2,048: 39,000 clocks, 25,000 of them the
+// pivots (50,000 with 1 x 1 pivots, and 73,000 with their square roots and divisions).
 __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) {
-  __shared__ double X[32][33], V[32][33], Lm[32][33], prow[2][32], pv[32];
+  __shared__ double X[32][33], V[32][33], Lm[32][33], pa[16][32], pb[16][32];
+  __shared__ double pv[32], i1[16], l2[16], i2[16];
   __shared__ int mx[4][32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t np = a.np;
-  double* Wk = a.W + (int64_t)a.k0 * np + a.k0;
-  // lane = column, registers = rows w + 4 t
+  const double* Wk = a.W + (int64_t)a.k0 * np + a.k0;
+  // lane = column; registers 2 s, 2 s + 1 = rows 2 (w + 4 s), 2 (w + 4 s) + 1
   double d[8];
-  for (int r = w; r < 32; r += 4) V[r][lane] = lane <= r ? Wk[r * np + lane] : 0.0;
-  __syncthreads();
 #pragma unroll
   for (int t = 0; t < 8; ++t) {
-    const int r = w + 4 * t;
-    d[t] = lane <= r ? V[r][lane] : V[lane][r];
+    const int r = 2 * (w + 4 * (t >> 1)) + (t & 1);
+    d[t] = lane <= r ? Wk[r * np + lane] : Wk[lane * np + r];
   }
+  // the first group's entries, in flight during the factorization
+  const int row = lane & 15, half = lane >> 4;
+  const int gk = a.k0 / 16, ng = (int)(np / 16);
+  int g = (a.inverse ? 0 : gk) + blockIdx.x;
+  double pre[4];
+  auto fetch = [&](int gg) {
+    const int r0 = gg * 16;
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
+    for (int i = 0; i < 4; ++i)
+      pre[i] = gg > gk + 1 ? a.W[(int64_t)(r0 + w + 4 * i) * np + a.k0 + lane]
+               : gg < gk   ? a.W[(int64_t)(a.k0 + 2 * w + half + 8 * i) * np + r0 + row]
+                           : (2 * w + half + 8 * i == r0 - a.k0 + row ? 1.0 : 0.0);
+  };
+  if (g < ng) fetch(g);
+  // rows 2 j, 2 j + 1 (registers 2 s, 2 s + 1 of warp j & 3) times the inverse of their
+  // 2 x 2 pivot, whose own columns take the inverse itself
+  auto publish = [&](int j, double& da, double& db) {
+    const int k = 2 * j;
+    const double p11 = __shfl_sync(~0u, da, k), p12 = __shfl_sync(~0u, db, k), p22 = __shfl_sync(~0u, db, k + 1);
+    const double det = fma(p11, p22, -p12 * p12);
+    const double inv = reciprocal(det);
+    da = lane == k ? 1.0 : lane == k + 1 ? 0.0 : da;
+    db = lane == k ? 0.0 : lane == k + 1 ? 1.0 : db;
+    pa[j][lane] = fma(p22, da, -p12 * db) * inv;
+    pb[j][lane] = fma(p11, db, -p12 * da) * inv;
+    if (lane == 0) {
+      pv[k] = p11;
+      pv[k + 1] = det;  // over p11 below
+      l2[j] = p12;
+    }
+    asm volatile("bar.arrive %0, 128;" ::"r"(1 + (j & 7)) : "memory");
+  };
+  if (w == 0) publish(0, d[0], d[1]);
+#pragma unroll
+  for (int ss = 0; ss < 4; ++ss) {
+#pragma unroll 1
     for (int ww = 0; ww < 4; ++ww) {
-      const int k = 4 * kk + ww, b = k & 1;
-      if (w == ww) {
-        const double p = __shfl_sync(~0u, d[kk], k);
-        const double inv = 1.0 / p;
-        prow[b][lane] = lane == k ? inv : d[kk] * inv;
-        if (lane == k) {
-          pv[k] = p;
-          d[kk] = 1.0;
-        }
+      const int j = 4 * ss + ww, k = 2 * j;
+      if (w != ww) asm volatile("bar.sync %0, 128;" ::"r"(1 + (j & 7)) : "memory");
+      const double qa = pa[j][lane], qb = pb[j][lane];
+      const bool piv = (lane >> 1) == j;
+      auto update = [&](int t) {
+        const double f1 = __shfl_sync(~0u, d[t], k), f2 = __shfl_sync(~0u, d[t], k + 1);
+        const int r = 2 * (w + 4 * (t >> 1)) + (t & 1);
+        if (lane == k) Lm[r][k] = f1;
+        if (lane == k + 1) Lm[r][k + 1] = f2;
+        d[t] = fma(-f2, qb, fma(-f1, qa, piv ? 0.0 : d[t]));
+      };
+      // the next pivot's rows first, and their pivot, before the other rows
+      if (w > ww) {
+        update(2 * ss);
+        update(2 * ss + 1);
+        if (w == ww + 1) publish(j + 1, d[2 * ss], d[2 * ss + 1]);
       }
-      __syncthreads();
-      const double qv = prow[b][lane];
+      if (ss < 3) {
+        update(2 * ss + 2);
+        update(2 * ss + 3);
+        if (ww == 3 && w == 0) publish(j + 1, d[2 * ss + 2], d[2 * ss + 3]);
+      }
 #pragma unroll
-      for (int t = kk; t < 8; ++t) {
-        if (t > kk || w > ww) {
-          const double f = __shfl_sync(~0u, d[t], k);
-          if (lane == k) Lm[w + 4 * t][k] = f;
-          d[t] = fma(-f, qv, lane == k ? 0.0 : d[t]);
-        }
-      }
+      for (int t = 2 * ss + 4; t < 8; ++t) update(t);
+    }
+  }
+  __syncthreads();
+  // 2 x 2 Cholesky factors of the pivots: [1 / i1, 0; l2, 1 / i2]
+  if (tid < 16) {
+    const double p11 = pv[2 * tid], r1 = rsqrt(p11), p2 = pv[2 * tid + 1] * r1 * r1;
+    i1[tid] = r1;
+    l2[tid] *= r1;
+    i2[tid] = rsqrt(p2);
+    pv[2 * tid + 1] = p2;
+    if (blockIdx.x == 0) {
+      a.piv[a.k0 + 2 * tid] = p11;
+      a.piv[a.k0 + 2 * tid + 1] = p2;
+      if (!(p11 > 0.0) || !(p2 > 0.0) || !isfinite(p11) || !isfinite(p2)) atomicExch(a.bad, 1);
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int r = w + 4 * t;
-    X[r][lane] = lane <= r ? d[t] / sqrt(pv[r]) : 0.0;
-  }
-  if (blockIdx.x == 0 && tid < 32) {
-    const double p = pv[tid];
-    a.piv[a.k0 + tid] = p;
-    if (!(p > 0.0) || !isfinite(p)) atomicExch(a.bad, 1);
+  for (int t = 0; t < 8; t += 2) {
+    const int j = w + 2 * t, r = 2 * j;
+    const double x0 = lane <= r ? d[t] * i1[j] : 0.0;
+    X[r][lane] = x0;
+    X[r + 1][lane] = lane <= r + 1 ? fma(-l2[j], x0, d[t + 1]) * i2[j] : 0.0;
   }
   __syncthreads();
-  const int gk = a.k0 / 32, ng = (int)(np / 32), g0 = a.inverse ? 0 : gk;
-  for (int g = g0 + blockIdx.x; g < ng; g += gridDim.x) {
-    const int r0 = g * 32, r = r0 + lane;
+  pdl_launch();
+  // groups of 16 rows: lane = (row, half of the columns)
+  for (; g < ng; g += gridDim.x) {
+    const int r0 = g * 16;
+    const bool below = g > gk + 1, left = g < gk;
     // V[l][row]
-    if (g > gk) {
-      for (int i = w; i < 32; i += 4) V[lane][i] = a.W[(int64_t)(r0 + i) * np + a.k0 + lane];
-    } else if (g < gk) {
-      for (int l = w; l < 32; l += 4) V[l][lane] = a.W[(int64_t)(a.k0 + l) * np + r];
-    } else {
-      for (int l = w; l < 32; l += 4) V[l][lane] = l == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (below) V[lane][w + 4 * i] = pre[i];
+      else V[2 * w + half + 8 * i][row] = pre[i];
     }
     __syncthreads();
-    double acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.0;
+    if (g + (int)gridDim.x < ng) fetch(g + gridDim.x);
+    const int c0 = 2 * w + half;  // columns c0 + 8 j
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int l = 0; l < 32; ++l) {
-      const double v = V[l][lane];
+      const double v = V[l][row];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (l <= 4 * j + 3) acc[j] = fma(v, X[w + 4 * j][l], acc[j]);
+      for (int j = 0; j < 4; ++j)
+        if (l <= 8 * j + 7) acc[j] = fma(v, X[c0 + 8 * j][l], acc[j]);
     }
     __syncthreads();
     int e = EX_MIN;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      V[w + 4 * j][lane] = acc[j];
+    for (int j = 0; j < 4; ++j) {
+      V[c0 + 8 * j][row] = acc[j];
       if (acc[j] != 0.0) e = max(e, expo(acc[j]));
     }
     mx[w][lane] = e;
     __syncthreads();
-    e = max(max(mx[0][lane], mx[1][lane]), max(mx[2][lane], mx[3][lane]));
-    if (w == 0) {
-      a.ex[r] = e;
-      a.exo[r] = (a.k0 == a.K0 || g == gk) ? e : max(e, a.exo[r]);
-      if (a.inverse && g <= gk) a.exm[r] = g == gk ? e : max(e, a.exm[r]);
-    }
-    double v8[8];
+    if (tid < 64) {  // (row, K group)
+      const int rr = tid & 15, kg = tid >> 4, r = r0 + rr;
+      e = EX_MIN;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v8[i] = V[w * 8 + i][lane];
-    put_digits(v8, e, a.dig + (size_t)(r0 / 128) * BLK, r & 127, w);
-    if (g > gk) {
-      for (int i = w; i < 32; i += 4) {
+      for (int i = 0; i < 4; ++i) e = max(e, max(mx[i][rr], mx[i][rr + 16]));
+      if (kg == 0) {
+        a.ex[r] = e;
+        a.exo[r] = (a.k0 == a.K0 || !(below || left)) ? e : max(e, a.exo[r]);
+        if (a.inverse && !below) a.exm[r] = left ? max(e, a.exm[r]) : e;
+      }
+      double v8[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v8[i] = V[kg * 8 + i][rr];
+      put_digits(v8, e, a.dig + (size_t)(r0 / 128) * BLK, r & 127, kg);
+    } else if (below) {
+      for (int i = w - 2; i < 16; i += 2) {
         const double l = V[lane][i];
         a.P[(int64_t)(r0 + i) * a.B + (a.k0 - a.K0) + lane] = l;
         a.W[(int64_t)(r0 + i) * np + a.k0 + lane] = a.inverse ? 0.0 : l;
       }
-    } else if (g < gk) {
-      for (int l = w; l < 32; l += 4) a.W[(int64_t)(a.k0 + l) * np + r] = V[l][lane];
+    } else if (left) {
+      for (int l = 2 * (w - 2) + half; l < 32; l += 4) a.W[(int64_t)(a.k0 + l) * np + r0 + row] = V[l][row];
     } else {
-      for (int l = w; l < 32; l += 4) {
-        const double x = a.inverse ? X[l][lane] : lane < l ? Lm[l][lane] / sqrt(pv[lane]) : sqrt(pv[l]);
+      for (int i = w - 2; i < 16; i += 2) {
+        const int l = r0 - a.k0 + i, j = lane >> 1;
+        double x = X[l][lane];
+        if (!a.inverse) {
+          if ((l >> 1) == j) x = (l & 1) == 0 ? pv[l] * i1[j] : (lane & 1) ? pv[l] * i2[j] : l2[j];
+          else if (lane < l) x = (lane & 1) ? (Lm[l][lane] - Lm[l][lane - 1] * i1[j] * l2[j]) * i2[j] : Lm[l][lane] * i1[j];
+        }
         a.D[(a.k0 + l) * 32 + lane] = lane <= l ? x : 0.0;
       }
     }
@@ -558,10 +736,13 @@ __global__ void __launch_bounds__(128) k_panel_digits(const __grid_constant__ Pa
 }
 // Digits of M' (row j = column j of M = L^-1, K steps from the row tile's own on)
 __global__ void __launch_bounds__(128) k_minv_digits(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int n, int ks,
-                                                     const int32_t* __restrict__ ex, uint8_t* __restrict__ dig) {
+                                                     const int32_t* __restrict__ ex, const int32_t* __restrict__ sc,
+                                                     int32_t* __restrict__ exd, uint8_t* __restrict__ dig) {
   const int rt = blockIdx.x, k0 = blockIdx.y;
   if (k0 < 4 * rt) return;
   const int r = rt * 128 + threadIdx.x;
+  // A^-1 = D (M'M) D: the scaling goes into the product's exponents
+  if (k0 == 4 * rt) exd[r] = r < n ? ex[r] - sc[r] : EX_MIN;
   uint8_t* blk = dig + blk_of(rt, k0, ks, 1) * BLK;
   const int e = r < n ? ex[r] : EX_MIN;
 #pragma unroll
@@ -575,11 +756,12 @@ __global__ void __launch_bounds__(128) k_minv_digits(const double* __restrict__ 
     put_digits(v, e, blk, threadIdx.x, kg);
   }
 }
-// sum of log pivots, in a fixed order
-__global__ void __launch_bounds__(256) k_logsum(const double* __restrict__ piv, int n, double* __restrict__ out) {
+// sum of log pivots of A, in a fixed order
+__global__ void __launch_bounds__(256) k_logsum(const double* __restrict__ piv, const int32_t* __restrict__ sc, int n,
+                                                double* __restrict__ out) {
   __shared__ double red[256];
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += 256) s += log(piv[i]);
+  for (int i = threadIdx.x; i < n; i += 256) s += log(piv[i]) + sc[i] * (2.0 * 0.69314718055994530942);
   red[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
@@ -589,11 +771,12 @@ __global__ void __launch_bounds__(256) k_logsum(const double* __restrict__ piv, 
   if (threadIdx.x == 0) out[0] = red[0];
 }
 // U = L' (column-major upper = row-major lower), zeros elsewhere
-__global__ void k_store_factor(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int64_t n, double* __restrict__ out) {
+__global__ void k_store_factor(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int64_t n,
+                               const int32_t* __restrict__ sc, double* __restrict__ out) {
   const int64_t total = n * n;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / n, c = i % n;
-    out[i] = c <= r ? lower(W, D, np, r, c) : 0.0;
+    out[i] = c <= r ? lower(W, D, np, r, c) * pow2d(sc[r]) : 0.0;
   }
 }
 
@@ -604,7 +787,7 @@ constexpr size_t kKeepBytes = (size_t)1 << 30;
 struct Scratch {
   DevBuf<double> W, P, D, piv;
   DevBuf<uint8_t> din, dout, dm;
-  DevBuf<int32_t> ex, exo, exm;
+  DevBuf<int32_t> ex, exo, exm, sc;
   DevBuf<int> bad;
   size_t bytes() const { return W.n * 8 + P.n * 8 + din.n + dout.n + dm.n; }
 };
@@ -617,12 +800,39 @@ static Scratch& scratch(cbx_handle* h) {
   return *static_cast<Scratch*>(h->fx_slot.get());
 }
 
-static void launch(cbx_handle* h, Job& J) {
-  J.tiles = J.seg[0].count() + J.seg[1].count();
-  if (J.tiles <= 0 || J.ks1 <= 0) return;
-  ensure_smem((const void*)k_fx64, SMEM, h->device);
-  k_fx64<<<std::min(J.tiles, h->num_sms), THREADS, SMEM, h->stream>>>(J, h->status.p);
+template <typename K, typename... A>
+static void launch_pdl(cbx_handle* h, K kern, dim3 grid, int threads, int smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CBX_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+// Segments count 32-column tiles; pairs of them make the 64-wide ones.  A 32-wide tile costs
+// about 0.6 of a 64-wide one (the same A digits for half the columns): narrow tiles where
+// they fill SMs that wide ones leave idle in the last wave.
+template <int NT>
+static void launch_tiles(cbx_handle* h, Job J) {
+  for (Seg& s : J.seg) {
+    s.ca /= NT / 32;
+    s.cb = (s.cb + NT / 32 - 1) / (NT / 32);
+  }
+  J.tiles = J.seg[0].count(128 / NT) + J.seg[1].count(128 / NT);
+  ensure_smem((const void*)k_fx64<NT>, Tile<NT>::SMEM, h->device);
+  launch_pdl(h, k_fx64<NT>, dim3(std::min(J.tiles, h->num_sms)), Tile<NT>::THREADS, Tile<NT>::SMEM, J, h->status.p);
   h->launched("k_fx64");
+}
+static void launch(cbx_handle* h, const Job& J) {
+  const int64_t t32 = (int64_t)J.seg[0].count(4) + J.seg[1].count(4), sms = h->num_sms;
+  if (t32 <= 0 || J.ks1 <= 0) return;
+  if (6 * ((t32 + sms - 1) / sms) < 10 * ((t32 / 2 + sms - 1) / sms)) launch_tiles<32>(h, J);
+  else launch_tiles<64>(h, J);
 }
 
 }  // namespace fx
@@ -654,7 +864,7 @@ void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int
   J.ea = A.ex.p;
   J.eb = B.ex.p;
   J.ka = J.kb = J.ks1 = A.ks;
-  J.seg[0] = {0, A.rt, 0, (int)((n + 63) / 64), 0, 0};
+  J.seg[0] = {0, A.rt, 0, (int)((n + 31) / 32), 0, 0};
   J.mode = 1;
   J.m = (int)m;
   J.n = (int)n;
@@ -679,9 +889,12 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
   fx::at_least(S.ex, (size_t)np);
   fx::at_least(S.exo, (size_t)np);
   fx::at_least(S.exm, (size_t)np);
+  fx::at_least(S.sc, (size_t)np);
   fx::at_least(S.bad, 1);
   CBX_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), s));
-  fx::k_load_lower<<<dim3((unsigned)(np / 32), (unsigned)(np / 32)), 256, 0, s>>>(A, n, np, S.W.p);
+  fx::k_scales<<<(unsigned)(np / 128), 128, 0, s>>>(A, n, np, S.sc.p);
+  h->launched("k_scales");
+  fx::k_load_lower<<<dim3((unsigned)(np / 32), (unsigned)(np / 32)), 256, 0, s>>>(A, n, np, S.sc.p, S.W.p);
   h->launched("k_load_lower");
   fx::Panel a{S.W.p, np, 0, 0, 0, B, inverse ? 1 : 0, S.din.p, S.ex.p, S.exo.p, S.exm.p, S.P.p, S.D.p, S.piv.p,
               S.bad.p};
@@ -694,7 +907,7 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
     const int tp = a.K1 / 128;
     for (int k0 = a.K0; k0 < a.K1 && k0 < n; k0 += 32) {
       a.k0 = k0;
-      const int groups = (int)(np / 32) - (inverse ? 0 : k0 / 32);
+      const int groups = (int)(np / 16) - (inverse ? 0 : k0 / 16);
       fx::k_panel<<<std::min(groups, h->num_sms), 128, 0, s>>>(a);
       h->launched("k_panel");
       const int next = k0 + 32;
@@ -704,8 +917,8 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
       J.ea = J.eb = S.ex.p;
       J.ka = J.kb = J.ks1 = 1;
       J.rmin = next;
-      J.seg[0] = {next / 128, tp, inverse ? 0 : next / 64, 0, 1, inverse ? 0 : next};
-      J.seg[1] = {tp, rt, next / 64, 2 * tp, 0, next};
+      J.seg[0] = {next / 128, tp, inverse ? 0 : next / 32, 0, 1, inverse ? 0 : next};
+      J.seg[1] = {tp, rt, next / 32, 4 * tp, 0, next};
       fx::launch(h, J);
     }
     if (a.K1 >= n) break;
@@ -716,14 +929,14 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
     J.ea = J.eb = S.exo.p;
     J.ka = J.kb = J.ks1 = B / 32;
     J.rmin = a.K1;
-    J.seg[0] = {tp, rt, inverse ? 0 : 2 * tp, 0, 1, 0};
+    J.seg[0] = {tp, rt, inverse ? 0 : 4 * tp, 0, 1, 0};
     J.seg[1] = {0, 0, 0, 0, 0, 0};
     fx::launch(h, J);
   }
   double ld = 0.0;
   int bad = 0;
   if (logdet) {
-    fx::k_logsum<<<1, 256, 0, s>>>(S.piv.p, (int)n, S.piv.p + np);
+    fx::k_logsum<<<1, 256, 0, s>>>(S.piv.p, S.sc.p, (int)n, S.piv.p + np);
     h->launched("k_logsum");
     CBX_CUDA(cudaMemcpyAsync(&ld, S.piv.p + np, sizeof(double), cudaMemcpyDeviceToHost, s));
   }
@@ -733,11 +946,11 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
   if (!bad && inverse) {
     const int ks = (int)(np / 32);
     fx::at_least(S.dm, ((size_t)rt * ks - 2 * (size_t)rt * (rt - 1)) * fx::BLK);
-    fx::k_minv_digits<<<dim3(rt, ks), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, S.exm.p, S.dm.p);
+    fx::k_minv_digits<<<dim3(rt, ks), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, S.exm.p, S.sc.p, S.ex.p, S.dm.p);
     h->launched("k_minv_digits");
     fx::Job M{};
     M.A = M.B = S.dm.p;
-    M.ea = M.eb = S.exm.p;
+    M.ea = M.eb = S.ex.p;
     M.ka = M.kb = M.ks1 = ks;
     M.ktri = 1;
     M.seg[0] = {0, rt, 0, 0, 1, 0};
@@ -747,8 +960,8 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
     M.ldc = n;
     fx::launch(h, M);
   } else if (!bad && out) {
-    fx::k_store_factor<<<(unsigned)std::min<int64_t>((n * n + 255) / 256, 8 * h->num_sms), 256, 0, s>>>(S.W.p, S.D.p, np, n,
-                                                                                                      out);
+    fx::k_store_factor<<<(unsigned)std::min<int64_t>((n * n + 255) / 256, 8 * h->num_sms), 256, 0, s>>>(
+        S.W.p, S.D.p, np, n, S.sc.p, out);
     h->launched("k_store_factor");
   }
   if (logdet) *logdet = ld;
