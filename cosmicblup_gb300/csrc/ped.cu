@@ -16,8 +16,11 @@
 // children, the D scaling, and a forward pass that pulls from parents, one
 // kernel per generation.  The result is the same matrix A[geno, geno].
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <set>
+#include <system_error>
+#include <thread>
 #include <vector>
 #include <cublas_v2.h>
 #include <cusolverDn.h>
@@ -79,10 +82,204 @@ static void ml(const std::vector<int64_t>& dam, const std::vector<int64_t>& sire
   }
 }
 
-struct Trip {
-  int64_t r, c;
-  double v;
+// All nt threads arrive before any leaves (few arrivals, short waits: it spins).
+class Rendezvous {
+ public:
+  void wait(int nt) {
+    const int ph = phase_.load(std::memory_order_acquire);
+    if (count_.fetch_add(1, std::memory_order_acq_rel) == nt - 1) {
+      count_.store(0, std::memory_order_relaxed);
+      phase_.store(ph + 1, std::memory_order_release);
+    } else {
+      while (phase_.load(std::memory_order_acquire) == ph) std::this_thread::yield();
+    }
+  }
+
+ private:
+  std::atomic<int> count_{0}, phase_{0};
 };
+// Runs body(t, k) on k <= nt threads, t = 0 on the caller's; k is as many as could be
+// started.  body must not throw.
+template <typename F>
+static void on_threads(int nt, F&& body) {
+  std::vector<std::thread> pool;
+  pool.reserve(nt);
+  std::atomic<int> go{0};
+  try {
+    for (int t = 1; t < nt; ++t)
+      pool.emplace_back([&, t] {
+        int k = 0;
+        while ((k = go.load(std::memory_order_acquire)) == 0) std::this_thread::yield();
+        body(t, k);
+      });
+  } catch (const std::system_error&) {
+  }
+  const int k = (int)pool.size() + 1;
+  go.store(k, std::memory_order_release);
+  body(0, k);
+  for (auto& th : pool) th.join();
+}
+
+// Generation of every animal (0 for founders, one above the later parent), the animals
+// by generation in index order, and where each generation starts; false when some
+// parent is not listed before its progeny.
+static bool generations(const std::vector<int64_t>& dam, const std::vector<int64_t>& sire,
+                        std::vector<int64_t>& order, std::vector<int64_t>& start) {
+  const int64_t n = (int64_t)dam.size();
+  std::vector<int32_t> level(n, 0);
+  int64_t nlev = 0;
+  for (int64_t i = 0; i < n; ++i) {
+    if (dam[i] >= i || sire[i] >= i) return false;
+    int32_t lv = 0;
+    if (dam[i] >= 0) lv = std::max(lv, level[dam[i]] + 1);
+    if (sire[i] >= 0) lv = std::max(lv, level[sire[i]] + 1);
+    level[i] = lv;
+    nlev = std::max<int64_t>(nlev, lv + 1);
+  }
+  start.assign(nlev + 1, 0);
+  for (int64_t i = 0; i < n; ++i) start[level[i] + 1]++;
+  for (int64_t l = 0; l < nlev; ++l) start[l + 1] += start[l];
+  order.resize(n);
+  std::vector<int64_t> at(start.begin(), start.end() - 1);
+  for (int64_t i = 0; i < n; ++i) order[at[level[i]]++] = i;
+  return true;
+}
+
+// ml for a pedigree listed parents first.  An animal's F reads only earlier generations,
+// so each generation's animals run in parallel, every one with the same operations in the
+// same order: ancestors by descending index, here from a heap (an ancestor enters it when
+// its coefficient leaves 0, so once).  It was 98 ms for 15,000 animals in ten generations
+// with one thread and a std::set.
+static void ml_ordered(const std::vector<int64_t>& dam, const std::vector<int64_t>& sire,
+                       const std::vector<int64_t>& order, const std::vector<int64_t>& start, std::vector<double>& f,
+                       std::vector<double>& dii) {
+  const int64_t n = (int64_t)dam.size(), nlev = (int64_t)start.size() - 1;
+  f.assign(n, 0.0);
+  dii.assign(n, 1.0);
+  const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
+  const int nt = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(16, hw), n / 256));
+  Rendezvous meet;
+  std::vector<std::atomic<int64_t>> next(nlev);
+  for (int64_t l = 0; l < nlev; ++l) next[l].store(start[l]);
+  std::vector<std::vector<double>> Ls(nt, std::vector<double>(n, 0.0));
+  std::vector<std::vector<int64_t>> heaps(nt);
+  for (auto& hp : heaps) hp.reserve(n);
+  on_threads(nt, [&](int t, int k) {
+    std::vector<double>& L = Ls[t];
+    std::vector<int64_t>& heap = heaps[t];
+    auto add = [&](int64_t j, double v) {
+      if (!(v > 0.0)) return;  // underflowed: it counts nothing
+      if (L[j] == 0.0) {
+        heap.push_back(j);
+        std::push_heap(heap.begin(), heap.end());
+      }
+      L[j] += v;
+    };
+    constexpr int64_t kChunk = 16;
+    for (int64_t l = 0; l < nlev; ++l) {
+      for (int64_t a = next[l].fetch_add(kChunk); a < start[l + 1]; a = next[l].fetch_add(kChunk))
+        for (int64_t e = a; e < std::min(a + kChunk, start[l + 1]); ++e) {
+          const int64_t i = order[e], s = sire[i], d = dam[i];
+          const double Fs = s >= 0 ? f[s] : 0.0, Fd = d >= 0 ? f[d] : 0.0;
+          if (s >= 0 && d >= 0) dii[i] = 1.0 - 0.25 * (1.0 + Fs) - 0.25 * (1.0 + Fd);
+          else if (s >= 0) dii[i] = 1.0 - 0.25 * (1.0 + Fs);
+          else if (d >= 0) dii[i] = 1.0 - 0.25 * (1.0 + Fd);
+          if (s < 0 || d < 0) continue;
+          add(s, 0.5);
+          add(d, 0.5);
+          double F_calc = 0.0;
+          while (!heap.empty()) {
+            const int64_t j = heap.front();
+            std::pop_heap(heap.begin(), heap.end());
+            heap.pop_back();
+            const double lj = L[j];
+            L[j] = 0.0;
+            F_calc += lj * lj * dii[j];
+            if (sire[j] >= 0) add(sire[j], 0.5 * lj);
+            if (dam[j] >= 0) add(dam[j], 0.5 * lj);
+          }
+          f[i] = F_calc + dii[i] - 1.0;
+          if (f[i] < 0.0) f[i] = 0.0;
+        }
+      meet.wait(k);
+    }
+  });
+}
+
+// Henderson's A^-1 with Meuwissen-Luo inbreeding.  Each row's terms are summed in the
+// order in which the animals emit them.
+struct Ainv {
+  std::vector<int64_t> ptr;
+  std::vector<int32_t> col;
+  std::vector<double> val, F, dii;
+};
+static Ainv ainv(const std::vector<int64_t>& d, const std::vector<int64_t>& s, const std::vector<int64_t>& order,
+                 const std::vector<int64_t>& start, bool ordered) {
+  const int64_t n = (int64_t)d.size();
+  Ainv A;
+  if (ordered) ml_ordered(d, s, order, start, A.F, A.dii);
+  else ml(d, s, A.F, A.dii);
+  // terms by row, in emission order (a counting sort), then by column within a row
+  struct Term {
+    int32_t c;
+    double v;
+  };
+  std::vector<int64_t> at(n + 1, 0);
+  auto emit = [&](auto&& out) {
+    for (int64_t i = 0; i < n; ++i) {
+      const int64_t di = d[i], si = s[i];
+      const double dinv = 1.0 / A.dii[i];
+      out(i, i, dinv);
+      if (si >= 0) {
+        out(i, si, -0.5 * dinv);
+        out(si, i, -0.5 * dinv);
+        out(si, si, 0.25 * dinv);
+      }
+      if (di >= 0) {
+        out(i, di, -0.5 * dinv);
+        out(di, i, -0.5 * dinv);
+        out(di, di, 0.25 * dinv);
+      }
+      if (si >= 0 && di >= 0) {
+        out(si, di, 0.25 * dinv);
+        out(di, si, 0.25 * dinv);
+      }
+    }
+  };
+  emit([&](int64_t r, int64_t, double) { ++at[r + 1]; });
+  for (int64_t i = 0; i < n; ++i) at[i + 1] += at[i];
+  std::vector<Term> t(at[n]);
+  {
+    std::vector<int64_t> fill(at.begin(), at.end() - 1);
+    emit([&](int64_t r, int64_t c, double v) { t[fill[r]++] = {(int32_t)c, v}; });
+  }
+  A.ptr.assign(n + 1, 0);
+  A.col.reserve(t.size());
+  A.val.reserve(t.size());
+  for (int64_t r = 0; r < n; ++r) {
+    Term* b = t.data() + at[r];
+    Term* e = t.data() + at[r + 1];
+    std::stable_sort(b, e, [](const Term& x, const Term& y) { return x.c < y.c; });
+    bool has_diag = false;
+    while (b < e) {
+      const int32_t c = b->c;
+      double v = 0.0;
+      for (; b < e && b->c == c; ++b) v += b->v;
+      if (c == r) {
+        has_diag = true;
+        if (v < 1e-15) v = 1e-12;  // enforceSymmetryAndDiagonal(A, 1e-12, 1e-15)
+      }
+      if (std::fabs(v) > 1e-24) {  // prune(1e-12) with Eigen's dummy precision
+        A.col.push_back(c);
+        A.val.push_back(v);
+      }
+    }
+    A.ptr[r + 1] = (int64_t)A.col.size();
+    // every row has a diagonal (a founder-only animal at least has 1/dii)
+    CBX_REQUIRE(has_diag, CBX_ERR_ARG, "internal: missing diagonal");
+  }
+  return A;
+}
 
 // Backward pass of T^T: y_j = x_j + 1/2 sum over children c of y_c, for the
 // animals of one generation (children already final).  Y row-major n x ng.
@@ -179,63 +376,18 @@ extern "C" int cbx_ainv_henderson(cbx_handle* h, int64_t n, const int64_t* dam, 
       if (!(d[j] >= 0 && d[j] < n)) d[j] = -1;
       if (!(s[j] >= 0 && s[j] < n)) s[j] = -1;
     }
-    std::vector<double> f, dii;
-    ped::ml(d, s, f, dii);
-    std::vector<ped::Trip> t;
-    t.reserve((size_t)n * 9);
-    for (int64_t i = 0; i < n; ++i) {
-      const int64_t di = d[i], si = s[i];
-      const double dinv = 1.0 / dii[i];
-      t.push_back({i, i, dinv});
-      if (si >= 0) {
-        t.push_back({i, si, -0.5 * dinv});
-        t.push_back({si, i, -0.5 * dinv});
-        t.push_back({si, si, 0.25 * dinv});
-      }
-      if (di >= 0) {
-        t.push_back({i, di, -0.5 * dinv});
-        t.push_back({di, i, -0.5 * dinv});
-        t.push_back({di, di, 0.25 * dinv});
-      }
-      if (si >= 0 && di >= 0) {
-        t.push_back({si, di, 0.25 * dinv});
-        t.push_back({di, si, 0.25 * dinv});
-      }
-    }
-    std::stable_sort(t.begin(), t.end(),
-                     [](const ped::Trip& a, const ped::Trip& b) { return a.r != b.r ? a.r < b.r : a.c < b.c; });
-    std::vector<int64_t> rp(n + 1, 0);
-    std::vector<int32_t> cc;
-    std::vector<double> vv;
-    std::vector<bool> has_diag(n, false);
-    for (size_t k = 0; k < t.size();) {
-      size_t e = k;
-      double v = 0.0;
-      while (e < t.size() && t[e].r == t[k].r && t[e].c == t[k].c) v += t[e++].v;
-      const int64_t r = t[k].r, c = t[k].c;
-      if (r == c) {
-        has_diag[r] = true;
-        if (v < 1e-15) v = 1e-12;  // enforceSymmetryAndDiagonal(A, 1e-12, 1e-15)
-      }
-      if (std::fabs(v) > 1e-24) {  // prune(1e-12) with Eigen's dummy precision
-        cc.push_back((int32_t)c);
-        vv.push_back(v);
-        rp[r + 1]++;
-      }
-      k = e;
-    }
-    // every row has a diagonal (a founder-only animal at least has 1/dii)
-    for (int64_t i = 0; i < n; ++i) CBX_REQUIRE(has_diag[i], CBX_ERR_ARG, "internal: missing diagonal");
-    for (int64_t i = 0; i < n; ++i) rp[i + 1] += rp[i];
-    *nnz = (int64_t)cc.size();
+    std::vector<int64_t> order, start;
+    const bool ordered = ped::generations(d, s, order, start);
+    const ped::Ainv A = ped::ainv(d, s, order, start, ordered);
+    *nnz = (int64_t)A.col.size();
     if (ptr) {
       CBX_REQUIRE(col && val, CBX_ERR_ARG, "col / val must be given with ptr");
-      std::copy(rp.begin(), rp.end(), ptr);
-      std::copy(cc.begin(), cc.end(), col);
-      std::copy(vv.begin(), vv.end(), val);
+      std::copy(A.ptr.begin(), A.ptr.end(), ptr);
+      std::copy(A.col.begin(), A.col.end(), col);
+      std::copy(A.val.begin(), A.val.end(), val);
     }
-    if (F) std::copy(f.begin(), f.end(), F);
-    if (dii_out) std::copy(dii.begin(), dii.end(), dii_out);
+    if (F) std::copy(A.F.begin(), A.F.end(), F);
+    if (dii_out) std::copy(A.dii.begin(), A.dii.end(), dii_out);
   });
 }
 
@@ -249,35 +401,20 @@ extern "C" int cbx_ssgblup_qinv(cbx_handle* h, int64_t n, const int64_t* dam, co
     CBX_REQUIRE(ng > 0 && ng <= n && gmap, CBX_ERR_ARG, "bad genotyped map");
     CBX_CUDA(cudaSetDevice(h->device));
     cudaStream_t s = h->stream;
-    // A^-1 and inbreeding on the host
-    int64_t nnz = 0;
-    if (int rc = cbx_ainv_henderson(h, n, dam, sire, &nnz, nullptr, nullptr, nullptr, nullptr, nullptr); rc != CBX_OK)
-      throw Error(rc, h->last_error);
-    std::vector<int64_t> ap(n + 1);
-    std::vector<int32_t> ac(nnz);
-    std::vector<double> av(nnz), dii(n);
-    if (int rc = cbx_ainv_henderson(h, n, dam, sire, &nnz, ap.data(), ac.data(), av.data(), nullptr, dii.data());
-        rc != CBX_OK)
-      throw Error(rc, h->last_error);
-    // generations and children lists (parents first)
-    std::vector<int64_t> d(dam, dam + n), sr(sire, sire + n), level(n, 0);
+    CBX_REQUIRE(n > 0 && dam && sire, CBX_ERR_ARG, "bad pedigree arguments");
+    std::vector<int64_t> d(dam, dam + n), sr(sire, sire + n);
     for (int64_t i = 0; i < n; ++i) {
       if (!(d[i] >= 0 && d[i] < n)) d[i] = -1;
       if (!(sr[i] >= 0 && sr[i] < n)) sr[i] = -1;
-      CBX_REQUIRE(d[i] < i && sr[i] < i, CBX_ERR_ARG,
-                  "pedigree must list parents before their progeny (as genmatrix::ml assumes)");
-      int64_t lv = 0;
-      if (d[i] >= 0) lv = std::max(lv, level[d[i]] + 1);
-      if (sr[i] >= 0) lv = std::max(lv, level[sr[i]] + 1);
-      level[i] = lv;
     }
-    const int64_t nlev = n ? *std::max_element(level.begin(), level.end()) + 1 : 0;
-    std::vector<int64_t> order(n);
-    for (int64_t i = 0; i < n; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int64_t a, int64_t b) { return level[a] < level[b]; });
-    std::vector<int64_t> lstart(nlev + 1, 0);
-    for (int64_t i = 0; i < n; ++i) lstart[level[i] + 1]++;
-    for (int64_t l = 0; l < nlev; ++l) lstart[l + 1] += lstart[l];
+    std::vector<int64_t> order, lstart;
+    CBX_REQUIRE(ped::generations(d, sr, order, lstart), CBX_ERR_ARG,
+                "pedigree must list parents before their progeny (as genmatrix::ml assumes)");
+    const int64_t nlev = (int64_t)lstart.size() - 1;
+    // A^-1 and inbreeding on the host
+    const ped::Ainv A = ped::ainv(d, sr, order, lstart, true);
+    const std::vector<double>& dii = A.dii;
+    // children lists
     std::vector<int64_t> cptr(n + 1, 0), cidx;
     for (int64_t i = 0; i < n; ++i) {
       if (d[i] >= 0) cptr[d[i] + 1]++;
@@ -394,7 +531,7 @@ extern "C" int cbx_ssgblup_qinv(cbx_handle* h, int64_t n, const int64_t* dam, co
     h->Hd = std::move(Gd);
     h->Hd_n = ng;
     ++h->Hd_gen;
-    if (int rc = cbx_mme_set_qinv_split(h, ap.data(), ac.data(), av.data(), nullptr, ng, gmap); rc != CBX_OK)
+    if (int rc = cbx_mme_set_qinv_split(h, A.ptr.data(), A.col.data(), A.val.data(), nullptr, ng, gmap); rc != CBX_OK)
       throw Error(rc, h->last_error);
   });
 }
