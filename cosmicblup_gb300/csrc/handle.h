@@ -45,6 +45,7 @@ struct cbx_handle {
   std::vector<char> probe_z_have;
   int probe_z_seed = -1;
   int64_t probe_z_q = -1;
+  int64_t qinv_count = 0;  // Qinvs set on this handle so far
   // mixed-model equations and REML state
   std::unique_ptr<cbx::Mme> mme;
   // cbx_mme_keep_warm: an MME rebuilt with the same shape starts its solves from

@@ -1781,6 +1781,7 @@ extern "C" int cbx_mme_set_qinv_dense(cbx_handle* h, const double* Qinv, int64_t
                                cudaMemcpyDeviceToDevice, s));
     m.has_dense = true;
     m.has_sparse = false;
+    m.qinv_id = ++h->qinv_count;
     m.drop_carry(h->keep_warm);
     CBX_CUDA(cudaStreamSynchronize(s));
     for (auto& sp : m.solvers)
@@ -1817,6 +1818,7 @@ extern "C" int cbx_mme_set_qinv_split(cbx_handle* h, const int64_t* a_ptr, const
     upload_csr_pair(h, q, ptr, a_col, a_val, m.Qs64, m.Qs32);
     m.has_sparse = true;
     m.has_dense = ng > 0;
+    m.qinv_id = ++h->qinv_count;
     m.drop_carry(h->keep_warm);
     if (ng > 0) {
       CBX_REQUIRE(gmap, CBX_ERR_ARG, "genotyped map missing");

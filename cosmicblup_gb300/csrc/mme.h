@@ -64,6 +64,7 @@ struct Mme {
   // there; a later MME built from the same, unchanged block keeps them
   const void* planes_src = nullptr;
   int64_t planes_gen = -1;
+  int64_t qinv_id = 0;             // which Qinv of the handle this is (cbx_handle::qinv_count at its setting)
   // row scales of the Qd32 / Qlo32 planes for the fixed-point tensor-core
   // refinement product (valid while fx_rows_ok), and its scratch
   DevBuf<int32_t> fx_rowexp;

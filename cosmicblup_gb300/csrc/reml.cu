@@ -54,10 +54,12 @@ __global__ void k_build_lhs(int64_t dim, int64_t p, const int32_t* __restrict__ 
     C[i] = (r >= p && c >= p) ? lam * Qd[(r - p) * ld + (c - p)] : 0.0;
   }
 }
+// one warp per row: a fixed-effect row may hold an entry per record
 __global__ void k_scatter_csr(int64_t dim, const int32_t* __restrict__ Dptr, const int32_t* __restrict__ Dcol,
                               const double* __restrict__ Dval, double* __restrict__ C) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < dim; r += (int64_t)gridDim.x * blockDim.x)
-    for (int32_t j = Dptr[r]; j < Dptr[r + 1]; ++j) C[(int64_t)Dcol[j] * dim + r] += Dval[j];
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); r < dim; r += nw)
+    for (int32_t j = Dptr[r] + (threadIdx.x & 31); j < Dptr[r + 1]; j += 32) C[(int64_t)Dcol[j] * dim + r] += Dval[j];
 }
 // P[i, j] = (delta_ij - (W C^-1 W^T)[i, j]) / ve from the explicit C^-1 (dim x
 // dim, column-major, symmetric): a gather over the two records' design rows
@@ -781,17 +783,24 @@ static void reml_gradient(cbx_handle* h, double vu, double ve, int nprobe, int s
 struct DenseExact {
   bool init = false;
   int64_t n = 0, dim = 0;
+  int64_t qinv_id = -1;  // the Qinv (Mme::qinv_id) this belongs to
   DevBuf<double> ZAZt;
   FxPanel Vdig, Pdig;
   // kept between steps up to order kKeepDense (0.5 GB each), where allocating them costs
   // as much as the step: LHS, its inverse, P, P V
   DevBuf<double> C, Ci, P, Mu;
   double log_det_A = 0;
+  // the point whose LHS, inverse and solution C, Ci and sol hold: cbx_reml_solve's steps
+  // start where the one before ended, so each factors one LHS and not two
+  bool at = false;
+  double at_vu = 0, at_ve = 0, at_logL = 0;
+  DevBuf<double> sol;
   static constexpr int64_t kKeepDense = 8192;
   struct Trim {
     DenseExact& d;
     ~Trim() {
       if (d.n <= kKeepDense && d.dim <= kKeepDense) return;
+      d.at = false;
       d.C.release();
       d.Ci.release();
       d.P.release();
@@ -802,6 +811,11 @@ struct DenseExact {
 static DenseExact& dense_state(cbx_handle* h) {
   if (!h->dense_slot) h->dense_slot = std::make_shared<DenseExact>();
   return *static_cast<DenseExact*>(h->dense_slot.get());
+}
+
+// A point is kept within one call only: each entry starts with none.
+static void forget_point(cbx_handle* h) {
+  if (h->dense_slot) dense_state(h).at = false;
 }
 
 static void dense_init(cbx_handle* h, DenseExact& D) {
@@ -825,6 +839,8 @@ static void dense_init(cbx_handle* h, DenseExact& D) {
   CBX_CUDA(cudaStreamSynchronize(s));
   D.n = n;
   D.dim = dim;
+  D.qinv_id = m.qinv_id;
+  D.at = false;
   D.init = true;
 }
 
@@ -837,7 +853,7 @@ static void build_lhs(cbx_handle* h, double lam, DevBuf<double>& C) {
   k_build_lhs<<<gridn(dim * dim, 256, 8 * h->num_sms), 256, 0, s>>>(dim, m.p, m.D64.ptr.p, m.D64.col.p, m.D64.val.p,
                                                                      m.Qd64.p, m.ld, lam, C.p);
   h->launched("k_build_lhs");
-  k_scatter_csr<<<gridn(dim, 256, 4 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, C.p);
+  k_scatter_csr<<<gridn(dim * 32, 256, 8 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, C.p);
   h->launched("k_scatter_csr");
 }
 // y = A x (+ y0 when given, minus A x when neg) for a symmetric n x n matrix: one warp
@@ -875,29 +891,29 @@ static void solve_by_inverse(cbx_handle* h, const double* C, const double* Ci, i
 }
 
 // compute_logL of run_dense_exact_step (vce.cpp:2974-3007); -1e18 if C is not PD.  D.C
-// keeps the LHS (its factor when inverse is false), D.Ci its inverse.
-static double dense_logL(cbx_handle* h, DenseExact& D, double vu, double ve, bool inverse, DevBuf<double>& sol) {
+// keeps the LHS, D.Ci its inverse and D.sol the solution.
+static double dense_logL(cbx_handle* h, DenseExact& D, double vu, double ve) {
   Mme& m = *h->mme;
   const int64_t n = m.n_rec, p = m.p, q = m.q, dim = m.dim;
+  if (D.at && D.at_vu == vu && D.at_ve == ve) return D.at_logL;
+  D.at = false;
   build_lhs(h, ve / vu, D.C);
-  if (inverse) D.Ci.resize((size_t)dim * dim);
+  D.Ci.resize((size_t)dim * dim);
   double ld_C = 0.0;
-  if (!fx64_cholesky(h, D.C.p, dim, inverse, inverse ? D.Ci.p : D.C.p, &ld_C)) return -1e18;
+  if (!fx64_cholesky(h, D.C.p, dim, true, D.Ci.p, &ld_C)) return -1e18;
   if (!std::isfinite(ld_C)) return -1e18;
-  if (inverse) {
-    solve_by_inverse(h, D.C.p, D.Ci.p, dim, m.rhs.p, sol);
-  } else {
-    sol.resize(dim);
-    CBX_CUDA(cudaMemcpyAsync(sol.p, m.rhs.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    potrs(h, D.C.p, dim, sol.p, 1);
-  }
+  solve_by_inverse(h, D.C.p, D.Ci.p, dim, m.rhs.p, D.sol);
   DevBuf<double> e;
   e.resize(n);
-  record_residual(h, sol.p, e.p);
+  record_residual(h, D.sol.p, e.p);
   const auto eh = d2h(h, e.p, n);
   const double yPy = dot_h(m.y_host, eh) / ve;
   const double m2 = ld_C + (double)(n - p - q) * std::log(ve) + (double)q * std::log(vu) + yPy + D.log_det_A;
-  return -0.5 * m2;
+  D.at = true;
+  D.at_vu = vu;
+  D.at_ve = ve;
+  D.at_logL = -0.5 * m2;
+  return D.at_logL;
 }
 
 static void project_spd_2x2(double A[2][2], double eps_rel = 1e-8, double eps_abs = 1e-12) {
@@ -930,15 +946,18 @@ static void project_spd_2x2(double A[2][2], double eps_rel = 1e-8, double eps_ab
 static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterInfo& info) {
   Mme& m = *h->mme;
   DenseExact& D = dense_state(h);
-  if (!D.init || D.n != m.n_rec || D.dim != m.dim) dense_init(h, D);
+  if (!D.init || D.qinv_id != m.qinv_id) dense_init(h, D);
   cudaStream_t s = h->stream;
   Libs& L = libs(h);
   const int64_t n = m.n_rec, dim = m.dim;
   const double vu = vu_io, ve = ve_io;
   DenseExact::Trim trim{D};
-  DevBuf<double> sol;
-  const double cur0 = dense_logL(h, D, vu, ve, true, sol);
+  const double cur0 = dense_logL(h, D, vu, ve);
   if (cur0 <= -1e18) return false;
+  // the data solution at the starting point: the step's result
+  DevBuf<double> sol0;
+  sol0.resize(dim);
+  CBX_CUDA(cudaMemcpyAsync(sol0.p, D.sol.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, s));
   double cur = cur0;
   // P = (I - W C^-1 W^T) / ve from the explicit C^-1, then M_u = P ZAZ^T by digits
   DevBuf<double>&P = D.P, &Mu = D.Mu;
@@ -962,7 +981,7 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   DevBuf<double> e, ZPy;
   e.resize(n);
   ZPy.resize(n);
-  record_residual(h, sol.p, e.p);
+  record_residual(h, D.sol.p, e.p);
   std::vector<double> Py = d2h(h, e.p, n);
   for (auto& v : Py) v /= ve;
   DevBuf<double> dPy;
@@ -998,15 +1017,14 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   for (int k = 0; k < max_halving; ++k) {
     const double vu_n = vu + delta[0], ve_n = ve + delta[1];
     if (vu_n > 0 && ve_n > 0) {
-      DevBuf<double> s2;
-      const double nl = dense_logL(h, D, vu_n, ve_n, false, s2);
+      const double nl = dense_logL(h, D, vu_n, ve_n);
       if (nl > cur || k == max_halving - 1) {
         cur = nl;
         vu_io = vu_n;
         ve_io = ve_n;
-        m.last_solution.resize(dim);
-        CBX_CUDA(cudaMemcpyAsync(m.last_solution.p, sol.p, dim * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        m.last_solution = std::move(sol0);
         m.has_last = true;
+        m.has_last_resid = false;
         info.kind = 1;
         info.logL = cur;
         info.var_u = vu_io;
@@ -1088,7 +1106,7 @@ static bool factor_lhs_q(cbx_handle* h, const double* Q, double lam, DevBuf<doub
   k_build_lhs<<<gridn(dim * dim, 256, 8 * h->num_sms), 256, 0, s>>>(dim, m.p, m.D64.ptr.p, m.D64.col.p, m.D64.val.p,
                                                                      Q, m.q, lam, C.p);
   h->launched("k_build_lhs");
-  k_scatter_csr<<<gridn(dim, 256, 4 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, C.p);
+  k_scatter_csr<<<gridn(dim * 32, 256, 8 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, C.p);
   h->launched("k_scatter_csr");
   return potrf(h, C.p, dim);
 }
@@ -1197,7 +1215,7 @@ static bool ai_data_step(cbx_handle* h, double& vu_io, double& ve_io, IterInfo& 
     k_build_lhs<<<gridn(dim * dim, 256, 8 * h->num_sms), 256, 0, s>>>(dim, p, m.D64.ptr.p, m.D64.col.p,
                                                                        m.D64.val.p, Q.p, q, lam, Ci.p);
     h->launched("k_build_lhs");
-    k_scatter_csr<<<gridn(dim, 256, 4 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, Ci.p);
+    k_scatter_csr<<<gridn(dim * 32, 256, 8 * h->num_sms), 256, 0, s>>>(dim, m.D64.ptr.p, m.D64.col.p, m.D64.val.p, Ci.p);
     h->launched("k_scatter_csr");
     if (!chol_inverse_device(h, Ci.p, dim)) return false;
     const unsigned g = gridn(q * q, 256, 4 * h->num_sms);
@@ -1346,6 +1364,7 @@ extern "C" int cbx_reml_iterate(cbx_handle* h, const cbx_reml_config* cfg, doubl
     CBX_REQUIRE(var_u && var_e && *var_u > 0 && *var_e > 0, CBX_ERR_ARG, "variances must be positive");
     CBX_CUDA(cudaSetDevice(h->device));
     IterInfo it;
+    forget_point(h);
     reml_iterate(h, to_cfg(cfg), *var_u, *var_e, it);
     to_info(it, info);
   });
@@ -1362,6 +1381,7 @@ extern "C" int cbx_reml_iterate_grad(cbx_handle* h, const cbx_reml_config* cfg, 
     const RemlConfigI c = to_cfg(cfg);
     const double vu0 = *var_u, ve0 = *var_e;
     IterInfo it;
+    forget_point(h);
     reml_iterate(h, c, *var_u, *var_e, it, nprobe);
     to_info(it, info);
     cbx::reml_gradient(h, vu0, ve0, nprobe, c.seed, 0, c.precision, c.pcg_tol, c.pcg_max_iter, grad, trace,
@@ -1380,6 +1400,7 @@ extern "C" int cbx_reml_solve(cbx_handle* h, const cbx_reml_config* cfg, double*
     CBX_CUDA(cudaSetDevice(h->device));
     const RemlConfigI c = to_cfg(cfg);
     int iters = 0, conv = 0;
+    forget_point(h);
     for (int it = 0; it < c.max_iter; ++it) {
       const double ou = *var_u, oe = *var_e;
       IterInfo info;
@@ -1693,10 +1714,10 @@ extern "C" int cbx_reml_logl_dense(cbx_handle* h, double var_u, double var_e, do
     const cbx::Mme& m = *h->mme;
     if (m.has_dense && !m.has_sparse && m.ng == m.q) {
       cbx::DenseExact& D = cbx::dense_state(h);
-      if (!D.init || D.n != m.n_rec || D.dim != m.dim) cbx::dense_init(h, D);
+      if (!D.init || D.qinv_id != m.qinv_id) cbx::dense_init(h, D);
       cbx::DenseExact::Trim trim{D};
-      cbx::DevBuf<double> sol;
-      *logL = cbx::dense_logL(h, D, var_u, var_e, false, sol);
+      D.at = false;
+      *logL = cbx::dense_logL(h, D, var_u, var_e);
     } else {
       // a split Qinv: calc_logL_internal, without the constant log|A|
       CBX_REQUIRE(m.dim <= cbx::kAiDenseMax, CBX_ERR_UNSUPPORTED, "LHS too large for a dense factorization");
