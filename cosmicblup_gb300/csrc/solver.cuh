@@ -593,6 +593,19 @@ __device__ __forceinline__ double block_sum_cols(double v, double* red /*[NT]*/)
   }
 }
 
+// red[tid] summed over the groups tid / S of an N-thread block, by halves in a fixed order;
+// the totals are in red[0 .. S).  One thread per column adding N / S values in turn took
+// 35 us in FP64 (68 clocks an addition) where S is 1.
+template <typename T, int S, int N>
+__device__ __forceinline__ void tree_sum_cols(T* red) {
+#pragma unroll
+  for (int o = N / 2; o >= S; o >>= 1) {
+    __syncthreads();
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+  }
+  __syncthreads();
+}
+
 // Fixed-effect rows of W'W can hold one entry per record (the mean holds all of
 // them).  They are cut into segments of at most FIX_SEG entries; k_fix_seg
 // computes one partial sum per (segment, column) and k_spmv adds a row's
@@ -619,12 +632,8 @@ __global__ void __launch_bounds__(NT) k_fix_seg(OpView<T> op, const int32_t* __r
   }
   for (; j < hi; j += G) acc[0] += op.Dval[j] * X[(int64_t)op.Dcol[j] * S + c];
   redT[tid] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-  __syncthreads();
-  if (tid < S) {
-    T s = T(0);
-    for (int gg = 0; gg < G; ++gg) s += redT[gg * S + tid];
-    seg_part[(int64_t)sg * S + tid] = s;
-  }
+  tree_sum_cols<T, S, NT>(redT);
+  if (tid < S) seg_part[(int64_t)sg * S + tid] = redT[tid];
   (void)seg_row;
 }
 
@@ -840,11 +849,10 @@ __global__ void __launch_bounds__(NT) k_spmv(OpView<T> op, const T* __restrict__
     if (use_D && c < ncp)
       for (int32_t k = fix_seg_ptr[i] + g; k < fix_seg_ptr[i + 1]; k += GS) s += seg_part[(int64_t)k * S + c];
     redT[tid] = s;
-    __syncthreads();
+    tree_sum_cols<T, S, NT>(redT);
     if (tid >= ncp && tid < S) Y[i * S + tid] = T(0);  // defined, never read
     if (tid < ncp) {
-      T t = T(0);
-      for (int gg = 0; gg < GS; ++gg) t += redT[gg * S + tid];
+      const T t = redT[tid];
       Y[i * S + tid] = t;
       if (P) pq = (double)P[i * S + tid] * (double)t;
     }
@@ -923,10 +931,9 @@ __global__ void __launch_bounds__(NT_FIXED) k_fixed(OpView<T> op, const T* __res
   const int64_t kend = (col == nullptr || col[c].active) ? op.p : 0;  // inactive columns: nothing to do
   for (int64_t k = g; k < kend; k += G) acc += op.A11inv[f * op.p + k] * R[k * S + c];
   redT[tid] = acc;
-  __syncthreads();
+  tree_sum_cols<T, S, NT_FIXED>(redT);
   if (tid < S) {
-    T s = T(0);
-    for (int gg = 0; gg < G; ++gg) s += redT[gg * S + tid];
+    const T s = redT[tid];
     const bool act = col == nullptr || col[tid].active;
     if (act) Z[f * S + tid] = s;
     const T zf = act ? s : Z[f * S + tid];
@@ -1257,12 +1264,14 @@ __global__ void __launch_bounds__(NTC) k_scalar_beta_c(Col* col, const double* p
     last = atomicAdd(done, 1u) == (unsigned)(S - 1);
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
+  if (last) {
+    // all columns' flags in flight at once: one thread reading them in turn took 5 us
     __threadfence();
-    int n_act = 0;
-    for (int k = 0; k < S; ++k) n_act += __ldcg(&col[k].active);
-    *active_count = n_act;
-    *done = 0u;
+    const int n_act = __syncthreads_count((int)threadIdx.x < S && __ldcg(&col[threadIdx.x].active) != 0);
+    if (threadIdx.x == 0) {
+      *active_count = n_act;
+      *done = 0u;
+    }
   }
 }
 
