@@ -29,7 +29,7 @@
 namespace cbx {
 namespace mt {
 
-constexpr int EM_NT = 512;
+constexpr int EM_NT = 128;
 constexpr int kMaxTraits = 8;
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -74,167 +74,239 @@ __global__ void k_half_cov(const double* __restrict__ Y, int64_t n, int t, doubl
     }
 }
 
-// In-register inverse of an SPD T x T matrix by Cholesky; false if not PD.
+// 1 / d from the hardware's 20-bit approximation by one third-order (Householder) step
+__device__ __forceinline__ double reciprocal(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// In-register inverse of an SPD T x T matrix V = L D L' (unit lower L); false if not PD.
+// No square root and T reciprocals: FP64 issue bounds the EM loop.
 template <int T>
 __device__ __forceinline__ bool spd_inverse(const double (&V)[T][T], double (&P)[T][T]) {
-  double L[T][T];
+  double L[T][T], id[T];
+  bool ok = true;
 #pragma unroll
   for (int j = 0; j < T; ++j) {
+    double w[T];  // w_k = L_jk d_k
     double d = V[j][j];
 #pragma unroll
-    for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
-    if (!(d > 0.0)) return false;
-    const double ljj = sqrt(d);
-    L[j][j] = ljj;
+    for (int k = 0; k < j; ++k) {
+      // L[j][k] holds L_jk d_k until here
+      w[k] = L[j][k];
+      L[j][k] = w[k] * id[k];
+      d = fma(-w[k], L[j][k], d);
+    }
+    ok = ok && d > 0.0;
+    id[j] = reciprocal(d);
 #pragma unroll
     for (int i = j + 1; i < T; ++i) {
       double s = V[i][j];
 #pragma unroll
-      for (int k = 0; k < j; ++k) s -= L[i][k] * L[j][k];
-      L[i][j] = s / ljj;
+      for (int k = 0; k < j; ++k) s = fma(-L[i][k], L[j][k], s);  // (L_ik d_k) L_jk
+      L[i][j] = s;
     }
   }
-  // Linv (lower), then P = Linv' Linv
-  double Li[T][T];
+  // M = L^-1 (unit lower), P = M' D^-1 M
+  double M[T][T];
 #pragma unroll
   for (int j = 0; j < T; ++j) {
 #pragma unroll
-    for (int i = 0; i < T; ++i) Li[i][j] = 0.0;
-    Li[j][j] = 1.0 / L[j][j];
-#pragma unroll
     for (int i = j + 1; i < T; ++i) {
-      double s = 0;
+      double s = -L[i][j];
 #pragma unroll
-      for (int k = j; k < i; ++k) s -= L[i][k] * Li[k][j];
-      Li[i][j] = s / L[i][i];
+      for (int k = j + 1; k < i; ++k) s = fma(-L[i][k], M[k][j], s);
+      M[i][j] = s;
     }
   }
 #pragma unroll
-  for (int a = 0; a < T; ++a)
+  for (int b = 0; b < T; ++b) {
+    double g[T];  // g_k = M_kb / d_k
 #pragma unroll
-    for (int b = a; b < T; ++b) {
-      double s = 0;
+    for (int k = b; k < T; ++k) g[k] = k == b ? id[b] : M[k][b] * id[k];
 #pragma unroll
-      for (int k = (a > b ? a : b); k < T; ++k) s += Li[k][a] * Li[k][b];
+    for (int a = 0; a <= b; ++a) {
+      double s = a == b ? g[b] : M[b][a] * g[b];
+#pragma unroll
+      for (int k = b + 1; k < T; ++k) s = fma(M[k][a], g[k], s);
       P[a][b] = s;
       P[b][a] = s;
     }
-  return true;
+  }
+  return ok;
 }
 
-// The whole MvEigenVce EM loop (runNullModel) in one block.  D: eigenvalues
-// (clamped at 0 here), R: rotated responses (n x T, column-major).  VgVe holds
-// the start values and receives the result; info = {iterations, converged,
-// status (0 ok, 1 V_i not positive definite)}.
+// The whole MvEigenVce EM loop (runNullModel) in one cooperative launch.  D: eigenvalues
+// (clamped at 0 here), R: rotated responses (n x T, column-major).  VgVe holds the start
+// values and receives the result; info = {iterations, converged, status (0 ok, 1 V_i not
+// positive definite)}.
+//
+// FP64 issue bounds an iteration: a warp's FP64 instruction holds a quarter of an SM's
+// pipe for 64 clocks.  So the samples are spread over one 128-thread block per SM (a
+// warp per quarter), every block adds all blocks' partial sums and makes the same
+// update, in the same order, and one grid barrier an iteration suffices (the partials
+// alternate between two buffers).  part: 2 x gridDim x (K + 1); sync: {arrivals, gave up},
+// zero.
 template <int T>
 __global__ void __launch_bounds__(EM_NT) k_mv_em(const double* __restrict__ D, const double* __restrict__ R, int64_t n,
                                                  int max_iter, double tol, double* __restrict__ VgVe,
-                                                 int* __restrict__ info) {
+                                                 int* __restrict__ info, double* part,
+                                                 unsigned long long* sync, int* status) {
   constexpr int NS = T * (T + 1) / 2;  // packed upper triangle
   constexpr int K = 2 * NS;
-  __shared__ double Vg[T][T], Ve[T][T];
-  __shared__ double part[EM_NT / 32][K];
-  __shared__ double tot[K];
-  __shared__ int done, bad;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x < T * T) {
-    Vg[threadIdx.x / T][threadIdx.x % T] = VgVe[threadIdx.x];
-    Ve[threadIdx.x / T][threadIdx.x % T] = VgVe[T * T + threadIdx.x];
+  constexpr int NW = EM_NT / 32;
+  __shared__ double Vg[T][T], Ve[T][T], Tg[T][T], Te[T][T], Ng[T][T], Ne[T][T];
+  __shared__ double wsum[NW][(K + 8) / 8 * 8], buf[NW][8][33];
+  __shared__ double tot[K + 1], sub[8][K + 1], nrm[4];
+  __shared__ int done, quit;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < T * T) {
+    Vg[tid / T][tid % T] = VgVe[tid];
+    Ve[tid / T][tid % T] = VgVe[T * T + tid];
   }
-  if (threadIdx.x == 0) { done = 0; bad = 0; }
+  if (tid == 0) done = quit = 0;
   __syncthreads();
-  int it = 0;
-  for (; it < max_iter && !done && !bad; ++it) {
-    double acc[K];
+  int it = 0, bad = 0;
+  while (it < max_iter) {
+    double acc[(K + 8) / 8 * 8];
 #pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += EM_NT) {
+    for (int k = 0; k < (K + 8) / 8 * 8; ++k) acc[k] = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)EM_NT + tid; i < n; i += (int64_t)gridDim.x * EM_NT) {
       const double d = D[i] > 0.0 ? D[i] : 0.0;
       double V[T][T], P[T][T], r[T], q[T];
 #pragma unroll
       for (int a = 0; a < T; ++a) {
         r[a] = R[a * n + i];
 #pragma unroll
-        for (int b = 0; b < T; ++b) V[a][b] = Vg[a][b] * d + Ve[a][b];
+        for (int b = 0; b <= a; ++b) V[a][b] = fma(Vg[a][b], d, Ve[a][b]);
       }
-      if (!spd_inverse<T>(V, P)) { atomicExch(&bad, 1); continue; }
+      if (!spd_inverse<T>(V, P)) { acc[K] += 1.0; continue; }
 #pragma unroll
       for (int a = 0; a < T; ++a) {
         double s = 0;
 #pragma unroll
-        for (int b = 0; b < T; ++b) s += P[a][b] * r[b];
+        for (int b = 0; b < T; ++b) s = fma(P[a][b], r[b], s);
         q[a] = s;
       }
-      const bool big = d > 1e-12;
+      const double db = d > 1e-12 ? d : 0.0;
       int k = 0;
 #pragma unroll
       for (int a = 0; a < T; ++a)
 #pragma unroll
         for (int b = a; b < T; ++b, ++k) {
-          const double m = q[a] * q[b] - P[a][b];
+          const double m = fma(q[a], q[b], -P[a][b]);
           acc[NS + k] += m;
-          if (big) acc[k] += d * m;
+          acc[k] = fma(db, m, acc[k]);
         }
     }
+    // warp sums, eight values at a time through shared memory: ten additions for eight sums
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const double v = warp_sum(acc[k]);
-      if (lane == 0) part[warp][k] = v;
+    for (int k0 = 0; k0 <= K; k0 += 8) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) buf[warp][k][lane] = acc[k0 + k];
+      __syncwarp();
+      double s = 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += buf[warp][lane >> 2][(lane & 3) * 8 + j];
+      s += __shfl_xor_sync(~0u, s, 1);
+      s += __shfl_xor_sync(~0u, s, 2);
+      if ((lane & 3) == 0) wsum[warp][k0 + (lane >> 2)] = s;
+      __syncwarp();
     }
     __syncthreads();
-    if (threadIdx.x < K) {
+    double* mine = part + ((size_t)(it & 1) * gridDim.x + blockIdx.x) * (K + 1);
+    for (int k = tid; k <= K; k += EM_NT) {
       double s = 0;
-      for (int w = 0; w < EM_NT / 32; ++w) s += part[w][threadIdx.x];
-      tot[threadIdx.x] = s;
+      for (int w = 0; w < NW; ++w) s += wsum[w][k];
+      __stcg(mine + k, s);
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && !bad) {
-      double Ag[T][T], Ae[T][T];
-      int k = 0;
-      for (int a = 0; a < T; ++a)
-        for (int b = a; b < T; ++b, ++k) {
-          Ag[a][b] = Ag[b][a] = tot[k];
-          Ae[a][b] = Ae[b][a] = tot[NS + k];
-        }
-      double Ng[T][T], Ne[T][T], ng = 0, ne = 0, dg = 0, de = 0;
-      const double inv_n = 1.0 / (double)n;
-      for (int a = 0; a < T; ++a)
-        for (int b = a; b < T; ++b) {
-          double sg = 0, se = 0;
-          for (int c = 0; c < T; ++c) {
-            double tg = 0, te = 0;
-            for (int e = 0; e < T; ++e) {
-              tg += Ag[c][e] * Vg[e][b];
-              te += Ae[c][e] * Ve[e][b];
-            }
-            sg += Vg[a][c] * tg;
-            se += Ve[a][c] * te;
+    if (gridDim.x > 1) {
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) {
+        atomicAdd(sync, 1ull);
+        const unsigned long long want = (unsigned long long)(it + 1) * gridDim.x;
+        const uint64_t t0 = global_ns();
+        while (*(volatile unsigned long long*)sync < want) {
+          if (*(volatile unsigned long long*)(sync + 1) || global_ns() - t0 > kWaitLimitNs) {
+            sync[1] = 1ull;
+            quit = 1;
+            break;
           }
-          Ng[a][b] = Ng[b][a] = Vg[a][b] + sg * inv_n;
-          Ne[a][b] = Ne[b][a] = Ve[a][b] + se * inv_n;
         }
-      for (int a = 0; a < T; ++a)
-        for (int b = 0; b < T; ++b) {
-          ng += Vg[a][b] * Vg[a][b];
-          ne += Ve[a][b] * Ve[a][b];
-          dg += (Ng[a][b] - Vg[a][b]) * (Ng[a][b] - Vg[a][b]);
-          de += (Ne[a][b] - Ve[a][b]) * (Ne[a][b] - Ve[a][b]);
-        }
-      const double rg = sqrt(dg) / fmax(sqrt(ng), 1e-12), re = sqrt(de) / fmax(sqrt(ne), 1e-12);
-      for (int a = 0; a < T; ++a)
-        for (int b = 0; b < T; ++b) {
-          Vg[a][b] = Ng[a][b];
-          Ve[a][b] = Ne[a][b];
-        }
-      if (rg < tol && re < tol) done = 1;
+        __threadfence();
+      }
     }
     __syncthreads();
+    if (quit) {
+      if (tid == 0) atomicExch(status, DEV_TIMEOUT);
+      break;
+    }
+    {
+      const double* all = part + (size_t)(it & 1) * gridDim.x * (K + 1);
+      for (int t = tid; t < 8 * (K + 1); t += EM_NT) {
+        const int g = t & 7, k = t >> 3;
+        double s = 0;
+        for (int b = g; b < (int)gridDim.x; b += 8) s += __ldcg(all + (size_t)b * (K + 1) + k);
+        sub[g][k] = s;
+      }
+    }
+    __syncthreads();
+    for (int k = tid; k <= K; k += EM_NT)
+      tot[k] = ((sub[0][k] + sub[1][k]) + (sub[2][k] + sub[3][k])) + ((sub[4][k] + sub[5][k]) + (sub[6][k] + sub[7][k]));
+    __syncthreads();
+    ++it;
+    if (tot[K] != 0.0) {
+      bad = 1;
+      break;
+    }
+    // T = A V, N = V + V A V / n, entry by entry; threads past T^2 take the other matrix
+    const int half = tid >= 64, e = tid & 63, a = e / T, b = e % T;
+    auto packed = [&](int x, int y) {
+      const int lo = x < y ? x : y, hi = x < y ? y : x;
+      return tot[half * NS + lo * T - lo * (lo - 1) / 2 + hi - lo];
+    };
+    if (e < T * T) {
+      double s = 0;
+      for (int c = 0; c < T; ++c) s = fma(packed(a, c), half ? Ve[c][b] : Vg[c][b], s);
+      (half ? Te : Tg)[a][b] = s;
+    }
+    __syncthreads();
+    if (e < T * T && a <= b) {
+      double s = 0;
+      for (int c = 0; c < T; ++c) s = half ? fma(Ve[a][c], Te[c][b], s) : fma(Vg[a][c], Tg[c][b], s);
+      const double v = (half ? Ve[a][b] : Vg[a][b]) + s * (1.0 / (double)n);
+      (half ? Ne : Ng)[a][b] = v;
+      (half ? Ne : Ng)[b][a] = v;
+    }
+    __syncthreads();
+    if (tid < 4) {  // squared norms of Vg, Ve and of their changes
+      double s = 0;
+      for (int x = 0; x < T; ++x)
+        for (int y = 0; y < T; ++y) {
+          const double o = (tid & 1) ? Ve[x][y] : Vg[x][y];
+          const double v = tid < 2 ? o : ((tid & 1) ? Ne[x][y] : Ng[x][y]) - o;
+          s = fma(v, v, s);
+        }
+      nrm[tid] = sqrt(s);
+    }
+    __syncthreads();
+    if (e < T * T) {
+      if (half) Ve[a][b] = Ne[a][b];
+      else Vg[a][b] = Ng[a][b];
+    }
+    if (tid == 0 && nrm[2] / fmax(nrm[0], 1e-12) < tol && nrm[3] / fmax(nrm[1], 1e-12) < tol) done = 1;
+    __syncthreads();
+    if (done) break;
   }
-  if (threadIdx.x < T * T) {
-    VgVe[threadIdx.x] = Vg[threadIdx.x / T][threadIdx.x % T];
-    VgVe[T * T + threadIdx.x] = Ve[threadIdx.x / T][threadIdx.x % T];
+  if (blockIdx.x != 0) return;
+  if (tid < T * T) {
+    VgVe[tid] = Vg[tid / T][tid % T];
+    VgVe[T * T + tid] = Ve[tid / T][tid % T];
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     info[0] = it;
     info[1] = done;
     info[2] = bad;
@@ -344,8 +416,24 @@ static void load_g(cbx_handle* h, const double* G, int64_t n, DevBuf<double>& Gd
 template <int T>
 static void launch_em(cbx_handle* h, const double* D, const double* R, int64_t n, int max_iter, double tol,
                       double* VgVe, int* info) {
-  k_mv_em<T><<<1, EM_NT, 0, h->stream>>>(D, R, n, max_iter, tol, VgVe, info);
+  const unsigned grid = gridn(n, EM_NT, h->num_sms);
+  DevBuf<double> part;
+  DevBuf<unsigned long long> sync;
+  part.resize((size_t)2 * grid * (T * (T + 1) + 1));
+  sync.resize(2);
+  sync.zero(h->stream);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(EM_NT);
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CBX_CUDA(cudaLaunchKernelEx(&cfg, k_mv_em<T>, D, R, n, max_iter, tol, VgVe, info, part.p, sync.p, h->status.p));
   h->launched("k_mv_em");
+  h->check_status("multi-trait EM");  // also waits: part and sync go out of scope
 }
 
 }  // namespace mt
