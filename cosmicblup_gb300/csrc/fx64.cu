@@ -164,6 +164,10 @@ struct Job {
   int m, n;          // output bounds (modes 1, 2)
   double* C;
   int64_t ldc;
+  // split sum (mode 1): nz slices of kper K steps, slice z writes C + z * cz
+  int nz, kper;
+  int64_t cz;
+  const int* active;  // nothing to do when it points to 0
 };
 struct Bars {
   uint64_t full[NSTAGE], empty[NSTAGE], acc_full, acc_empty, drain;
@@ -171,13 +175,24 @@ struct Bars {
   int abort;
 };
 
+// Tile t: row and column tile, the segment's cmin, and the K steps [k0, k1) it sums.
+struct Where {
+  int rt, ct, cmin, k0, k1, z;
+};
 template <int NT>
-__device__ __forceinline__ void tile_of(const Job& J, int t, int& rt, int& ct, int& cmin) {
+__device__ __forceinline__ Where tile_of(const Job& J, int t) {
   constexpr int CPT = 128 / NT;
+  Where o;
+  o.z = 0;
+  if (J.nz > 1) {
+    const int per = J.tiles / J.nz;
+    o.z = t / per;
+    t -= o.z * per;
+  }
   const int c0 = J.seg[0].count(CPT);
   const Seg& s = t < c0 ? J.seg[0] : J.seg[1];
   if (t >= c0) t -= c0;
-  cmin = s.cmin;
+  o.cmin = s.cmin;
   int x;
   if (s.tri) {
     // the root of upto(x) = t, then the exact row tile beside it
@@ -189,8 +204,11 @@ __device__ __forceinline__ void tile_of(const Job& J, int t, int& rt, int& ct, i
   } else {
     x = s.ra + t / (s.cb - s.ca);
   }
-  rt = x;
-  ct = s.ca + t - s.upto(CPT, x);
+  o.rt = x;
+  o.ct = s.ca + t - s.upto(CPT, x);
+  o.k0 = J.ktri ? 4 * x : J.ks0 + o.z * J.kper;
+  o.k1 = J.nz > 1 ? min(J.ks1, o.k0 + J.kper) : J.ks1;
+  return o;
 }
 // first block of a row tile in a panel's storage (triangular panels keep K steps >= 4 rt)
 __device__ __forceinline__ size_t blk_of(int rt, int ks, int stride, int tri) {
@@ -206,6 +224,7 @@ __device__ __forceinline__ size_t blk_of(int rt, int ks, int stride, int tri) {
 template <int NT>
 __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_constant__ Job J, int* status) {
   using T = Tile<NT>;
+  if (J.active && *J.active == 0) return;
   extern __shared__ uint8_t dsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
   Bars* bars = reinterpret_cast<Bars*>(smem + T::OFF_BAR);
@@ -241,9 +260,9 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
       uint32_t g = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
-        int rt, ct, cmin;
-        tile_of<NT>(J, t, rt, ct, cmin);
-        for (int k = J.ktri ? 4 * rt : J.ks0; k < J.ks1; ++k, ++g) {
+        const Where o = tile_of<NT>(J, t);
+        const int rt = o.rt, ct = o.ct;
+        for (int k = o.k0; k < o.k1; ++k, ++g) {
           const uint32_t s = g % NSTAGE;
           if (!mbar_wait(&bars->empty[s], ((g / NSTAGE) & 1) ^ 1, abort_flag)) { ok = false; break; }
           mbar_expect_tx(&bars->full[s], T::STAGE);
@@ -263,11 +282,9 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
       uint32_t g = 0, c = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
-        int rt, ct, cmin;
-        tile_of<NT>(J, t, rt, ct, cmin);
-        const int k0 = J.ktri ? 4 * rt : J.ks0;
-        for (int k = k0; k < J.ks1; ++k, ++g) {
-          const int ci = (k - k0) % CHUNK;
+        const Where o = tile_of<NT>(J, t);
+        for (int k = o.k0; k < o.k1; ++k, ++g) {
+          const int ci = (k - o.k0) % CHUNK;
           if (ci == 0) {
             if (!mbar_wait(&bars->acc_empty, (c & 1) ^ 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
@@ -293,7 +310,7 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
             }
           }
           umma_commit(&bars->empty[s]);
-          if (ci == CHUNK - 1 || k == J.ks1 - 1) {
+          if (ci == CHUNK - 1 || k == o.k1 - 1) {
             umma_commit(&bars->acc_full);
             ++c;
           }
@@ -312,10 +329,10 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
     uint32_t c = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < J.tiles && ok; t += gridDim.x) {
-      int rt, ct, cmin;
-      tile_of<NT>(J, t, rt, ct, cmin);
-      const int steps = J.ks1 - (J.ktri ? 4 * rt : J.ks0);
-      const int nch = (steps + CHUNK - 1) / CHUNK;
+      const Where o = tile_of<NT>(J, t);
+      const int rt = o.rt, ct = o.ct, cmin = o.cmin;
+      const int nch = (o.k1 - o.k0 + CHUNK - 1) / CHUNK;
+      double* const C = J.C + o.z * J.cz;
       const int rb = rt * 128 + q * 32, row = rb + lane, col0 = ct * NT + j0;
       const int ea = J.ea[row] - 66;  // 56 - 2 * 61
       const int el = J.eb[col0 + (lane & 15)];
@@ -416,7 +433,7 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
             const int rl = 4 * i + (lane >> 3), r = rb + rl;
             const double x =
                 *reinterpret_cast<const double*>(out + rl * 64 + (((col >> 1) ^ ((rl >> 1) & 3)) << 4) + (col & 1) * 8);
-            if (r < J.m && cc < J.n && (J.mode == 1 || cc <= r)) J.C[(int64_t)r * J.ldc + cc] = x;
+            if (r < J.m && cc < J.n && (J.mode == 1 || cc <= r)) C[(int64_t)r * J.ldc + cc] = x;
           }
         }
       }
@@ -479,6 +496,62 @@ __global__ void __launch_bounds__(128) k_digits(const double* __restrict__ src, 
       v[i] = (r < rows && kk < k) ? (trans ? src[kk * ld + r] : src[r * ld + kk]) : 0.0;
     }
     put_digits(v, e, blk, threadIdx.x, kg);
+  }
+}
+
+// Columns of an interleaved block as rows of an operand: element (c, k) is
+// X[(p + gmap[k]) * xs + c].  Exponents (columns from ncols on are zero), then digits.
+__global__ void __launch_bounds__(256) k_colexp(const double* __restrict__ X, int xs, int64_t p,
+                                                const int32_t* __restrict__ gmap, int64_t ng, int ncols,
+                                                int32_t* __restrict__ ex, const int* active) {
+  if (active && *active == 0) return;
+  __shared__ int red[8];
+  const int c = blockIdx.x;
+  int e = EX_MIN;
+  if (c < ncols)
+    for (int64_t k = threadIdx.x; k < ng; k += 256) {
+      const double v = X[(p + gmap[k]) * xs + c];
+      if (v != 0.0) e = max(e, expo(v));
+    }
+  e = __reduce_max_sync(~0u, e);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) e = max(e, red[i]);
+    ex[c] = e;
+  }
+}
+__global__ void __launch_bounds__(128) k_coldigits(const double* __restrict__ X, int xs, int64_t p,
+                                                   const int32_t* __restrict__ gmap, int64_t ng, int ncols, int ks,
+                                                   const int32_t* __restrict__ ex, uint8_t* __restrict__ dig,
+                                                   const int* active) {
+  if (active && *active == 0) return;
+  const int64_t total = (int64_t)ks * ncols * 4;
+  for (int64_t i = blockIdx.x * 128ll + threadIdx.x; i < total; i += gridDim.x * 128ll) {
+    const int c = (int)(i % ncols), kg = (int)(i / ncols & 3);
+    const int64_t st = i / (4 * ncols);
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int64_t k = st * 32 + kg * 8 + j;
+      v[j] = k < ng ? X[(p + gmap[k]) * xs + c] : 0.0;
+    }
+    put_digits(v, ex[c], dig + (size_t)st * BLK, c, kg);
+  }
+}
+// out[i * os + c] = the slices' sum in slice order for c < ncols, 0 for ncols <= c < oc
+__global__ void __launch_bounds__(256) k_slices(const double* __restrict__ part, int nz, int64_t cz, int ldp, int64_t ng,
+                                                int ncols, double* __restrict__ out, int os, int oc,
+                                                const int* active) {
+  if (active && *active == 0) return;
+  const int64_t total = ng * oc;
+  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+    const int64_t r = i / oc;
+    const int c = (int)(i - r * oc);
+    double s = 0.0;
+    if (c < ncols)
+      for (int z = 0; z < nz; ++z) s += part[z * cz + r * ldp + c];
+    out[r * os + c] = s;
   }
 }
 
@@ -823,7 +896,7 @@ static void launch_tiles(cbx_handle* h, Job J) {
     s.ca /= NT / 32;
     s.cb = (s.cb + NT / 32 - 1) / (NT / 32);
   }
-  J.tiles = J.seg[0].count(128 / NT) + J.seg[1].count(128 / NT);
+  J.tiles = (J.seg[0].count(128 / NT) + J.seg[1].count(128 / NT)) * std::max(1, J.nz);
   ensure_smem((const void*)k_fx64<NT>, Tile<NT>::SMEM, h->device);
   launch_pdl(h, k_fx64<NT>, dim3(std::min(J.tiles, h->num_sms)), Tile<NT>::THREADS, Tile<NT>::SMEM, J, h->status.p);
   h->launched("k_fx64");
@@ -871,6 +944,59 @@ void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int
   J.C = C;
   J.ldc = ldc;
   fx::launch(h, J);
+}
+
+void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,
+                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active) {
+  CBX_REQUIRE(ncols >= 1 && ncols <= 64 && ng <= (int64_t)Q.rt * 128, CBX_ERR_ARG, "bad block product");
+  cudaStream_t s = h->stream;
+  const int nt = ncols <= 32 ? 32 : 64;
+  if (V.dig.n < (size_t)Q.ks * fx::BLK) {  // rows past the columns hold finite digits
+    V.dig.resize((size_t)Q.ks * fx::BLK);
+    V.dig.zero(s);
+  }
+  fx::at_least(V.ex, 128);
+  V.rt = 1;
+  V.ks = Q.ks;
+  fx::k_colexp<<<nt, 256, 0, s>>>(X, xs, p, gmap, ng, ncols, V.ex.p, active);
+  h->launched("k_colexp");
+  const int64_t work = (int64_t)Q.ks * ncols * 4;
+  fx::k_coldigits<<<(unsigned)std::min<int64_t>((work + 127) / 128, 8 * h->num_sms), 128, 0, s>>>(
+      X, xs, p, gmap, ng, ncols, Q.ks, V.ex.p, V.dig.p, active);
+  h->launched("k_coldigits");
+  // K slices: as many as leave the last wave of row tiles x slices fullest, 8 K steps or more each
+  int nz = 1;
+  double best = 1e30;
+  for (int z = 1; z <= 32 && 8 * z <= std::max(8, Q.ks); ++z) {
+    const int64_t waves = ((int64_t)Q.rt * z + h->num_sms - 1) / h->num_sms;
+    const double cost = (double)waves / z + 0.01 * z;
+    if (cost < best) {
+      best = cost;
+      nz = z;
+    }
+  }
+  fx::Job J{};
+  J.kper = ((Q.ks + nz - 1) / nz + 3) / 4 * 4;
+  J.nz = (Q.ks + J.kper - 1) / J.kper;
+  J.cz = (int64_t)ng * nt;
+  fx::at_least(part, (size_t)J.nz * J.cz);
+  J.A = Q.dig.p;
+  J.B = V.dig.p;
+  J.ea = Q.ex.p;
+  J.eb = V.ex.p;
+  J.ka = J.kb = J.ks1 = Q.ks;
+  J.seg[0] = {0, Q.rt, 0, nt / 32, 0, 0};
+  J.mode = 1;
+  J.m = (int)ng;
+  J.n = ncols;
+  J.C = part.p;
+  J.ldc = nt;
+  J.active = active;
+  if (nt == 32) fx::launch_tiles<32>(h, J);
+  else fx::launch_tiles<64>(h, J);
+  fx::k_slices<<<(unsigned)std::min<int64_t>((ng * oc + 255) / 256, 8 * h->num_sms), 256, 0, s>>>(
+      part.p, J.nz, J.cz, nt, ng, ncols, out, os, oc, active);
+  h->launched("k_slices");
 }
 
 bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet) {

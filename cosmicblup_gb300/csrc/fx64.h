@@ -3,7 +3,9 @@
 // dense-AI paths.
 #pragma once
 #include <cstdint>
-#include "handle.h"
+#include "devbuf.h"
+
+struct cbx_handle;
 
 namespace cbx {
 
@@ -19,6 +21,12 @@ struct FxPanel {
 void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans);
 // C[i * ldc + j] = sum_k A(i, k) B(j, k) for i < m, j < n.
 void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int64_t n, double* C, int64_t ldc);
+
+// out[i * os + c] = sum_k Q(i, k) X[(p + gmap[k]) * xs + c] for i < ng, c < ncols <= 64, zero
+// for ncols <= c < oc.  Q holds the digits of the ng x ng block; V and part are scratch.
+// Does nothing while active (may be null) points to 0.
+void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,
+                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active);
 
 // Cholesky of the symmetric n x n matrix A (column-major, its lower triangle is
 // read).  Returns false when a pivot is not positive.  logdet (may be null) gets

@@ -432,14 +432,24 @@ constexpr int rpw_ff() {
 // Vt[c * ld + k] = X[(p + gmap[k]) * xs + c] for c < ncols, k < ng (the gathered
 // dense-block rows of an interleaved block, as columns of a column-major
 // ld x ncols matrix).
-__global__ void k_gather_cols(const double* __restrict__ X, int xs, int ncols, double* __restrict__ Vt, int64_t p,
-                              int64_t ng, int64_t ld, const int32_t* __restrict__ gmap) {
-  const int64_t total = (int64_t)ncols * ld;
+__global__ void k_gather_cols(const double* __restrict__ X, int xs, int ncols, int rows, double* __restrict__ Vt,
+                              int64_t p, int64_t ng, int64_t ld, const int32_t* __restrict__ gmap) {
+  const int64_t total = (int64_t)rows * ld;  // rows from ncols on are zero
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = idx / ld, k = idx - c * ld;
-    Vt[idx] = k < ng ? X[(p + gmap[k]) * xs + c] : 0.0;
+    Vt[idx] = c < ncols && k < ng ? X[(p + gmap[k]) * xs + c] : 0.0;
   }
+}
+
+// The FP64 solver's block product by digits (fx64.cu) from 2 columns and ng^2 columns =
+// kFx64From on: below, the CUDA-core product's FP64 issue (1.05 TFLOP/s) takes less than the
+// digit product's four launches (about 15 us).  Its digits take 16 bytes an entry: past
+// kFx64MaxNg (17 GB) the block stays on cuBLAS DGEMM.
+constexpr double kFx64From = 8e6;
+constexpr int64_t kFx64MaxNg = 32768;
+static bool use_fx64(int64_t ng, int ncols) {
+  return ncols >= 2 && ng <= kFx64MaxNg && (double)ng * ng * ncols > kFx64From;
 }
 
 // Float-float block products are FP32-issue-bound, so they run on the
@@ -520,8 +530,9 @@ static void ff_plan(cbx_handle* h, const sv::OpView<double>& op, const double* X
 // accuracy: float-float on the CUDA cores (ff), or cuBLAS DGEMM / DGEMV on the
 // gathered columns (the block is an ng x ng column-major matrix with leading
 // dimension ld; it is symmetric, so either orientation gives Qinv X).
-static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X, int S, int ncols, double* Vt,
-                    double* Tout, const int* active, bool ff, double* colsum) {
+template <int S>
+static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X, int ncols, double* Vt, double* Tout,
+                    const int* active, bool ff, double* colsum) {
   if (ff) {
     // the compensated FP64 column sums that restore the block's shift
     sv::k_colsum_x<<<ncols, 256, 0, h->stream>>>(X, S, op.p, op.ng, op.gmap, colsum);
@@ -558,20 +569,43 @@ static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X
     return;
   }
   cudaStream_t s = h->stream;
-  k_gather_cols<<<grid_for((int64_t)ncols * op.ld, 256, 4 * h->num_sms), 256, 0, s>>>(X, S, ncols, Vt, op.p, op.ng,
-                                                                                     op.ld, op.gmap);
+  if (use_fx64(op.ng, ncols)) {
+    Mme& mm = *h->mme;
+    if (!mm.fxQ_ok) {
+      fx64_digits(h, mm.fxQ, op.Qd, op.ld, op.ng, op.ng, false);
+      mm.fxQ_ok = true;
+    }
+    for (int c0 = 0; c0 < ncols; c0 += 64) {
+      const int nc = std::min(64, ncols - c0);
+      fx64_product(h, mm.fxQ, mm.fxV, mm.fxQ_part, X + c0, S, op.p, op.gmap, op.ng, nc, Tout + c0, S,
+                   c0 + nc < ncols ? nc : S - c0, active);
+    }
+    return;
+  }
+  k_gather_cols<<<grid_for((int64_t)S * op.ld, 256, 4 * h->num_sms), 256, 0, s>>>(X, S, ncols, S, Vt, op.p, op.ng,
+                                                                                 op.ld, op.gmap);
   h->launched("k_gather_cols<f64>");
+  if (ncols == 1 && S == 1) {
+    sv::k_gemv<double, 2, 4><<<(unsigned)((op.ng + 15) / 16), 256, 0, s>>>(op.Qd, op.ng, op.ld, Vt, Tout, active);
+    h->launched("k_gemv<f64>");
+    return;
+  }
+  if constexpr (S <= 64) {
+    if (op.ng <= kFx64MaxNg) {
+      constexpr int R = rpw<double, S>();
+      constexpr int smem = S * 32 * 2 * 4 * (int)sizeof(double);
+      ensure_smem((const void*)sv::k_dense<double, S, R>, smem, h->device);
+      sv::k_dense<double, S, R><<<(unsigned)((op.ng + 8 * R - 1) / (8 * R)), 256, smem, s>>>(op.Qd, op.ng, op.ld, Vt,
+                                                                                           Tout, active);
+      h->launched("k_dense<f64>");
+      return;
+    }
+  }
   Libs& L = libs(h);
   const double one = 1.0, zero = 0.0;
-  if (ncols == 1) {
-    // Tout[i * S] = sum_k Q(k, i) v(k)
-    CBX_BLAS(cublasDgemv(L.blas, CUBLAS_OP_T, (int)op.ng, (int)op.ng, &one, op.Qd, (int)op.ld, Vt, 1, &zero, Tout,
-                         S));
-  } else {
-    // Tout^T (ncols x ng, leading dimension S) = Vt^T (ncols x ng) * Q (ng x ng)
-    CBX_BLAS(cublasDgemm(L.blas, CUBLAS_OP_T, CUBLAS_OP_N, ncols, (int)op.ng, (int)op.ng, &one, Vt, (int)op.ld,
-                         op.Qd, (int)op.ld, &zero, Tout, S));
-  }
+  // Tout^T (ncols x ng, leading dimension S) = Vt^T (ncols x ng) * Q (ng x ng)
+  CBX_BLAS(cublasDgemm(L.blas, CUBLAS_OP_T, CUBLAS_OP_N, ncols, (int)op.ng, (int)op.ng, &one, Vt, (int)op.ld, op.Qd,
+                       (int)op.ld, &zero, Tout, S));
   h->launched("cublas_dgemm<f64>");
 }
 
@@ -663,11 +697,11 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       CBX_CUDA(cudaEventCreate(&pr.b));
       CBX_CUDA(cudaEventRecord(pr.a, s));
     }
-    if (ncols < S) {
+    if (ncols < S && (ff || op.ng > kFx64MaxNg || S > 64)) {
       CBX_CUDA(cudaMemsetAsync(w.Tout.p, 0, (size_t)op.ng * S * sizeof(double), s));
       CBX_CUDA(cudaMemsetAsync(w.colsum.p, 0, S * sizeof(double), s));
     }
-    dense64(h, op, X, S, ncols, w.Vt.p, w.Tout.p, active, ff, w.colsum.p);
+    dense64<S>(h, op, X, ncols, w.Vt.p, w.Tout.p, active, ff, w.colsum.p);
     if (h->prof_on) {
       CBX_CUDA(cudaEventRecord(pr.b, s));
       pr.bucket = 1;
@@ -754,10 +788,9 @@ void run_pcg(cbx_handle* h, Mme& m, const sv::OpView<T>& op, Workspace<T, S>& w,
   h->launched(sizeof(T) == 4 ? "k_scalar_init<f32>" : "k_scalar_init<f64>");
   CBX_CUDA(cudaMemcpyAsync(w.P.p, w.Z.p, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
   int host_active = 1;
-  // host check of the active-column count every CHECK iterations; the FP64
-  // block product is slow enough (and cannot skip finished blocks) to check
-  // after every iteration
-  const int CHECK = (sizeof(T) == 8 && op.Qd) ? 1 : 8;
+  // host check of the active-column count every CHECK iterations; cuBLAS's FP64
+  // block product cannot skip finished blocks, so it is checked after every iteration
+  const int CHECK = (sizeof(T) == 8 && op.Qd && op.ng > kFx64MaxNg && S > 1) ? 1 : 8;
   // FP32: one persistent cooperative kernel per iteration after the dense
   // product (pcg_fused.cuh); CHECK is even, so the direction is back in w.P
   // after every block of CHECK iterations
@@ -1159,9 +1192,9 @@ void pcg_solve(cbx_handle* h, double lam, int ncols, const double* B_cm, double*
   // 128-wide block when there are more than 64: its PCG bulk reads the FP32
   // block once per iteration for all of them (the tensor-core product takes at
   // most 80 populated columns), and the FP64-class refinement products run on
-  // the populated columns only.  The FP64 solver's product is FP64-bound, so it
-  // stays at 32.
-  const int chunk = precision != 0 ? (ncols > 64 ? 80 : 64) : 32;
+  // the populated columns only.  The FP64 solver's digit product takes 64; cuBLAS's
+  // is FP64-bound, so a block that is too large for digits stays at 32.
+  const int chunk = precision != 0 ? (ncols > 64 ? 80 : 64) : (m.has_dense && m.ng > kFx64MaxNg) ? 32 : 64;
   for (int c0 = 0; c0 < ncols; c0 += chunk) {
     const int nc = std::min(chunk, ncols - c0);
     PcgResult r;
@@ -1667,6 +1700,10 @@ extern "C" int cbx_mme_create(cbx_handle* h, int64_t n_rec, int64_t p, int64_t q
       m->ld = o.ld;
       m->qshift = o.qshift;
       m->fx_rows_ok = o.fx_rows_ok;
+      m->fxQ = std::move(o.fxQ);
+      m->fxV = std::move(o.fxV);
+      m->fxQ_part = std::move(o.fxQ_part);
+      m->fxQ_ok = o.fxQ_ok;
       m->planes_src = o.planes_src;
       m->planes_gen = o.planes_gen;
       if (o.dim == m->dim)
@@ -1737,6 +1774,7 @@ static void upload_dense(cbx_handle* h, Mme& m, const double* src, int64_t ng, i
                                                                        m.Qlo32.p);
   h->launched("k_lowp_block");
   m.fx_rows_ok = false;
+  m.fxQ_ok = false;
   if (use_bf16() && m.ld % 8 == 0) {
     m.Qbf.resize((size_t)ng * m.ld);
     dense_bf_block(h, m.Qd64.p, ng, m.ld, m.qshift, m.Qbf.p);
