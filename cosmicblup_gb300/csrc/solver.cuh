@@ -593,15 +593,25 @@ __device__ __forceinline__ double block_sum_cols(double v, double* red /*[NT]*/)
   }
 }
 
-// red[tid] summed over the groups tid / S of an N-thread block, by halves in a fixed order;
-// the totals are in red[0 .. S).  One thread per column adding N / S values in turn took
-// 35 us in FP64 (68 clocks an addition) where S is 1.
+// red[tid] summed over the groups tid / S of an N-thread block in a fixed order; the totals
+// are in red[0 .. S).  Narrow blocks have many groups and sum them by halves: one thread
+// per column adding N / S values in turn took 35 us in FP64 (68 clocks an addition) where S
+// is 1.  Wide ones add their few groups in turn.
 template <typename T, int S, int N>
-__device__ __forceinline__ void tree_sum_cols(T* red) {
+__device__ __forceinline__ void sum_groups(T* red) {
+  if constexpr (S < 32) {
 #pragma unroll
-  for (int o = N / 2; o >= S; o >>= 1) {
+    for (int o = N / 2; o >= S; o >>= 1) {
+      __syncthreads();
+      if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    }
+  } else {
     __syncthreads();
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (threadIdx.x < S) {
+      T s = T(0);
+      for (int g = 0; g < N / S; ++g) s += red[g * S + threadIdx.x];
+      red[threadIdx.x] = s;
+    }
   }
   __syncthreads();
 }
@@ -632,7 +642,7 @@ __global__ void __launch_bounds__(NT) k_fix_seg(OpView<T> op, const int32_t* __r
   }
   for (; j < hi; j += G) acc[0] += op.Dval[j] * X[(int64_t)op.Dcol[j] * S + c];
   redT[tid] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-  tree_sum_cols<T, S, NT>(redT);
+  sum_groups<T, S, NT>(redT);
   if (tid < S) seg_part[(int64_t)sg * S + tid] = redT[tid];
   (void)seg_row;
 }
@@ -849,7 +859,7 @@ __global__ void __launch_bounds__(NT) k_spmv(OpView<T> op, const T* __restrict__
     if (use_D && c < ncp)
       for (int32_t k = fix_seg_ptr[i] + g; k < fix_seg_ptr[i + 1]; k += GS) s += seg_part[(int64_t)k * S + c];
     redT[tid] = s;
-    tree_sum_cols<T, S, NT>(redT);
+    sum_groups<T, S, NT>(redT);
     if (tid >= ncp && tid < S) Y[i * S + tid] = T(0);  // defined, never read
     if (tid < ncp) {
       const T t = redT[tid];
@@ -931,7 +941,7 @@ __global__ void __launch_bounds__(NT_FIXED) k_fixed(OpView<T> op, const T* __res
   const int64_t kend = (col == nullptr || col[c].active) ? op.p : 0;  // inactive columns: nothing to do
   for (int64_t k = g; k < kend; k += G) acc += op.A11inv[f * op.p + k] * R[k * S + c];
   redT[tid] = acc;
-  tree_sum_cols<T, S, NT_FIXED>(redT);
+  sum_groups<T, S, NT_FIXED>(redT);
   if (tid < S) {
     const T s = redT[tid];
     const bool act = col == nullptr || col[tid].active;
