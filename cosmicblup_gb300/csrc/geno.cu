@@ -29,17 +29,10 @@
 // sample, k (w2_j - w0_j) and, where both bits are set, w3_j - 2 w2_j + w0_j (w_c =
 // the float term of code c, which is not linear in x); a missing call then receives
 // w2_j, which the sample-major missing list takes back out.  Missing calls are rare
-// in genotype data: the dense passes cost a few integer operations per code, the
-// sparse ones one gather per missing call.
+// in genotype data: the sparse passes cost one gather per missing call.
 //
-// The k-weighted sums run on the integer multiply path instead of as masked adds.
-// For one 32-bit word of 16 codes, kw = (w & 0x55..) + ((w >> 1) & 0x55..) holds the
-// k_t in 2-bit fields, and with a_t = kw >> 2t (so that k_t = a_t - 4 a_{t+1}, a_16 = 0)
-//   sum_t k_t v_t = sum_t a_t (v_t - 4 v_{t-1})      (v_{-1} = 0),
-// one 32 x 64-bit multiply-add per code against u_t = v_t - 4 v_{t-1}, precomputed per
-// 16-sample word; modulo 2^64 it is two multiply-adds (the low word widening, the high
-// word 32-bit).  Z v telescopes over the accumulators instead: P_t = sum_j a_t(j) d_j
-// gives sum_j k_t(j) d_j = P_t - 4 P_{t+1}.
+// The k-weighted sums run on the tensor cores as sums of six balanced base-2048 digits of
+// the fixed-point values (k_geno_zt, k_geno_z).
 //
 // Layout: the payload is copied once into rows of `pitch` bytes (a multiple of 16,
 // the padding bytes zero).  Samples at or beyond n get v = 0 (Z^T v) or are dropped
@@ -49,6 +42,7 @@
 #include <cmath>
 #include <vector>
 #include <cublas_v2.h>
+#include <cuda_fp16.h>
 #include "dense.h"
 #include "handle.h"
 #include "pcg.h"
@@ -57,9 +51,9 @@
 namespace cbx {
 namespace geno {
 
-constexpr int ZT_THREADS = 256;   // one SNP row per thread
-constexpr int Z_THREADS = 256;    // 16 samples (one 32-bit word) per thread
-constexpr int Z_MAX_ROWS = 2048;  // SNP rows per CTA (48 KB of deltas in shared memory)
+constexpr int ZT_THREADS = 256;   // 32 SNP rows per warp
+constexpr int Z_THREADS = 256;    // 256 samples per warp
+constexpr int Z_MAX_ROWS = 4096;  // SNP rows per CTA
 constexpr int PREP_THREADS = 1024;
 
 // Deterministic block sum of a double (fixed shuffle tree, then warp 0 over the warps).
@@ -243,79 +237,112 @@ __global__ void k_geno_miss_transpose(const int64_t* __restrict__ ptr, const int
   }
 }
 
+// This lane's share of the sum of x[list[k]], lo <= k < hi: eight gathers in flight.
+__device__ __forceinline__ unsigned long long gather_sum(const int32_t* __restrict__ list, int64_t lo, int64_t hi,
+                                                         const long long* __restrict__ x, int lane) {
+  unsigned long long s[8] = {};
+  int64_t k = lo + lane;
+  for (; k + 7 * 32 < hi; k += 8 * 32) {
+    int32_t e[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e[u] = list[k + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s[u] += (unsigned long long)x[e[u]];
+  }
+  for (; k < hi; k += 32) s[0] += (unsigned long long)x[list[k]];
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
 // M_j = sum of V over SNP j's missing calls, into acc[m + j] (one warp per SNP).
 __global__ void k_geno_miss_zt(const int64_t* __restrict__ ptr, const int32_t* __restrict__ snp_list, int64_t m,
                                const long long* __restrict__ V, unsigned long long* __restrict__ acc) {
   const int lane = threadIdx.x & 31;
   const int64_t j = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (j >= m) return;
-  unsigned long long s = 0;
-  for (int64_t k = ptr[j] + lane; k < ptr[j + 1]; k += 32) s += (unsigned long long)V[snp_list[k]];
+  unsigned long long s = gather_sum(snp_list, ptr[j], ptr[j + 1], V, lane);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) acc[m + j] = s;
 }
 
-// Takes the missing calls' spurious terms back out of Z v: acc[i] -= sum of D[3j + 2]
-// over the SNPs j where sample i is missing (one warp per sample).
+// Takes the missing calls' spurious terms back out of Z v: acc[i] -= sum of W2[j] over the SNPs j where sample i is missing (one warp per sample).
 __global__ void k_geno_miss_z(const int64_t* __restrict__ samp_ptr, const int32_t* __restrict__ samp_list,
-                              int64_t n, const long long* __restrict__ D, unsigned long long* __restrict__ acc) {
+                              int64_t n, const long long* __restrict__ W2, unsigned long long* __restrict__ acc) {
   const int lane = threadIdx.x & 31;
   const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= n) return;
-  unsigned long long s = 0;
-  for (int64_t k = samp_ptr[i] + lane; k < samp_ptr[i + 1]; k += 32)
-    s += (unsigned long long)D[3 * (int64_t)samp_list[k] + 2];
+  unsigned long long s = gather_sum(samp_list, samp_ptr[i], samp_ptr[i + 1], W2, lane);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) acc[i] -= s;
 }
 
-// v (n, FP64) -> V (n_pad, int64 at scale 2^s) and U_i = V_i - 4 V_{i-1} within each
-// 16-sample word (V_{i-1} = 0 at a word's first sample); meta[0] = s, meta[1] = T = sum V.
-__global__ void __launch_bounds__(PREP_THREADS) k_geno_vprep(const double* __restrict__ v, int64_t n,
-                                                            int64_t n_pad, long long* __restrict__ V,
-                                                            long long* __restrict__ U,
-                                                            long long* __restrict__ meta, int* status) {
+// Blocks of the two-pass preparations: partial sums of one per block, added in block order.
+constexpr int PREP_BLOCKS = 128;
+constexpr int PREP_NT = 256;
+
+__device__ double sum_parts(const double* part, double* red) {
+  return block_sum_f64(threadIdx.x < PREP_BLOCKS ? part[threadIdx.x] : 0.0, red);
+}
+// sum of the blocks' integer partials, in every thread
+__device__ unsigned long long all_sum_u64(const unsigned long long* part) {
+  __shared__ unsigned long long red[32], tot;
+  const unsigned long long t = block_sum_u64(threadIdx.x < PREP_BLOCKS ? part[threadIdx.x] : 0ull, red);
+  if (threadIdx.x == 0) tot = t;
+  __syncthreads();
+  return tot;
+}
+
+// Sums of |v| per block.
+__global__ void __launch_bounds__(PREP_NT) k_geno_vsum(const double* __restrict__ v, int64_t n,
+                                                      double* __restrict__ part) {
   __shared__ double red[32];
-  __shared__ unsigned long long redu[32];
-  __shared__ int s_sh;
   double a = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) a += fabs(v[i]);
+  for (int64_t i = blockIdx.x * (int64_t)PREP_NT + threadIdx.x; i < n; i += PREP_BLOCKS * (int64_t)PREP_NT)
+    a += fabs(v[i]);
   a = block_sum_f64(a, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = a;
+}
+// The scale exponent of the sum of the partials; a non-finite one sets the status.
+__device__ int scale_of(const double* part, long long* meta, int* status) {
+  __shared__ double red[32];
+  __shared__ int s_sh;
+  const double a = sum_parts(part, red);
   if (threadIdx.x == 0) {
-    int s = 0;
-    if (!isfinite(a)) atomicExch(status, DEV_NONFINITE);
-    else s = fix_exponent(a);
-    s_sh = s;
-    meta[0] = s;
+    const bool ok = isfinite(a);
+    s_sh = ok ? fix_exponent(a) : 0;
+    if (blockIdx.x == 0) {
+      if (!ok) atomicExch(status, DEV_NONFINITE);
+      meta[0] = s_sh;
+    }
   }
   __syncthreads();
-  const int s = s_sh;
+  return s_sh;
+}
+// v (n, FP64) -> V (n_pad, int64 at scale 2^s, zero past n) and their sums per block;
+// meta[0] = s.
+__global__ void __launch_bounds__(PREP_NT) k_geno_vprep(const double* __restrict__ v, int64_t n, int64_t n_pad,
+                                                       const double* __restrict__ part, long long* __restrict__ V,
+                                                       unsigned long long* __restrict__ tpart,
+                                                       long long* __restrict__ meta, int* status) {
+  __shared__ unsigned long long redu[32];
+  const int s = scale_of(part, meta, status);
   unsigned long long t = 0;
-  for (int64_t i = threadIdx.x; i < n_pad; i += blockDim.x) {
+  for (int64_t i = blockIdx.x * (int64_t)PREP_NT + threadIdx.x; i < n_pad; i += PREP_BLOCKS * (int64_t)PREP_NT) {
     const long long x = i < n ? __double2ll_rn(ldexp(v[i], s)) : 0ll;
-    const long long xp = (i % 16) && i - 1 < n ? __double2ll_rn(ldexp(v[i - 1], s)) : 0ll;
     V[i] = x;
-    U[i] = (long long)((unsigned long long)x - 4ull * (unsigned long long)xp);
     t += (unsigned long long)x;
   }
   t = block_sum_u64(t, redu);
-  if (threadIdx.x == 0) meta[1] = (long long)t;
+  if (threadIdx.x == 0) tpart[blockIdx.x] = t;
 }
 
-// Per-SNP float terms of multiply_Z_v (plink_reader.cpp:258-270) -> int64 values
-// at scale 2^s: D[3j..3j+2] = (W2 - W0 per unit of k, W3 - 2 W2 + W0 where both bits
-// are set, W2 = the spurious term of a missing call); meta[0] = s, meta[1] =
-// C = sum_j W0_j (added to every sample).  w (3m floats) is scratch.
-__global__ void __launch_bounds__(PREP_THREADS) k_geno_zprep(const double* __restrict__ v,
-                                                            const double* __restrict__ mean,
-                                                            const double* __restrict__ inv_std, int64_t m,
-                                                            float* __restrict__ w, long long* __restrict__ D,
-                                                            long long* __restrict__ meta, int* status) {
+// Float terms of multiply_Z_v per SNP (plink_reader.cpp:258-270), w[3j..], and the sums of
+// their largest magnitudes per block.
+__global__ void __launch_bounds__(PREP_NT) k_geno_zterms(const double* __restrict__ v, const double* __restrict__ mean,
+                                                        const double* __restrict__ inv_std, int64_t m,
+                                                        float* __restrict__ w, double* __restrict__ part) {
   __shared__ double red[32];
-  __shared__ unsigned long long redu[32];
-  __shared__ int s_sh;
   double a = 0.0;
-  for (int64_t j = threadIdx.x; j < m; j += blockDim.x) {
+  for (int64_t j = blockIdx.x * (int64_t)PREP_NT + threadIdx.x; j < m; j += PREP_BLOCKS * (int64_t)PREP_NT) {
     float w0 = 0.f, w2 = 0.f, w3 = 0.f;
     const double is = inv_std[j];
     if (is != 0.0) {
@@ -331,128 +358,228 @@ __global__ void __launch_bounds__(PREP_THREADS) k_geno_zprep(const double* __res
     a += (double)fmaxf(fabsf(w0), fmaxf(fabsf(w2), fabsf(w3)));
   }
   a = block_sum_f64(a, red);
-  if (threadIdx.x == 0) {
-    int s = 0;
-    if (!isfinite(a)) atomicExch(status, DEV_NONFINITE);
-    else s = fix_exponent(a);
-    s_sh = s;
-    meta[0] = s;
-  }
-  __syncthreads();
-  const int s = s_sh;
+  if (threadIdx.x == 0) part[blockIdx.x] = a;
+}
+// Their int64 values at scale 2^s: D[2j], D[2j + 1] = W2 - W0 per unit of k, W3 - 2 W2 + W0
+// where both bits are set; D[2m + j] = W2, the spurious term of a missing call; meta[0] = s,
+// and the sums of W0 (added to every sample) per block.
+__global__ void __launch_bounds__(PREP_NT) k_geno_zprep(const float* __restrict__ w, int64_t m,
+                                                       const double* __restrict__ part, long long* __restrict__ D,
+                                                       unsigned long long* __restrict__ cpart,
+                                                       long long* __restrict__ meta, int* status) {
+  __shared__ unsigned long long redu[32];
+  const int s = scale_of(part, meta, status);
   unsigned long long c = 0;
-  for (int64_t j = threadIdx.x; j < m; j += blockDim.x) {
+  for (int64_t j = blockIdx.x * (int64_t)PREP_NT + threadIdx.x; j < m; j += PREP_BLOCKS * (int64_t)PREP_NT) {
     const long long W0 = __double2ll_rn(ldexp((double)w[3 * j], s));
     const long long W2 = __double2ll_rn(ldexp((double)w[3 * j + 1], s));
     const long long W3 = __double2ll_rn(ldexp((double)w[3 * j + 2], s));
-    D[3 * j] = W2 - W0;
-    D[3 * j + 1] = W3 - 2 * W2 + W0;
-    D[3 * j + 2] = W2;
+    D[2 * j] = W2 - W0;
+    D[2 * j + 1] = W3 - 2 * W2 + W0;
+    D[2 * m + j] = W2;
     c += (unsigned long long)W0;
   }
   c = block_sum_u64(c, redu);
-  if (threadIdx.x == 0) meta[1] = (long long)c;
+  if (threadIdx.x == 0) cpart[blockIdx.x] = c;
 }
 
-// sum_t k_t V_t for one 32-bit word of 16 codes against u = U of its 16 samples
-// (the telescoped form above): lo accumulates the low words' 64-bit products, hi
-// the high words' products modulo 2^32.
-__device__ __forceinline__ void kdot16(uint32_t w, const uint2* __restrict__ u, unsigned long long& lo,
-                                       uint32_t& hi) {
-  const uint32_t kw = (w & 0x55555555u) + ((w >> 1) & 0x55555555u);
-#pragma unroll
-  for (int t = 0; t < 16; ++t) {
-    const uint32_t at = kw >> (2 * t);
-    const uint2 x = u[t];
-    lo += (unsigned long long)at * x.x;
-    hi += at * x.y;
+// ---- products on the tensor cores ---------------------------------------------
+// A fixed-point value is cut into six balanced base-2048 digits (|d| <= 1024, exact in
+// f16; the top one holds the sign).  A 2-bit field is an f16 as it stands: the bit patterns
+// 0, 1, 2, 3 are the subnormals 0, 1, 2, 3 times 2^-24.  So codes become operands of
+// mma.m16n8k16 (f16, FP32 accumulation) with one shift and one mask for two of them, the six
+// digits are columns of the other operand, and the accumulators are exact integers times
+// 2^-24 while a chunk's sum of magnitudes stays below 2^24: 5,461 terms of at most 3,072.
+// Each chunk's digits are put together modulo 2^64 and added to the totals, so results do
+// not depend on the order.  The codes are decoded in registers and used in place, which a
+// tile staged in shared memory for tcgen05 would write and read twice.
+constexpr int NDIG = 6;
+
+__device__ __forceinline__ int digit_of(long long x, int j) {
+  constexpr unsigned long long bias = 1024ull * (1ull + (1ull << 11) + (1ull << 22) + (1ull << 33) + (1ull << 44));
+  const unsigned long long g = (unsigned long long)x + bias;
+  return j < 5 ? (int)((g >> (11 * j)) & 2047) - 1024 : j == 5 ? (int)((long long)g >> 55) : 0;
+}
+__device__ __forceinline__ uint32_t digit_pair(long long lo, long long hi, int j) {
+  return (uint32_t)__half_as_ushort(__int2half_rn(digit_of(lo, j))) |
+         (uint32_t)__half_as_ushort(__int2half_rn(digit_of(hi, j))) << 16;
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the digits of two columns of one row, as one integer; summed over the quad's columns
+__device__ __forceinline__ unsigned long long total_of(float c0, float c1, int t) {
+  unsigned long long s = 0;
+  if (t < 3)
+    s = ((unsigned long long)(long long)__float2int_rn(c0 * 0x1p24f) << (22 * t)) +
+        ((unsigned long long)(long long)__float2int_rn(c1 * 0x1p24f) << (22 * t + 11));
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s;
+}
+
+// Digits of V as the second operand of Z^T v: entry ((seg 4 + q) 4 + i) 32 + lane holds
+// column lane / 4 of samples base + {2i, 2i + 8} and base + {2i + 1, 2i + 9}, base = 256 seg +
+// 64 (lane % 4) + 16 q: the order in which k_geno_zt meets them.
+__global__ void __launch_bounds__(256) k_geno_vdig(const long long* __restrict__ V, int64_t n_pad, int64_t total,
+                                                   uint2* __restrict__ B) {
+  for (int64_t e = blockIdx.x * 256ll + threadIdx.x; e < total; e += gridDim.x * 256ll) {
+    const int lane = (int)(e & 31), i = (int)(e >> 5 & 3), q = (int)(e >> 7 & 3), j = lane >> 2;
+    const int64_t base = (e >> 9) * 256 + 64 * (lane & 3) + 16 * q + 2 * i;
+    uint2 o = make_uint2(0u, 0u);
+    if (j < NDIG && base < n_pad) {
+      o.x = digit_pair(V[base], V[base + 8], j);
+      o.y = digit_pair(V[base + 1], V[base + 9], j);
+    }
+    B[e] = o;
   }
 }
 
-// Z^T v: one SNP row per thread over a chunk of CHUNK samples (2,048 to 8,192, a
-// tuned launch shape).  The chunk's U sits in shared memory and is read as
-// broadcasts; each thread streams its own row 16 bytes (64 samples) at a time.
-// acc[row] += S (64-bit atomics).
-template <int CHUNK>
-__global__ void __launch_bounds__(ZT_THREADS) k_geno_zt(const uint8_t* __restrict__ bed, int64_t pitch,
-                                                       int64_t m, const long long* __restrict__ U,
+// Z^T v: a warp takes 32 SNP rows and a chunk of samples, 256 at a time: each lane loads
+// 64 samples (16 bytes) of four rows, and 16 MMAs a row pair use them.  acc[row] += sum of
+// k V (64-bit atomics).  Bound by mma.sync, at its legacy rate of about 280 multiply-adds a clock
+// and SM: at n = 20,000, m = 50,000 0.10 ms (0.20 ms as two integer multiply-adds a code).
+constexpr int ZT_ROWS = 32 * (ZT_THREADS / 32);
+__global__ void __launch_bounds__(ZT_THREADS) k_geno_zt(const uint8_t* __restrict__ bed, int64_t pitch, int64_t m,
+                                                       int segs_per_cta, const uint2* __restrict__ B,
                                                        unsigned long long* __restrict__ acc) {
-  __shared__ __align__(16) long long su[CHUNK];
-  const int64_t c0 = (int64_t)blockIdx.y * CHUNK;
-  const int len = (int)std::min<int64_t>(CHUNK, 4 * pitch - c0);  // multiple of 64
-  for (int i = threadIdx.x; i < len; i += ZT_THREADS) su[i] = U[c0 + i];
-  __syncthreads();
-  const int64_t row = (int64_t)blockIdx.x * ZT_THREADS + threadIdx.x;
-  if (row >= m) return;
-  const uint4* p = reinterpret_cast<const uint4*>(bed + row * pitch + c0 / 4);
-  const uint2* u = reinterpret_cast<const uint2*>(su);
-  unsigned long long lo = 0;
-  uint32_t hi = 0;
-  const int nv = len / 64;  // 16-byte words of this row in the chunk
-  for (int k = 0; k < nv; ++k) {
-    const uint4 a = __ldg(p + k);
-    kdot16(a.x, u + 64 * k, lo, hi);
-    kdot16(a.y, u + 64 * k + 16, lo, hi);
-    kdot16(a.z, u + 64 * k + 32, lo, hi);
-    kdot16(a.w, u + 64 * k + 48, lo, hi);
-  }
-  atomicAdd(acc + row, lo + ((unsigned long long)hi << 32));
-}
-
-// Z v: 16 samples per thread (one 32-bit word per row, 128 coalesced bytes per
-// warp), looping over a chunk of SNP rows whose values sit in shared memory.
-// Per sample t: P_t = sum_j (kw_j >> 2t) D[3j] (telescoped, split into a 64-bit low
-// and a 32-bit high accumulator) and Q_t = sum of D[3j+1] where both bits are set;
-// acc[t] += P_t - 4 P_{t+1} + Q_t (64-bit atomics, one word per sample of n_pad).
-__global__ void __launch_bounds__(Z_THREADS) k_geno_z(const uint8_t* __restrict__ bed, int64_t pitch,
-                                                     int64_t m, int rows_per_cta,
-                                                     const long long* __restrict__ D,
-                                                     unsigned long long* __restrict__ acc) {
-  extern __shared__ __align__(16) long long sd[];
-  const int64_t r0 = (int64_t)blockIdx.y * rows_per_cta;
-  const int nr = (int)std::min<int64_t>(rows_per_cta, m - r0);
-  for (int i = threadIdx.x; i < 3 * nr; i += Z_THREADS) sd[i] = D[3 * r0 + i];
-  __syncthreads();
-  const int64_t byte_off = ((int64_t)blockIdx.x * Z_THREADS + threadIdx.x) * 4;
-  if (byte_off >= pitch) return;
-  const uint8_t* p = bed + r0 * pitch + byte_off;
-  unsigned long long P[16], Q[16];
-  uint32_t H[16];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t row0 = (int64_t)blockIdx.x * ZT_ROWS + (threadIdx.x >> 5) * 32;
+  if (row0 >= m) return;
+  const int64_t segs = (pitch + 63) / 64;
+  const int64_t s0 = (int64_t)blockIdx.y * segs_per_cta, s1 = std::min<int64_t>(segs, s0 + segs_per_cta);
+  float c[2][4] = {};
+  for (int64_t sg = s0; sg < s1; ++sg) {
+    const int64_t off = sg * 64 + 16 * t;
+    uint4 w[4];
 #pragma unroll
-  for (int t = 0; t < 16; ++t) { P[t] = 0; Q[t] = 0; H[t] = 0; }
-#pragma unroll 2
-  for (int r = 0; r < nr; ++r) {
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p + (int64_t)r * pitch));
-    const unsigned long long d1 = (unsigned long long)sd[3 * r];
-    const unsigned long long d2 = (unsigned long long)sd[3 * r + 1];
-    const uint32_t d1l = (uint32_t)d1, d1h = (uint32_t)(d1 >> 32);
-    const uint32_t kw = (w & 0x55555555u) + ((w >> 1) & 0x55555555u);
-    const uint32_t both = w & (w >> 1);
+    for (int r = 0; r < 4; ++r) {
+      const int64_t row = row0 + g + 8 * r;
+      w[r] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < m && off < pitch) w[r] = __ldg(reinterpret_cast<const uint4*>(bed + row * pitch + off));
+    }
+    const uint2* bp = B + sg * 512 + lane;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const uint32_t at = kw >> (2 * t);
-      P[t] += (unsigned long long)at * d1l;
-      H[t] += at * d1h;
-      if (both & (1u << (2 * t))) Q[t] += d2;
+    for (int q = 0; q < 4; ++q) {
+      uint32_t kw[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t x = q == 0 ? w[r].x : q == 1 ? w[r].y : q == 2 ? w[r].z : w[r].w;
+        kw[r] = (x & 0x55555555u) + ((x >> 1) & 0x55555555u);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint2 b = __ldg(bp + (q * 4 + i) * 32);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          mma_f16(c[h], (kw[2 * h] >> (4 * i)) & 0x00030003u, (kw[2 * h + 1] >> (4 * i)) & 0x00030003u,
+                  (kw[2 * h] >> (4 * i + 2)) & 0x00030003u, (kw[2 * h + 1] >> (4 * i + 2)) & 0x00030003u, b.x, b.y);
+      }
     }
   }
-  const int64_t i0 = byte_off * 4;
 #pragma unroll
-  for (int t = 0; t < 16; ++t) {
-    const unsigned long long pt = P[t] + ((unsigned long long)H[t] << 32);
-    const unsigned long long pn = t < 15 ? P[t + 1] + ((unsigned long long)H[t + 1] << 32) : 0ull;
-    atomicAdd(acc + i0 + t, pt - 4ull * pn + Q[t]);
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const unsigned long long s = total_of(c[h][2 * k], c[h][2 * k + 1], t);
+      const int64_t row = row0 + 16 * h + 8 * k + g;
+      if (t == 0 && row < m) atomicAdd(acc + row, s);
+    }
+}
+
+// Digits of D as the second operand of Z v: entry blk 32 + lane holds column lane / 4 of
+// the SNPs 16 blk + {2t, 2t + 1} and {2t + 8, 2t + 9} (t = lane % 4), of D[2j] and then of
+// D[2j + 1].
+__global__ void __launch_bounds__(256) k_geno_zdig(const long long* __restrict__ D, int64_t m, int64_t total,
+                                                   uint4* __restrict__ B) {
+  for (int64_t e = blockIdx.x * 256ll + threadIdx.x; e < total; e += gridDim.x * 256ll) {
+    const int lane = (int)(e & 31), j = lane >> 2;
+    const int64_t r = (e >> 5) * 16 + 2 * (lane & 3);
+    auto d = [&](int64_t row, int k) { return row < m ? D[2 * row + k] : 0ll; };
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if (j < NDIG) {
+      o.x = digit_pair(d(r, 0), d(r + 1, 0), j);
+      o.y = digit_pair(d(r + 8, 0), d(r + 9, 0), j);
+      o.z = digit_pair(d(r, 1), d(r + 1, 1), j);
+      o.w = digit_pair(d(r + 8, 1), d(r + 9, 1), j);
+    }
+    B[e] = o;
   }
+}
+
+// Z v: a warp takes 256 samples (two words of 16 per lane group) and a chunk of SNPs, 16
+// at a time: lane (g, t) holds the words of SNPs 2t, 2t + 1, 2t + 8, 2t + 9, whose halves
+// pair up to samples 0-7 and 8-15 of two SNPs; MMA i multiplies samples i and i + 8 of
+// eight words.  A second MMA adds the term of codes with both bits set.  acc[i] += the
+// sum (64-bit atomics).  Bound by mma.sync's rate: at n = 20,000, m = 50,000
+// 0.20 ms (0.52 ms as integer multiply-adds).
+constexpr int Z_SAMPLES = 256 * (Z_THREADS / 32);
+__global__ void __launch_bounds__(Z_THREADS) k_geno_z(const uint8_t* __restrict__ bed, int64_t pitch, int64_t m,
+                                                     int blks_per_cta, const uint4* __restrict__ B,
+                                                     unsigned long long* __restrict__ acc) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t off = (int64_t)blockIdx.x * (Z_SAMPLES / 4) + (threadIdx.x >> 5) * 64 + 8 * g;
+  const int64_t blks = (m + 15) / 16;
+  const int64_t b0 = (int64_t)blockIdx.y * blks_per_cta, b1 = std::min<int64_t>(blks, b0 + blks_per_cta);
+  if (off - 8 * g >= pitch) return;
+  float c[2][8][4] = {};
+  for (int64_t blk = b0; blk < b1; ++blk) {
+    uint2 w[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t row = blk * 16 + 2 * t + (r & 1) + 8 * (r >> 1);
+      w[r] = make_uint2(0u, 0u);
+      if (row < m && off < pitch) w[r] = __ldg(reinterpret_cast<const uint2*>(bed + row * pitch + off));
+    }
+    const uint4 b = __ldg(B + blk * 32 + lane);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint32_t kw[4], bo[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t x = q == 0 ? w[r].x : w[r].y;
+        kw[r] = (x & 0x55555555u) + ((x >> 1) & 0x55555555u);
+        bo[r] = x & (x >> 1) & 0x55555555u;
+      }
+      const uint32_t k0 = __byte_perm(kw[0], kw[1], 0x5410), k1 = __byte_perm(kw[0], kw[1], 0x7632);
+      const uint32_t k2 = __byte_perm(kw[2], kw[3], 0x5410), k3 = __byte_perm(kw[2], kw[3], 0x7632);
+      const uint32_t o0 = __byte_perm(bo[0], bo[1], 0x5410), o1 = __byte_perm(bo[0], bo[1], 0x7632);
+      const uint32_t o2 = __byte_perm(bo[2], bo[3], 0x5410), o3 = __byte_perm(bo[2], bo[3], 0x7632);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        mma_f16(c[q][i], (k0 >> (2 * i)) & 0x00030003u, (k1 >> (2 * i)) & 0x00030003u, (k2 >> (2 * i)) & 0x00030003u,
+                (k3 >> (2 * i)) & 0x00030003u, b.x, b.y);
+        mma_f16(c[q][i], (o0 >> (2 * i)) & 0x00010001u, (o1 >> (2 * i)) & 0x00010001u, (o2 >> (2 * i)) & 0x00010001u,
+                (o3 >> (2 * i)) & 0x00010001u, b.z, b.w);
+      }
+    }
+  }
+  const int64_t i0 = off * 4;  // first sample of this lane group's two words
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const unsigned long long lo = total_of(c[q][i][0], c[q][i][1], t), hi = total_of(c[q][i][2], c[q][i][3], t);
+      if (off < pitch && t == (i & 3)) {
+        atomicAdd(acc + i0 + 16 * q + i, lo);
+        atomicAdd(acc + i0 + 16 * q + i + 8, hi);
+      }
+    }
 }
 
 // multiply_Zt_v's last step (plink_reader.cpp:387) and, when effect != null, the
 // back-solve's effect / frequency (result_writer.cpp:614-620).
 __global__ void k_geno_zt_fin(const unsigned long long* __restrict__ acc, const long long* __restrict__ meta,
+                              const unsigned long long* __restrict__ tpart,
                               const double* __restrict__ mean, const double* __restrict__ inv_std,
                               int64_t m, const double* __restrict__ total_2pq, double* __restrict__ y,
                               double* __restrict__ effect, double* __restrict__ freq) {
   const int s = (int)meta[0];
-  const unsigned long long T = (unsigned long long)meta[1];
+  const unsigned long long T = all_sum_u64(tpart);
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < m;
        j += (int64_t)gridDim.x * blockDim.x) {
     const unsigned long long S = acc[j], miss = acc[m + j];
@@ -475,9 +602,9 @@ __global__ void k_geno_zt_fin(const unsigned long long* __restrict__ acc, const 
 }
 
 __global__ void k_geno_z_fin(const unsigned long long* __restrict__ acc, const long long* __restrict__ meta,
-                             int64_t n, double* __restrict__ y) {
+                             const unsigned long long* __restrict__ cpart, int64_t n, double* __restrict__ y) {
   const int s = (int)meta[0];
-  const unsigned long long C = (unsigned long long)meta[1];
+  const unsigned long long C = all_sum_u64(cpart);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = ldexp(__ll2double_rn((long long)(C + acc[i])), -s);
@@ -487,7 +614,10 @@ struct State {
   DevBuf<uint8_t> bed;      // m x pitch
   int64_t n = 0, m = 0, pitch = 0;
   DevBuf<double> stats;     // mean (m), inv_std (m), var2pq (m), total_2pq (1)
-  DevBuf<long long> fixv;   // fixed-point V and U (2 n_pad) or per-SNP values (3m)
+  DevBuf<long long> fixv;   // fixed-point V (n_pad) or per-SNP values (3m)
+  DevBuf<uint4> dig;        // their digits, in the products' order
+  DevBuf<double> part;      // partial sums of the preparations
+  DevBuf<unsigned long long> tpart;
   DevBuf<float> wterm;      // float terms of Z v (3m)
   DevBuf<long long> meta;   // s, T or C
   DevBuf<unsigned long long> acc;
@@ -526,31 +656,45 @@ void timed(cbx_handle* h, int bucket, double bytes, F&& launch) {
   }
 }
 
+// Buffers of both products, made at the first and kept with the payload.
+void scratch(State& g) {
+  const int64_t segs = (g.pitch + 63) / 64, blks = (g.m + 15) / 16;
+  g.fixv.resize(std::max<int64_t>(g.n_pad(), 3 * g.m));
+  g.wterm.resize(3 * g.m);
+  g.dig.resize(std::max<int64_t>(segs * 256, blks * 32));
+  g.part.resize(PREP_BLOCKS);
+  g.tpart.resize(PREP_BLOCKS);
+  g.meta.resize(2);
+  g.acc.resize(std::max<int64_t>(2 * g.m, g.n_pad()));
+}
+
 // y (m) = Z^T v for a device vector v (n).  With effect != null also the
 // back-solve's effect and frequency columns.
 void zt_device(cbx_handle* h, State& g, const double* v, double* y, double* effect, double* freq) {
   cudaStream_t s = h->stream;
-  const int64_t n_pad = g.n_pad();
-  g.fixv.resize(std::max<int64_t>(2 * n_pad, 3 * g.m));
-  g.meta.resize(2);
-  g.acc.resize(std::max<int64_t>(2 * g.m, n_pad));
+  scratch(g);
   CBX_CUDA(cudaMemsetAsync(g.acc.p + g.m, 0, g.m * sizeof(unsigned long long), s));
   long long* V = g.fixv.p;
-  long long* U = g.fixv.p + n_pad;
-  k_geno_vprep<<<1, PREP_THREADS, 0, s>>>(v, g.n, n_pad, V, U, g.meta.p, h->status.p);
+  uint2* B = reinterpret_cast<uint2*>(g.dig.p);
+  k_geno_vsum<<<PREP_BLOCKS, PREP_NT, 0, s>>>(v, g.n, g.part.p);
+  h->launched("k_geno_vsum");
+  k_geno_vprep<<<PREP_BLOCKS, PREP_NT, 0, s>>>(v, g.n, g.n_pad(), g.part.p, V, g.tpart.p, g.meta.p, h->status.p);
   h->launched("k_geno_vprep");
+  const int64_t segs = (g.pitch + 63) / 64;
+  k_geno_vdig<<<gridn(segs * 512, 256, 8 * h->num_sms), 256, 0, s>>>(V, g.n_pad(), segs * 512, B);
+  h->launched("k_geno_vdig");
   // algorithmic bytes: the payload once, v once per SNP block of the grid, one row result
   const double bytes = (double)g.m * (double)((g.n + 3) / 4) + 8.0 * (double)g.n + 8.0 * (double)g.m;
-  const unsigned gx = (unsigned)((g.m + ZT_THREADS - 1) / ZT_THREADS);
-  // samples per CTA: 4,096 (default), 2,048 or 8,192; exact integer sums, so every
-  // shape gives the same bits (the accumulator is zeroed before each run)
+  const unsigned gx = (unsigned)((g.m + ZT_ROWS - 1) / ZT_ROWS);
+  // 256-sample segments per CTA: 16 (default), 8 or 4 -- at most 4,096 samples, so that the
+  // FP32 sums stay exact; exact integer totals, so every shape gives the same bits (the
+  // accumulator is zeroed before each run)
   auto zt = [&](int c) {
     CBX_CUDA(cudaMemsetAsync(g.acc.p, 0, g.m * sizeof(unsigned long long), s));
-    const int chunk = c == 1 ? 2048 : (c == 2 ? 8192 : 4096);
-    const dim3 grid(gx, (unsigned)((n_pad + chunk - 1) / chunk));
-    if (c == 1) k_geno_zt<2048><<<grid, ZT_THREADS, 0, s>>>(g.bed.p, g.pitch, g.m, U, g.acc.p);
-    else if (c == 2) k_geno_zt<8192><<<grid, ZT_THREADS, 0, s>>>(g.bed.p, g.pitch, g.m, U, g.acc.p);
-    else k_geno_zt<4096><<<grid, ZT_THREADS, 0, s>>>(g.bed.p, g.pitch, g.m, U, g.acc.p);
+    const int per = c == 1 ? 8 : (c == 2 ? 4 : 16);
+    const int64_t gy = (segs + per - 1) / per;
+    CBX_REQUIRE(gy <= 65535, CBX_ERR_ARG, "too many samples for the Z'v grid");
+    k_geno_zt<<<dim3(gx, (unsigned)gy), ZT_THREADS, 0, s>>>(g.bed.p, g.pitch, g.m, per, B, g.acc.p);
     h->launched("k_geno_zt");
   };
   const int choice = tune::choose(h, tune::GENO_ZT, tune::size_class(g.n), tune::size_class(g.m), 1, 3, zt);
@@ -559,46 +703,44 @@ void zt_device(cbx_handle* h, State& g, const double* v, double* y, double* effe
     k_geno_miss_zt<<<(unsigned)((g.m + 7) / 8), 256, 0, s>>>(g.miss_ptr.p, g.miss_snp.p, g.m, V, g.acc.p);
     h->launched("k_geno_miss_zt");
   }
-  k_geno_zt_fin<<<gridn(g.m, 256, 4 * h->num_sms), 256, 0, s>>>(g.acc.p, g.meta.p, g.mean(), g.inv_std(), g.m,
-                                                                g.total(), y, effect, freq);
+  k_geno_zt_fin<<<gridn(g.m, 256, 4 * h->num_sms), 256, 0, s>>>(g.acc.p, g.meta.p, g.tpart.p, g.mean(),
+                                                                g.inv_std(), g.m, g.total(), y, effect, freq);
   h->launched("k_geno_zt_fin");
 }
 
 // y (n) = Z v for a device vector v (m).
 void z_device(cbx_handle* h, State& g, const double* v, double* y) {
   cudaStream_t s = h->stream;
-  const int64_t n_pad = g.n_pad();
-  g.fixv.resize(std::max<int64_t>(2 * n_pad, 3 * g.m));
-  g.wterm.resize(3 * g.m);
-  g.meta.resize(2);
-  g.acc.resize(std::max<int64_t>(2 * g.m, n_pad));
-  k_geno_zprep<<<1, PREP_THREADS, 0, s>>>(v, g.mean(), g.inv_std(), g.m, g.wterm.p, g.fixv.p, g.meta.p,
-                                          h->status.p);
+  scratch(g);
+  const int64_t n_pad = g.n_pad(), blks = (g.m + 15) / 16;
+  k_geno_zterms<<<PREP_BLOCKS, PREP_NT, 0, s>>>(v, g.mean(), g.inv_std(), g.m, g.wterm.p, g.part.p);
+  h->launched("k_geno_zterms");
+  k_geno_zprep<<<PREP_BLOCKS, PREP_NT, 0, s>>>(g.wterm.p, g.m, g.part.p, g.fixv.p, g.tpart.p, g.meta.p, h->status.p);
   h->launched("k_geno_zprep");
-  const int gx = (int)((g.pitch + 4 * Z_THREADS - 1) / (4 * Z_THREADS));
+  k_geno_zdig<<<gridn(blks * 32, 256, 8 * h->num_sms), 256, 0, s>>>(g.fixv.p, g.m, blks * 32, g.dig.p);
+  h->launched("k_geno_zdig");
+  const int gx = (int)((g.pitch + Z_SAMPLES / 4 - 1) / (Z_SAMPLES / 4));
   const double bytes = (double)g.m * (double)((g.n + 3) / 4) + 8.0 * (double)g.m + 8.0 * (double)g.n;
-  // about 4 (default), 2 or 8 CTAs per SM, at most Z_MAX_ROWS SNP rows each; exact
-  // integer sums, so every shape gives the same bits (the accumulator is zeroed
-  // before each run)
+  // about 4 (default), 2 or 8 CTAs per SM, at most Z_MAX_ROWS SNPs each, so that the FP32
+  // sums stay exact; exact integer totals, so every shape gives the same bits (the
+  // accumulator is zeroed before each run)
   auto zk = [&](int c) {
     CBX_CUDA(cudaMemsetAsync(g.acc.p, 0, n_pad * sizeof(unsigned long long), s));
     const int per_sm = c == 1 ? 2 : (c == 2 ? 8 : 4);
     int64_t gy = std::max<int64_t>(1, (per_sm * (int64_t)h->num_sms + gx - 1) / gx);
-    int64_t rows = std::min<int64_t>((g.m + gy - 1) / gy, Z_MAX_ROWS);
-    gy = (g.m + rows - 1) / rows;
+    const int64_t per = std::min<int64_t>((blks + gy - 1) / gy, Z_MAX_ROWS / 16);
+    gy = (blks + per - 1) / per;
     CBX_REQUIRE(gy <= 65535, CBX_ERR_ARG, "too many SNPs for the Z v grid");
-    const int smem = (int)(3 * rows * sizeof(long long));
-    k_geno_z<<<dim3((unsigned)gx, (unsigned)gy), Z_THREADS, smem, s>>>(g.bed.p, g.pitch, g.m, (int)rows, g.fixv.p,
-                                                                      g.acc.p);
+    k_geno_z<<<dim3((unsigned)gx, (unsigned)gy), Z_THREADS, 0, s>>>(g.bed.p, g.pitch, g.m, (int)per, g.dig.p, g.acc.p);
     h->launched("k_geno_z");
   };
   const int choice = tune::choose(h, tune::GENO_Z, tune::size_class(g.n), tune::size_class(g.m), 1, 3, zk);
   timed(h, 4, bytes, [&] { zk(choice); });
   if (g.nmiss > 0) {
-    k_geno_miss_z<<<(unsigned)((g.n + 7) / 8), 256, 0, s>>>(g.samp_ptr.p, g.miss_samp.p, g.n, g.fixv.p, g.acc.p);
+    k_geno_miss_z<<<(unsigned)((g.n + 7) / 8), 256, 0, s>>>(g.samp_ptr.p, g.miss_samp.p, g.n, g.fixv.p + 2 * g.m, g.acc.p);
     h->launched("k_geno_miss_z");
   }
-  k_geno_z_fin<<<gridn(g.n, 256, 4 * h->num_sms), 256, 0, s>>>(g.acc.p, g.meta.p, g.n, y);
+  k_geno_z_fin<<<gridn(g.n, 256, 4 * h->num_sms), 256, 0, s>>>(g.acc.p, g.meta.p, g.tpart.p, g.n, y);
   h->launched("k_geno_z_fin");
 }
 
