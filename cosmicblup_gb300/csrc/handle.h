@@ -28,6 +28,7 @@ struct cbx_handle {
   // Genomic relationship matrix kept on the device after cbx_grm_bed, and its
   // eigen-bent inverse after cbx_invert_psd.
   cbx::DevBuf<double> G;
+  cbx::DevBuf<uint8_t> grm_ws[2];  // scratch of cbx_grm_bed, at most 64 MB each between calls
   int64_t G_n = 0;
   cbx::DevBuf<double> Ginv;
   int64_t Ginv_n = 0;
