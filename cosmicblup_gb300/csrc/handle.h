@@ -21,6 +21,9 @@ struct cbx_handle {
   // dense block product on `stream` (fork / join events, captured into graphs)
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // third stream: the sums of the gathered vectors, beside the same product
+  cudaStream_t stream3 = nullptr;
+  cudaEvent_t ev_join3 = nullptr;
   std::string last_error;
   int64_t launches = 0;
   cbx::DevBuf<int> status;  // device-side error word(s)

@@ -712,34 +712,42 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
     // FP32: gather the dense-block rows, their FP64 column sums, the product
     // (the populated 32-column groups only)
     const bool split = matvec_split(h, op);
-    if (split) {
-      // the sparse part on the second stream, beside the block product: k_spmv
-      // without the block term writes every row and its pq partials
-      cudaStream_t s2 = h->stream2;
-      CBX_CUDA(cudaEventRecord(h->ev_fork, s));
+    const Mme& mm = *h->mme;
+    cudaStream_t s2 = h->stream2, s3 = h->stream3;
+    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
+    if (split || (use_D && mm.nseg > 0)) {
+      // beside the block product on the second stream: the fixed rows' segments and,
+      // with the split, the rest of the sparse part (k_spmv without the block term
+      // writes every row and its pq partials)
       CBX_CUDA(cudaStreamWaitEvent(s2, h->ev_fork, 0));
       sv::OpView<T> ops = op;
       ops.Qd = nullptr;
-      if (use_D && h->mme->nseg > 0) {
-        const Mme& mm = *h->mme;
+      if (use_D && mm.nseg > 0) {
         sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s2>>>(ops, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X,
                                                         w.seg_part.p, active, ncp);
         h->launched("k_fix_seg<f32>");
       }
-      sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s2>>>(ops, X, nullptr, 1, nullptr, 0.0, h->mme->fix_seg_ptr.p,
-                                                        w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
-      h->launched("k_spmv<f32>");
+      if (split) {
+        sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s2>>>(ops, X, nullptr, 1, nullptr, 0.0, mm.fix_seg_ptr.p,
+                                                          w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
+        h->launched("k_spmv<f32>");
+      }
       CBX_CUDA(cudaEventRecord(h->ev_join, s2));
     }
     sv::k_gather_t<T, S><<<grid_for(ncp * op.ld, 256, 16 * h->num_sms), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld,
                                                                                  op.gmap, active, S, ncp);
     h->launched("k_gather_t<f32>");
-    sv::k_colsum_vt<T><<<ncp, 1024, 0, s>>>(w.Vt.p, op.ld, op.ng, w.colsum.p);
+    // the gathered vectors' sums, which only the last kernel reads, on the third
+    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
+    CBX_CUDA(cudaStreamWaitEvent(s3, h->ev_fork, 0));
+    sv::k_colsum_vt<T><<<ncp, 1024, 0, s3>>>(w.Vt.p, op.ld, op.ng, w.colsum.p);
     h->launched("k_colsum_vt<f32>");
+    CBX_CUDA(cudaEventRecord(h->ev_join3, s3));
     tsplit = product_from_vt<T, S>(h, op, w, active, ncols);
+    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join3, 0));
+    if (split || (use_D && mm.nseg > 0)) CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
     if (split) {
       // the block term of the genotyped rows, once both are done
-      CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
       sv::k_dense_add<T, S><<<w.nblk_dadd, sv::NT, 0, s>>>(op, w.Tout.p, tsplit, colsum, tshift, (T)lam, Y, P,
                                                            pq_part ? pq_part + (size_t)w.nblk_spmv * S : nullptr,
                                                            active, ncp);
@@ -747,7 +755,7 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       return;
     }
   }
-  if (use_D && h->mme->nseg > 0) {
+  if (use_D && h->mme->nseg > 0 && !(sizeof(T) == 4 && op.Qd)) {
     const Mme& mm = *h->mme;
     sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p, active,
                                                    ncp);
