@@ -767,6 +767,22 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   h->launched(sizeof(T) == 4 ? "k_spmv<f32>" : "k_spmv<f64>");
 }
 
+// A launch that may be set up while its predecessor on the stream still runs; the kernel
+// begins with wait_predecessor.
+template <typename... KArgs, typename... Args>
+void launch_next(void (*kern)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CBX_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+
 // Multi-RHS PCG in precision T on interleaved vectors; X receives the solution
 // (holds x0 when use_x0).  tol_col: per-column tolerance.
 template <typename T, int S>
@@ -866,20 +882,20 @@ void run_pcg(cbx_handle* h, Mme& m, const sv::OpView<T>& op, Workspace<T, S>& w,
     }
     for (int j = 0; j < CHECK; ++j) {
       matvec<T, S>(h, op, w, w.P.p, w.Q.p, lam, 1, w.P.p, w.pq_part.p, w.active.p, false, ncols);
-      sv::k_scalar_alpha_c<S><<<S, sv::NTC, 0, s>>>(w.col.p, w.pq_part.p,
-                                                    w.nblk_spmv + (matvec_split(h, op) ? w.nblk_dadd : 0));
+      launch_next(sv::k_scalar_alpha_c<S>, S, sv::NTC, s, w.col.p, w.pq_part.p,
+                  w.nblk_spmv + (matvec_split(h, op) ? w.nblk_dadd : 0));
       h->launched(sizeof(T) == 4 ? "k_scalar_alpha<f32>" : "k_scalar_alpha<f64>");
-      sv::k_update<T, S><<<w.nblk_vec, sv::NT, 0, s>>>(op, w.col.p, X, Xlo, w.R.p, w.P.p, w.Q.p, w.part.p);
+      launch_next(sv::k_update<T, S>, w.nblk_vec, sv::NT, s, op, w.col.p, X, Xlo, w.R.p, w.P.p, w.Q.p, w.part.p);
       h->launched(sizeof(T) == 4 ? "k_update<f32>" : "k_update<f64>");
       if (m.p > 0) {
-        sv::k_fixed<T, S><<<(unsigned)m.p, sv::NT_FIXED, 0, s>>>(op, w.R.p, w.Z.p, w.col.p, w.rz_fix.p);
+        launch_next(sv::k_fixed<T, S>, (int)m.p, sv::NT_FIXED, s, op, w.R.p, w.Z.p, w.col.p, w.rz_fix.p);
         h->launched(sizeof(T) == 4 ? "k_fixed<f32>" : "k_fixed<f64>");
       }
-      sv::k_scalar_beta_c<S><<<S, sv::NTC, 0, s>>>(w.col.p, w.part.p, w.nblk_vec, w.rz_fix.p, m.p, w.tol.p, abs_tol,
-                                                   maxit, w.active.p, w.done.p);
+      launch_next(sv::k_scalar_beta_c<S>, S, sv::NTC, s, w.col.p, w.part.p, w.nblk_vec, w.rz_fix.p, m.p, w.tol.p,
+                  abs_tol, maxit, w.active.p, w.done.p);
       h->launched(sizeof(T) == 4 ? "k_scalar_beta<f32>" : "k_scalar_beta<f64>");
-      sv::k_pupdate<T, S><<<grid_for(m.dim * S, sv::NT, 16 * h->num_sms), sv::NT, 0, s>>>(
-          m.dim, m.p, op.dinv, w.col.p, w.R.p, w.Z.p, w.P.p);
+      launch_next(sv::k_pupdate<T, S>, grid_for(m.dim * S, sv::NT, 16 * h->num_sms), sv::NT, s, m.dim, m.p, op.dinv,
+                  w.col.p, w.R.p, w.Z.p, w.P.p);
       h->launched(sizeof(T) == 4 ? "k_pupdate<f32>" : "k_pupdate<f64>");
     }
   };

@@ -70,6 +70,13 @@ __device__ __forceinline__ double dot16(const double2& a, const double2& b) {
   return a.x * b.x + a.y * b.y;
 }
 
+// The kernels between two block products follow one another in a few microseconds each;
+// they are launched as programmatic dependents, which are set up while their predecessor
+// still runs and begin with this wait for its end (and so for that of all before it).
+__device__ __forceinline__ void wait_predecessor() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Vt[c * ld + k] = X[(p + gmap[k]) * xs + c] for k < ng, 0 for ng <= k < ld
 // (S columns of a block whose rows are xs apart; xs = S for the whole block).
 template <typename T, int S>
@@ -933,6 +940,7 @@ template <typename T, int S>
 __global__ void __launch_bounds__(NT_FIXED) k_fixed(OpView<T> op, const T* __restrict__ R,
                                                     T* __restrict__ Z, const Col* __restrict__ col,
                                                     double* __restrict__ rz_fix /*[p][S]*/) {
+  wait_predecessor();
   __shared__ T redT[NT_FIXED];
   const int64_t f = blockIdx.x;
   constexpr int G = NT_FIXED / S;
@@ -964,6 +972,7 @@ __global__ void __launch_bounds__(NT) k_update(OpView<T> op, const Col* __restri
                                                const T* __restrict__ P,
                                                const T* __restrict__ Q,
                                                double* __restrict__ part /*[grid][2][S]*/) {
+  wait_predecessor();
   __shared__ double red[NT];
   DotAcc<T> arr, arz;
   const int c = threadIdx.x % S;
@@ -1016,6 +1025,7 @@ template <typename T, int S>
 __global__ void __launch_bounds__(NT) k_pupdate(int64_t dim, int64_t nfix, const T* __restrict__ dinv,
                                                 const Col* __restrict__ col, const T* __restrict__ R,
                                                 const T* __restrict__ Z, T* __restrict__ P) {
+  wait_predecessor();
   const int c = threadIdx.x % S;
   if (!col[c].active) return;
   const T beta = (T)col[c].beta;
@@ -1219,6 +1229,7 @@ __device__ __forceinline__ void col_totals_c(const double* const (&part)[K], con
 // alpha = rz / p'Ap per column (grid = S blocks), breakdown handling as k_scalar_alpha.
 template <int S>
 __global__ void __launch_bounds__(NTC) k_scalar_alpha_c(Col* col, const double* pq_part, int nblk) {
+  wait_predecessor();
   __shared__ double red[1][NTC];
   const int c = blockIdx.x;
   if (!col[c].active) return;  // uniform over the block
@@ -1253,6 +1264,7 @@ __global__ void __launch_bounds__(NTC) k_scalar_beta_c(Col* col, const double* p
                                                        const double* rz_fix, int64_t p, const double* tol_col,
                                                        int abs_tol, int maxit, int* active_count,
                                                        unsigned* done) {
+  wait_predecessor();
   __shared__ double red[3][NTC];
   __shared__ int last;
   const int c = blockIdx.x;
