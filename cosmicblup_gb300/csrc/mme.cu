@@ -687,8 +687,25 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   // qshift * (column sums) back; the FP64 product uses the block itself.
   const double* colsum = op.Qd ? w.colsum.p : nullptr;
   const double tshift = h->mme->qshift;
+  // the fixed rows' segments run on the second stream beside the block product (one
+  // stream under a launch trace, whose attribution assumes one)
+  const Mme& mm = *h->mme;
+  const bool segs = use_D && mm.nseg > 0;
+  cudaStream_t s2 = h->trace_on || !op.Qd ? s : h->stream2;
+  auto segments = [&]() {
+    if (!segs) return;
+    sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s2>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p,
+                                                    active, ncp);
+    h->launched(sizeof(T) == 4 ? "k_fix_seg<f32>" : "k_fix_seg<f64>");
+  };
+  if (op.Qd) {
+    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
+    CBX_CUDA(cudaStreamWaitEvent(s2, h->ev_fork, 0));
+  }
+  segments();
   if (!op.Qd) {
   } else if constexpr (sizeof(T) == 8) {
+    CBX_CUDA(cudaEventRecord(h->ev_join, s2));
     ff = ff && h->mme->Qlo32.p && h->mme->Qd32.p;
     if (!ff) colsum = nullptr;
     cbx_handle::ProfRec pr{};
@@ -708,34 +725,28 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       pr.bytes = 8.0 * (double)op.ng * op.ld + 8.0 * ncols * ((double)op.ld + (double)op.ng);
       h->prof.push_back(pr);
     }
+    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
   } else {
     // FP32: gather the dense-block rows, their FP64 column sums, the product
     // (the populated 32-column groups only)
     const bool split = matvec_split(h, op);
-    const Mme& mm = *h->mme;
-    cudaStream_t s2 = h->stream2, s3 = h->stream3;
-    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
-    if (split || (use_D && mm.nseg > 0)) {
-      // beside the block product on the second stream: the fixed rows' segments and,
-      // with the split, the rest of the sparse part (k_spmv without the block term
-      // writes every row and its pq partials)
-      CBX_CUDA(cudaStreamWaitEvent(s2, h->ev_fork, 0));
+    cudaStream_t s3 = h->trace_on ? s : h->stream3;
+    if (split) {
+      // the rest of the sparse part beside the product too: k_spmv without the block
+      // term writes every row and its pq partials
       sv::OpView<T> ops = op;
       ops.Qd = nullptr;
-      if (use_D && mm.nseg > 0) {
-        sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s2>>>(ops, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X,
-                                                        w.seg_part.p, active, ncp);
-        h->launched("k_fix_seg<f32>");
-      }
-      if (split) {
-        sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s2>>>(ops, X, nullptr, 1, nullptr, 0.0, mm.fix_seg_ptr.p,
-                                                          w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
-        h->launched("k_spmv<f32>");
-      }
-      CBX_CUDA(cudaEventRecord(h->ev_join, s2));
+      sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s2>>>(ops, X, nullptr, 1, nullptr, 0.0, mm.fix_seg_ptr.p,
+                                                        w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
+      h->launched("k_spmv<f32>");
     }
-    sv::k_gather_t<T, S><<<grid_for(ncp * op.ld, 256, 16 * h->num_sms), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld,
-                                                                                 op.gmap, active, S, ncp);
+    CBX_CUDA(cudaEventRecord(h->ev_join, s2));
+    if constexpr (S >= 32)
+      sv::k_gather_tile<T, S><<<(unsigned)((op.ld + 31) / 32), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld, op.gmap,
+                                                                            active, ncp);
+    else
+      sv::k_gather_t<T, S><<<grid_for(ncp * op.ld, 256, 16 * h->num_sms), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld,
+                                                                                   op.gmap, active, S, ncp);
     h->launched("k_gather_t<f32>");
     // the gathered vectors' sums, which only the last kernel reads, on the third
     CBX_CUDA(cudaEventRecord(h->ev_fork, s));
@@ -745,7 +756,7 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
     CBX_CUDA(cudaEventRecord(h->ev_join3, s3));
     tsplit = product_from_vt<T, S>(h, op, w, active, ncols);
     CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join3, 0));
-    if (split || (use_D && mm.nseg > 0)) CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
+    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
     if (split) {
       // the block term of the genotyped rows, once both are done
       sv::k_dense_add<T, S><<<w.nblk_dadd, sv::NT, 0, s>>>(op, w.Tout.p, tsplit, colsum, tshift, (T)lam, Y, P,
@@ -754,12 +765,6 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       h->launched("k_dense_add<f32>");
       return;
     }
-  }
-  if (use_D && h->mme->nseg > 0 && !(sizeof(T) == 4 && op.Qd)) {
-    const Mme& mm = *h->mme;
-    sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p, active,
-                                                   ncp);
-    h->launched(sizeof(T) == 4 ? "k_fix_seg<f32>" : "k_fix_seg<f64>");
   }
   sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s>>>(op, X, w.Tout.p, tsplit, colsum, tshift, h->mme->fix_seg_ptr.p,
                                                   w.seg_part.p,

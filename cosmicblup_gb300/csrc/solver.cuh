@@ -92,6 +92,29 @@ __global__ void k_gather_t(const T* __restrict__ X, T* __restrict__ Vt, int64_t 
   }
 }
 
+// The same for 32 and more columns, 32 rows a block through shared memory: rows are read
+// and written whole (n = 20,000, 64 columns: 12 us one element a thread, 9.7 so).
+template <typename T, int S>
+__global__ void __launch_bounds__(256) k_gather_tile(const T* __restrict__ X, T* __restrict__ Vt, int64_t p,
+                                                     int64_t ng, int64_t ld, const int32_t* __restrict__ gmap,
+                                                     const int* __restrict__ active, int nc) {
+  if (active && *active == 0) return;
+  __shared__ T tile[32][S + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t k0 = (int64_t)blockIdx.x * 32;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int64_t k = k0 + warp + 8 * j;
+    const T* row = X + (k < ng ? (p + gmap[k]) * S : 0);
+#pragma unroll
+    for (int c = 0; c < S; c += 32)
+      if (c + lane < nc) tile[warp + 8 * j][c + lane] = k < ng ? row[c + lane] : T(0);
+  }
+  __syncthreads();
+  if (k0 + lane < ld)
+    for (int c = warp; c < nc; c += 8) Vt[(int64_t)c * ld + k0 + lane] = tile[lane][c];
+}
+
 // Dense block product Tout[i * os + c] = sum_k Qd[i * ld + k] * Vt[c * ld + k]
 // (os = S unless the S columns are a piece of a wider block).
 // 8 warps per block, RPW rows per warp; lanes stream 16-byte vectors of each
@@ -681,7 +704,8 @@ __device__ __forceinline__ void spmv_random_row(const OpView<T>& op, int64_t i, 
 #pragma unroll
     for (int j = 0; j < CPL; ++j) acc[j] = qv[j] = T(0);
     // entries in batches of 4: all the batch's row loads are issued before its
-    // multiply-adds (same order of additions as one entry at a time)
+    // multiply-adds (same order of additions as one entry at a time); batches of 8 were
+    // 8 % slower at 200,000 rows of 128 (fewer warps)
     auto rowsum = [&](const int32_t* __restrict__ cidx, const T* __restrict__ val, int32_t e, int32_t e1,
                       int64_t off, T (&out)[CPL]) {
       for (; e + 3 < e1; e += 4) {
@@ -1019,6 +1043,11 @@ __global__ void __launch_bounds__(NT) k_update(OpView<T> op, const Col* __restri
   if (threadIdx.x < S) part[((int64_t)blockIdx.x * 2 + 1) * S + c] = t;
 }
 
+// Elements of a thread whose loads are in flight together in k_pupdate: one at a time it
+// was bound by the latency of the chain (200,000 x 80 columns of 128: 52 us, four 41, at
+// 6.2 TB/s; k_update, with twice the streams, gains nothing by it).
+constexpr int BATCH = 4;
+
 // p = z + beta p (active columns); z = Z on the fixed rows (k_fixed), Jacobi r on
 // the random rows (the same product k_update sums).
 template <typename T, int S>
@@ -1029,13 +1058,22 @@ __global__ void __launch_bounds__(NT) k_pupdate(int64_t dim, int64_t nfix, const
   const int c = threadIdx.x % S;
   if (!col[c].active) return;
   const T beta = (T)col[c].beta;
-  const int64_t total = dim * S;
-  for (int64_t idx = blockIdx.x * (int64_t)NT + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * NT) {
-    const int64_t i = idx / S;
-    const T z = i < nfix ? Z[idx] : dinv[i - nfix] * R[idx];
-    P[idx] = z + beta * P[idx];
-  }
+  const int64_t total = dim * S, step = (int64_t)gridDim.x * NT;
+  auto batch = [&](int64_t idx, auto count) {
+    constexpr int U = decltype(count)::value;
+    T z[U], pv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = idx + u * step, i = e / S;
+      z[u] = i < nfix ? Z[e] : dinv[i - nfix] * R[e];
+      pv[u] = P[e];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) P[idx + u * step] = z[u] + beta * pv[u];
+  };
+  int64_t idx = blockIdx.x * (int64_t)NT + threadIdx.x;
+  for (; idx + (BATCH - 1) * step < total; idx += BATCH * step) batch(idx, std::integral_constant<int, BATCH>{});
+  for (; idx < total; idx += step) batch(idx, std::integral_constant<int, 1>{});
 }
 
 // Sum of part[b * stride + c] over b < nblk for every column c < S, by all
