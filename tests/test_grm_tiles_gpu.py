@@ -50,3 +50,24 @@ def test_grm_largest_digits(handle):
     for j in range(m):
         g[j] = np.bincount(rng.permutation(2 * n)[:best[1]] // 2, minlength=n)
     check(handle, encode_bed(g), n, m)
+
+
+def test_grm_copied_behind_the_tiles(handle):
+    """Pinned output of an order whose copy follows the groups of tiles, against the copy
+    of the whole matrix that pageable output gets: every entry, counts too."""
+    import ctypes as C
+
+    import torch
+
+    from cosmicblup_gb300._lib import lib, ptr
+    n, m = 7001, 130
+    bed = np.frombuffer(simulate_bed(n, m, seed=8, miss=0.02)[0], np.uint8)
+    out = []
+    for pinned in (False, True):
+        G = torch.full((n, n), float("nan"), dtype=torch.float64, pin_memory=pinned).numpy()
+        s, k = C.c_double(), C.c_int64()
+        handle.check(lib().cbx_grm_bed(handle.raw, ptr(bed), bed.size, n, m, C.c_float(0.01), 1, 2048, ptr(G), None,
+                                       None, C.byref(s), C.byref(k)))
+        out.append(G)
+    np.testing.assert_array_equal(out[0], out[1])
+    assert np.array_equal(out[1], out[1].T)
