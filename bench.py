@@ -521,7 +521,7 @@ def run_gpu(args, cfg):
         _, Gd_h = ssgblup_qinv(dm, d["dam"], d["sire"], gmap, G=None, return_blocks=True)
         phases["hinv_setup_s"] = time.perf_counter() - t0
     else:
-        # eigen-bent G^-1 (FP64, cuSOLVER syevd + GEMM); host copy for the CPU baseline
+        # eigen-bent G^-1 in FP64; host copy for the CPU baseline
         t0 = time.perf_counter()
         Ginv_host = invert_psd(h, None, n, download=want_host)
         phases["g_inverse_s"] = time.perf_counter() - t0

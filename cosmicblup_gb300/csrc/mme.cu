@@ -1683,7 +1683,7 @@ extern "C" int cbx_mme_create(cbx_handle* h, int64_t n_rec, int64_t p, int64_t q
         if (ok)
           CBX_CUDA(cudaMemcpyAsync(m->A11inv64.p, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, s));
       } else {
-        // Cholesky inverse on the device (cuSOLVER potrf / potri)
+        // Cholesky inverse on the device (fx64.cu)
         CBX_CUDA(cudaMemcpyAsync(m->A11inv64.p, M.data(), M.size() * sizeof(double), cudaMemcpyHostToDevice, s));
         ok = chol_inverse_device(h, m->A11inv64.p, p);
       }
