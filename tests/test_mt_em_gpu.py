@@ -6,7 +6,8 @@ entry of Vg and Ve is a sum of n terms of its own size, so they agree to n * 2^-
 import numpy as np
 import pytest
 
-from cosmicblup_gb300 import MvEigenVce, MvOptions
+from cosmicblup_gb300 import GrmBuilder, GrmOptions, MvEigenVce, MvOptions, PlinkReader, invert_psd
+from cosmicblup_gb300.synth import simulate_bed
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +46,30 @@ def test_em_iterations(handle, n, t):
     assert v.iterations == 4
     assert np.abs(v.getVg() - Vg).max() <= tol * np.abs(Vg).max()
     assert np.abs(v.getVe() - Ve).max() <= tol * np.abs(Ve).max()
+
+
+@pytest.mark.parametrize("n,t", [(129, 2), (320, 3), (513, 2)])
+def test_g_recovered_from_the_device_inverse(handle, n, t):
+    """Vg and Ve of the G that the handle's eigen-bent G^-1 stands for, against those of the
+    bent G itself.  G^-1 has entries of 1 / (1e-6 n), each rounded at 2^-53 of that, and G's
+    other eigenvalues are about 1: an error of 1e-16 * 1e6 / n * sqrt(n) a row, 1e-11 at
+    these orders, and ten times that for the iterations' amplification."""
+    m = 12 * n
+    bed, _ = simulate_bed(n, m, seed=n, miss=0.02)
+    b = GrmBuilder(GrmOptions(), handle=handle)
+    b.compute(PlinkReader.from_bytes(bed, n, m))
+    w, U = np.linalg.eigh(b.getGrm())
+    G = (U * np.maximum(w, 1e-6)) @ U.T
+    invert_psd(handle, None, n, download=False)
+    rng = np.random.default_rng(n)
+    X = np.stack([np.ones(n), rng.integers(0, 2, n)], 1).astype(float)
+    Y = rng.standard_normal((n, t)) + np.linalg.cholesky(G + 0.01 * np.eye(n)) @ rng.standard_normal((n, t))
+    out = []
+    for g in (None, G):
+        v = MvEigenVce(handle, MvOptions())
+        v.prepare(Y, X, g)
+        v.runNullModel()
+        out.append((v.getVg(), v.getVe(), v.iterations))
+    assert out[0][2] == out[1][2]
+    for a, e in zip(out[0][:2], out[1][:2]):
+        assert np.linalg.norm(a - e) <= 1e-10 * np.linalg.norm(e)
