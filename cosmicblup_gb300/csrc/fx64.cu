@@ -16,8 +16,8 @@
 //
 // Factorization.  Right-looking in blocks of 32 inside outer panels of 128 to 512
 // columns, in a row-major lower triangle W.  Step k (k_panel) factors the 32 x 32
-// pivot block by FP64 elimination, giving X = L_kk^-1, and forms L_ik = S_ik X' for the
-// rows below; for the inverse also row k of M = L^-1, M_kj = X R_kj for j < k, where
+// pivot block by FP64 elimination, giving X = L_kk^-1, and substitutes L_ik L_kk' = S_ik for
+// the rows below; for the inverse also row k of M = L^-1, L_kk M_kj = R_kj for j < k, where
 // R_ij = -sum_l L_il M_lj is kept in the slot of W that L_ij has left.  Digit MMAs then
 // apply S_ij -= L_ik L_jk' and R_ij -= L_ik M_kj, within the panel after each step
 // (K = 32) and to the rest once per panel (K = the panel's width).  A^-1 = M'M is one
@@ -26,7 +26,7 @@
 // Bound: below n = 3,000 the chain of 32-wide steps (a pivot factor and a K = 32 update,
 // 26 us); above it the digit MMAs (36 per FP64 multiply-add) and the L2 reads that feed
 // them (96 KB a step of 2,304 tensor clocks).  Measured, inverse with its factor, against
-// cuSOLVER potrf + potri: n = 500 0.63 ms (4.2), 2,000 2.8 (31), 8,000 34 (1,194), 20,000
+// cuSOLVER potrf + potri: n = 500 0.63 ms (4.2), 2,000 2.8 (31), 8,000 35 (1,194), 20,000
 // 322 (about 11,000).  The product at n = 2,000: 0.60 ms (15.3 by cuBLAS DGEMM).  128 x 64
 // tiles: eight classes of 64 columns fill the 512 TMEM columns, and a narrower tile reads
 // the A digits more often.
@@ -604,21 +604,31 @@ __device__ __forceinline__ double reciprocal(double d) {
 }
 
 // One 32-wide step.  Every CTA factors the pivot block (it is small, and a separate
-// launch would cost more than the repeat), then takes 16-row groups: out = v X' with v
+// launch would cost more than the repeat), then takes 16-row groups: x L_kk' = v with v
 // the row's 32 entries in the pivot columns (rows below the pivot), the column's
-// entries in the pivot rows (columns left of it), or a unit vector (the pivot rows).
+// entries in the pivot rows (columns left of it), or a unit vector (the pivot rows, whose x
+// are the columns of X = L_kk^-1).
 //
 // A chain of FP64 latencies bounds it: a dependent multiply-add takes 68 clocks, a reciprocal
 // 230, a publish and barrier 120, and one warp-wide FP64 instruction holds its
 // quarter of the SM's FP64 pipe for 64.  Hence 2 x 2 pivots (one reciprocal and one
 // barrier for two columns), the next pivot's rows and its publication ahead of the other
 // rows of a step, no square root inside the chain, and groups of 16 rows, which put a
-// problem of 2,000 rows on 128 SMs.  Measured at n = 2,048: 39,000 clocks, 25,000 of them the
-// pivots (50,000 with 1 x 1 pivots, and 73,000 with their square roots and divisions).
+// problem of 2,000 rows on 128 SMs.
+//
+// A pivot pair is applied as L D L', never by its explicit inverse: with l = p12 / p11, the
+// second row less l times the first (w) is eliminated by p2 = p22 - l p12.  The inverse's
+// two terms cancel to the same small difference, but each is rounded at the size of p12 / p2
+// first, and the condition of the pair enters twice.  The groups' rows are forward
+// substitutions by the same pairs and not products with X, which lose the root of L_kk's
+// condition where two adjacent rows are near-duplicates.  Measured with the pair's inverse
+// and X before, both this way now: factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81, now 2.84;
+// at 8,000 18.3, now 18.2, and 34.4, now 35.0 (a substitution issues 92 FP64 instructions a
+// warp and group, the product 80).  L L' - A at n = 96 with adjacent rows 1e-3 apart: 0.02 of 4 n u,
+// before above it 200 times, and at 1e-5 apart no pivot was found.
 __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) {
-  __shared__ double X[32][33], V[32][33], Lm[32][33], pa[16][32], pb[16][32];
-  __shared__ double pv[32], i1[16], l2[16], i2[16];
-  __shared__ int mx[4][32];
+  __shared__ double X[32][33], V[4][32][5], pa[16][32], pb[16][32], ra[16][32], rw[16][32];
+  __shared__ double pv[32], lp[16], i1[16], l2[16], i2[16];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t np = a.np;
   const double* Wk = a.W + (int64_t)a.k0 * np + a.k0;
@@ -629,36 +639,45 @@ __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) 
     const int r = 2 * (w + 4 * (t >> 1)) + (t & 1);
     d[t] = lane <= r ? Wk[r * np + lane] : Wk[lane * np + r];
   }
-  // the first group's entries, in flight during the factorization
-  const int row = lane & 15, half = lane >> 4;
+  // groups of 16 rows: a warp takes four, eight lanes a row, columns c + 8 m.  The first
+  // group's entries are in flight during the factorization
+  const int c = lane & 7, row = 4 * w + (lane >> 3);
   const int gk = a.k0 / 16, ng = (int)(np / 16);
   int g = (a.inverse ? 0 : gk) + blockIdx.x;
-  double pre[4];
+  double pre[4] = {0.0, 0.0, 0.0, 0.0};
   auto fetch = [&](int gg) {
-    const int r0 = gg * 16;
+    if (gg == gk || gg == gk + 1) return;  // the pivot rows: from X
+    const int r = gg * 16 + row;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      pre[i] = gg > gk + 1 ? a.W[(int64_t)(r0 + w + 4 * i) * np + a.k0 + lane]
-               : gg < gk   ? a.W[(int64_t)(a.k0 + 2 * w + half + 8 * i) * np + r0 + row]
-                           : (2 * w + half + 8 * i == r0 - a.k0 + row ? 1.0 : 0.0);
+    for (int m = 0; m < 4; ++m)
+      pre[m] = gg > gk ? a.W[(int64_t)r * np + a.k0 + c + 8 * m] : a.W[(int64_t)(a.k0 + c + 8 * m) * np + r];
   };
   if (g < ng) fetch(g);
-  // rows 2 j, 2 j + 1 (registers 2 s, 2 s + 1 of warp j & 3) times the inverse of their
-  // 2 x 2 pivot, whose own columns take the inverse itself
+  // rows 2 j, 2 j + 1 (registers 2 s, 2 s + 1 of warp j & 3): the first (ra), the second less
+  // l times it (rw), and both over their pivots (pa, pb); their own columns take those of
+  // the pair's inverse
   auto publish = [&](int j, double& da, double& db) {
     const int k = 2 * j;
-    const double p11 = __shfl_sync(~0u, da, k), p12 = __shfl_sync(~0u, db, k), p22 = __shfl_sync(~0u, db, k + 1);
+    const double p11 = __shfl_sync(~0u, da, k), p12 = __shfl_sync(~0u, da, k + 1), p22 = __shfl_sync(~0u, db, k + 1);
     const double det = fma(p11, p22, -p12 * p12);
-    const double inv = reciprocal(det);
+    // both reciprocals in one pass of the chain, half a warp each
+    const double rcp = reciprocal(lane < 16 ? p11 : det);
+    const double r1 = __shfl_sync(~0u, rcp, 0), r2 = p11 * __shfl_sync(~0u, rcp, 16);  // 1 / p2 = p11 / det
+    const double l = p12 * r1;
     da = lane == k ? 1.0 : lane == k + 1 ? 0.0 : da;
     db = lane == k ? 0.0 : lane == k + 1 ? 1.0 : db;
-    pa[j][lane] = fma(p22, da, -p12 * db) * inv;
-    pb[j][lane] = fma(p11, db, -p12 * da) * inv;
+    const double wb = fma(-l, da, db);
+    ra[j][lane] = da;
+    rw[j][lane] = wb;
+    pa[j][lane] = da * r1;
+    pb[j][lane] = wb * r2;
     if (lane == 0) {
       pv[k] = p11;
       pv[k + 1] = det;  // over p11 below
+      lp[j] = l;
       l2[j] = p12;
     }
+    __syncwarp();  // this warp does not wait at the barrier it arrives at
     asm volatile("bar.arrive %0, 128;" ::"r"(1 + (j & 7)) : "memory");
   };
   if (w == 0) publish(0, d[0], d[1]);
@@ -666,16 +685,14 @@ __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) 
   for (int ss = 0; ss < 4; ++ss) {
 #pragma unroll 1
     for (int ww = 0; ww < 4; ++ww) {
-      const int j = 4 * ss + ww, k = 2 * j;
+      const int j = 4 * ss + ww;
       if (w != ww) asm volatile("bar.sync %0, 128;" ::"r"(1 + (j & 7)) : "memory");
       const double qa = pa[j][lane], qb = pb[j][lane];
       const bool piv = (lane >> 1) == j;
+      // a row's entries in the pivot columns are the pivot rows' in its own (symmetry)
       auto update = [&](int t) {
-        const double f1 = __shfl_sync(~0u, d[t], k), f2 = __shfl_sync(~0u, d[t], k + 1);
         const int r = 2 * (w + 4 * (t >> 1)) + (t & 1);
-        if (lane == k) Lm[r][k] = f1;
-        if (lane == k + 1) Lm[r][k + 1] = f2;
-        d[t] = fma(-f2, qb, fma(-f1, qa, piv ? 0.0 : d[t]));
+        d[t] = fma(-rw[j][r], qb, fma(-ra[j][r], qa, piv ? 0.0 : d[t]));
       };
       // the next pivot's rows first, and their pivot, before the other rows
       if (w > ww) {
@@ -716,70 +733,76 @@ __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) 
   }
   __syncthreads();
   pdl_launch();
-  // groups of 16 rows: lane = (row, half of the columns)
   for (; g < ng; g += gridDim.x) {
-    const int r0 = g * 16;
+    const int r = g * 16 + row;
     const bool below = g > gk + 1, left = g < gk;
-    // V[l][row]
+    double x[4];
+    if (below || left) {
+      // x L_kk' = v by forward substitution, a pivot pair at a time
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (below) V[lane][w + 4 * i] = pre[i];
-      else V[2 * w + half + 8 * i][row] = pre[i];
-    }
-    __syncthreads();
-    if (g + (int)gridDim.x < ng) fetch(g + gridDim.x);
-    const int c0 = 2 * w + half;  // columns c0 + 8 j
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int m = 0; m < 4; ++m) x[m] = pre[m];
+      if (g + (int)gridDim.x < ng) fetch(g + gridDim.x);
 #pragma unroll
-    for (int l = 0; l < 32; ++l) {
-      const double v = V[l][row];
+      for (int ss = 0; ss < 4; ++ss) {
+#pragma unroll 1
+        for (int ww = 0; ww < 4; ++ww) {
+          const int j = 4 * ss + ww, src = (lane & 24) + 2 * ww;
+          const double f1 = __shfl_sync(~0u, x[ss], src), f2 = __shfl_sync(~0u, x[ss], src + 1);
+          const double f = fma(-lp[j], f1, f2);
+          if (ww < 3) {
+            const double t = fma(-f, pb[j][c + 8 * ss], fma(-f1, pa[j][c + 8 * ss], x[ss]));
+            x[ss] = c > 2 * ww + 1 ? t : x[ss];
+          }
+          if (c == 2 * ww + 1) x[ss] = f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (l <= 8 * j + 7) acc[j] = fma(v, X[c0 + 8 * j][l], acc[j]);
-    }
-    __syncthreads();
-    int e = EX_MIN;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      V[c0 + 8 * j][row] = acc[j];
-      if (acc[j] != 0.0) e = max(e, expo(acc[j]));
-    }
-    mx[w][lane] = e;
-    __syncthreads();
-    if (tid < 64) {  // (row, K group)
-      const int rr = tid & 15, kg = tid >> 4, r = r0 + rr;
-      e = EX_MIN;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) e = max(e, max(mx[i][rr], mx[i][rr + 16]));
-      if (kg == 0) {
-        a.ex[r] = e;
-        a.exo[r] = (a.k0 == a.K0 || !(below || left)) ? e : max(e, a.exo[r]);
-        if (a.inverse && !below) a.exm[r] = left ? max(e, a.exm[r]) : e;
+          for (int m = ss + 1; m < 4; ++m) x[m] = fma(-f, pb[j][c + 8 * m], fma(-f1, pa[j][c + 8 * m], x[m]));
+        }
       }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) x[m] *= (c & 1) ? i2[(c >> 1) + 4 * m] : i1[(c >> 1) + 4 * m];
+    } else {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) x[m] = X[c + 8 * m][r - a.k0];
+      if (g + (int)gridDim.x < ng) fetch(g + gridDim.x);
+    }
+    int e = EX_MIN;
+    __syncwarp();  // V's last readers
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      V[w][c + 8 * m][lane >> 3] = x[m];
+      if (x[m] != 0.0) e = max(e, expo(x[m]));
+      if (below) {
+        a.P[(int64_t)r * a.B + (a.k0 - a.K0) + c + 8 * m] = x[m];
+        a.W[(int64_t)r * np + a.k0 + c + 8 * m] = a.inverse ? 0.0 : x[m];
+      } else if (left) {
+        a.W[(int64_t)(a.k0 + c + 8 * m) * np + r] = x[m];
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) e = max(e, __shfl_xor_sync(~0u, e, o));
+    if (c == 0) {
+      a.ex[r] = e;
+      a.exo[r] = (a.k0 == a.K0 || !(below || left)) ? e : max(e, a.exo[r]);
+      if (a.inverse && !below) a.exm[r] = left ? max(e, a.exm[r]) : e;
+    }
+    __syncwarp();
+    if (c < 4) {  // K group c of the row
       double v8[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v8[i] = V[kg * 8 + i][rr];
-      put_digits(v8, e, a.dig + (size_t)(r0 / 128) * BLK, r & 127, kg);
-    } else if (below) {
-      for (int i = w - 2; i < 16; i += 2) {
-        const double l = V[lane][i];
-        a.P[(int64_t)(r0 + i) * a.B + (a.k0 - a.K0) + lane] = l;
-        a.W[(int64_t)(r0 + i) * np + a.k0 + lane] = a.inverse ? 0.0 : l;
-      }
-    } else if (left) {
-      for (int l = 2 * (w - 2) + half; l < 32; l += 4) a.W[(int64_t)(a.k0 + l) * np + r0 + row] = V[l][row];
-    } else {
-      for (int i = w - 2; i < 16; i += 2) {
-        const int l = r0 - a.k0 + i, j = lane >> 1;
-        double x = X[l][lane];
+      for (int i = 0; i < 8; ++i) v8[i] = V[w][c * 8 + i][lane >> 3];
+      put_digits(v8, e, a.dig + (size_t)(r / 128) * BLK, r & 127, c);
+    }
+    if (!below && !left) {
+      for (int i = 0; i < 4; ++i) {
+        const int l = g * 16 + 4 * w + i - a.k0, j = lane >> 1;
+        double y = X[l][lane];
         if (!a.inverse) {
-          if ((l >> 1) == j) x = (l & 1) == 0 ? pv[l] * i1[j] : (lane & 1) ? pv[l] * i2[j] : l2[j];
-          else if (lane < l) x = (lane & 1) ? (Lm[l][lane] - Lm[l][lane - 1] * i1[j] * l2[j]) * i2[j] : Lm[l][lane] * i1[j];
+          if ((l >> 1) == j) y = (l & 1) == 0 ? pv[l] * i1[j] : (lane & 1) ? pv[l] * i2[j] : l2[j];
+          else if (lane < l) y = (lane & 1) ? rw[j][l] * i2[j] : ra[j][l] * i1[j];
         }
-        a.D[(a.k0 + l) * 32 + lane] = lane <= l ? x : 0.0;
+        a.D[(a.k0 + l) * 32 + lane] = lane <= l ? y : 0.0;
       }
     }
-    __syncthreads();
   }
 }
 
