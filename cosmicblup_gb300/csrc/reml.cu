@@ -1481,7 +1481,7 @@ __global__ void k_add_lowrank(double* __restrict__ A, int64_t n, const double* _
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = idx % n, c = idx / n;
     double a = 0.0;
-    for (int i = 0; i < k; ++i) a += w[i] * U[(int64_t)i * n + r] * U[(int64_t)i * n + c];
+    for (int i = 0; i < k; ++i) a = fma(w[i], U[(int64_t)i * n + r] * U[(int64_t)i * n + c], a);
     A[idx] += a;
   }
 }
@@ -1493,9 +1493,11 @@ __global__ void k_add_lowrank(double* __restrict__ A, int64_t n, const double* _
 //  * lambda_max <= ||M||_inf, so eps = 1e-6 whenever 1e-12 ||M||_inf <= 1e-6;
 //  * if every eigenvalue is above eps (M^-1 bounds them from below, or M - eps I has a
 //    Cholesky factor) none is raised and the result is M^-1 (Cholesky inverse);
-//  * otherwise only the eigenpairs below eps are computed (syevdx), M is raised
-//    to M + sum (eps - lambda_i) u_i u_i^T, whose eigenvalues are all >= eps,
-//    and that is inverted by Cholesky.
+//  * otherwise only the eigenpairs below eps are computed (syevdx), M is lifted
+//    to M + sum (c - lambda_i) u_i u_i^T, c = ||M||_inf, and that is inverted by
+//    Cholesky; sum (1/eps - 1/c) u_i u_i^T is added to the inverse.  (Raised to eps
+//    itself, the eigenvalues would carry the rounding of sums of the size of M and of
+//    lambda_i: 1e-9 to 1e-7 of the inverse for a GRM less 0.01 to 0.2, now 1e-13.)
 //  * when the all-ones direction is (nearly) null -- every VanRaden G, whose
 //    centred columns sum to zero -- the one eigenpair below eps and the inverse off it
 //    come from one inverse of M plus a rank-1 term (deflate_ones below).
@@ -1569,7 +1571,10 @@ __global__ void k_deflated(const double* __restrict__ N, int64_t n, const double
 //     so Mr's second smallest is above 100 eps too, and the smallest is the only one
 //     raised;
 //  2. its eigenvector u from (Mr + c v v') u = rho u + c (v'u) v: each step
-//     u <- N (rho u + c (v'u) v) shrinks the error by rho / lambda_2 < 1e-2;
+//     u <- N (rho u + c (v'u) v) multiplies the error by |rho| / lambda_i, i >= 2.  That
+//     shrinks it a hundredfold for |rho| < eps, but a negative rho of a larger magnitude can
+//     make it grow: the steps are taken, until the error is below 1e-16, while |rho| is
+//     below a quarter of the bound of step 1, and the residual of what they give is checked;
 //  3. with P = I - u u', w = N u, a = P w: P N P + rho / (1 - rho u'w) a a' is the inverse
 //     of Mr on the complement of u, and u u' / eps is added.
 // Returns false, with out_dev untouched, when step 1 or 2 fails.  N's condition is that of
@@ -1594,7 +1599,7 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
   k_add_lowrank<<<grid, 256, 0, s>>>(T.p, n, v.p, w1.p, 1);
   h->launched("k_add_lowrank");
   if (!fx64_cholesky(h, T.p, n, true, N.p, nullptr)) return false;
-  double ninf = 0.0;
+  double ninf = 0.0;  // in the end a bound of 1 / lambda_2
   k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(N.p, n, y.p);
   h->launched("k_col_abs_sum");
   for (double t : d2h(h, y.p, n)) ninf = std::isfinite(t) ? std::max(ninf, t) : HUGE_VAL;
@@ -1602,6 +1607,7 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
     k_add_ridge_copy<<<grid, 256, 0, s>>>(T.p, n, -100.0 * eps, T.p);
     h->launched("k_add_ridge_copy");
     if (!fx64_cholesky(h, T.p, n, false, nullptr, nullptr)) return false;
+    ninf = 1.0 / (100.0 * eps);
   }
   auto dot = [&](const double* a, const double* b) {
     double t = 0.0;
@@ -1611,7 +1617,7 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
   // u <- N v normalised (exact when rho = 0), then the steps of 2.
   CBX_CUDA(cudaMemcpyAsync(u.p, v.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   double rho = 0.0;
-  for (int it = 0; it < 8; ++it) {
+  for (int it = 0; it < 32; ++it) {
     const double vu = dot(v.p, u.p) * c;
     CBX_BLAS(cublasDscal(L.blas, ni, &rho, u.p, 1));
     CBX_BLAS(cublasDaxpy(L.blas, ni, &vu, v.p, 1, u.p, 1));
@@ -1623,9 +1629,16 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
     std::swap(u.p, y.p);
     symv(h, out_dev, n, u.p, nullptr, false, y.p);
     rho = dot(u.p, y.p);
-    if (std::abs(rho) < 1e-12 && it > 0) break;  // the next step would move u by less than 1e-8 of its error
+    const double q = std::abs(rho) * ninf;
+    if (!(q < 0.25)) return false;
+    if (it > 0 && std::pow(q, it + 1) < 1e-16) break;
   }
   if (!(rho < eps)) return false;
+  // Mr u - rho u: rounding leaves up to 7 n 2^-53 ||Mr||_inf (lambda_2 = 200 eps), a direction
+  // that is no eigenvector many times that
+  const double neg_rho = -rho;
+  CBX_BLAS(cublasDaxpy(L.blas, ni, &neg_rho, u.p, 1, y.p, 1));
+  if (!(std::sqrt(dot(y.p, y.p)) <= 32.0 * (double)n * 0x1p-53 * c)) return false;
   symv(h, N.p, n, u.p, nullptr, false, y.p);
   const double uw = dot(u.p, y.p), beta = rho / (1.0 - rho * uw);
   k_deflated<<<grid, 256, 0, s>>>(N.p, n, u.p, y.p, uw, uw + 1.0 / eps, beta, out_dev);
@@ -1698,7 +1711,7 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
   CBX_CUDA(cudaMemcpyAsync(T.p, out_dev, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   DevBuf<double> w;
   w.resize(n);
-  const double vl = -rinf - 1.0, vu = std::nextafter(eps, 0.0);
+  const double vl = -rinf - 1.0, vu = std::nextafter(eps, 0.0), c = rinf > 0.0 ? rinf : 1.0;
   int meig = 0, lw = 0;
   CBX_SOLVER(cusolverDnDsyevdx_bufferSize(L.sol, CUSOLVER_EIG_MODE_VECTOR, CUSOLVER_EIG_RANGE_V,
                                           CUBLAS_FILL_MODE_LOWER, (int)n, T.p, (int)n, vl, vu, 0, 0, &meig, w.p,
@@ -1720,12 +1733,22 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
   }
   if (meig > 0) {
     std::vector<double> wh = d2h(h, w.p, meig);
-    for (auto& v : wh) v = eps - v;
+    for (auto& v : wh) v = c - v;
     CBX_CUDA(cudaMemcpyAsync(w.p, wh.data(), meig * sizeof(double), cudaMemcpyHostToDevice, s));
     k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, T.p, w.p, meig);
     h->launched("k_add_lowrank");
   }
-  if (!chol_inverse_device(h, out_dev, n)) invert_psd_full(h, M_dev, n, ridge, out_dev);
+  if (!chol_inverse_device(h, out_dev, n)) {
+    invert_psd_full(h, M_dev, n, ridge, out_dev);
+    return;
+  }
+  if (meig > 0) {
+    std::vector<double> wh(meig, 1.0 / eps - 1.0 / c);
+    CBX_CUDA(cudaMemcpyAsync(w.p, wh.data(), meig * sizeof(double), cudaMemcpyHostToDevice, s));
+    k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, T.p, w.p, meig);
+    h->launched("k_add_lowrank");
+    CBX_CUDA(cudaStreamSynchronize(s));  // wh, w and T go out of scope
+  }
 }
 
 // In-place inverse of an SPD device matrix by Cholesky; false if not PD (A unchanged).
