@@ -398,23 +398,8 @@ static void host_inverse(int t, const double* A, double* Ai) {
   std::copy(I.begin(), I.end(), Ai);
 }
 
-// R = I - T (n x n)
-__global__ void k_mt_residual(double* __restrict__ T, int64_t n) {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * n; idx += (int64_t)gridDim.x * blockDim.x)
-    T[idx] = (idx / n == idx % n ? 1.0 : 0.0) - T[idx];
-}
-// G += (C + C') / 2 (n x n)
-__global__ void k_mt_add_sym(const double* __restrict__ C, int64_t n, double* __restrict__ G) {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * n; idx += (int64_t)gridDim.x * blockDim.x)
-    G[idx] += 0.5 * (C[idx] + C[idx % n * n + idx / n]);
-}
-
 // G from the handle's device G^-1 (the reference recovers G by an LDLT solve
-// of G^-1 against I), or uploaded from the host.  A raised eigenvalue of 1e-6 makes
-// G^-1's condition 1e6 and more: the factorization's rows come from inverses of its pivot
-// blocks, which loses the root of the first block's condition (1e-9 of G at n = 320), so
-// one Newton step G (2 I - G^-1 G) follows: two products, whose error is that of rounding
-// G^-1 itself.
+// of G^-1 against I), or uploaded from the host.
 static void load_g(cbx_handle* h, const double* G, int64_t n, DevBuf<double>& Gd) {
   cudaStream_t s = h->stream;
   Gd.resize((size_t)n * n);
@@ -426,21 +411,6 @@ static void load_g(cbx_handle* h, const double* G, int64_t n, DevBuf<double>& Gd
   CBX_CUDA(cudaMemcpyAsync(Gd.p, h->Ginv.p, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   CBX_REQUIRE(chol_inverse_device(h, Gd.p, n), CBX_ERR_FACTOR,
               "G^-1 is not positive-definite; cannot recover G");
-  DevBuf<double> R, C;
-  R.resize((size_t)n * n);
-  C.resize((size_t)n * n);
-  const unsigned grid = gridn(n * n, 256, 8 * h->num_sms);
-  FxPanel A, B;
-  fx64_digits(h, A, h->Ginv.p, n, n, n, false);
-  fx64_digits(h, B, Gd.p, n, n, n, false);
-  fx64_gemm(h, A, B, n, n, R.p, n);
-  k_mt_residual<<<grid, 256, 0, s>>>(R.p, n);
-  h->launched("k_mt_residual");
-  fx64_digits(h, A, R.p, n, n, n, true);
-  fx64_gemm(h, B, A, n, n, C.p, n);
-  k_mt_add_sym<<<grid, 256, 0, s>>>(C.p, n, Gd.p);
-  h->launched("k_mt_add_sym");
-  CBX_CUDA(cudaStreamSynchronize(s));  // the buffers go out of scope
 }
 
 template <int T>

@@ -780,45 +780,6 @@ static void reml_gradient(cbx_handle* h, double vu, double ve, int nprobe, int s
 
 // ---------------------------------------------------------------------------
 // dense exact AI step
-// upper triangle of a column-major n x n matrix from its lower one
-__global__ void k_dense_mirror(double* __restrict__ A, int64_t n) {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * n; idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = idx % n, c = idx / n;
-    if (r < c) A[idx] = A[r * n + c];
-  }
-}
-// Inverse and log-determinant of a symmetric matrix.  An eigen-bent Qinv holds 1e6 / n in
-// every entry, and the digit factorization loses the root of its first pivot block's
-// condition: variances off by 3.5e-9 at n = 301 (1.6e-11 by cuSOLVER), 4e-10 at 700, 1e-11 at
-// 2,000.  Up to kDenseLib it is cuSOLVER's (about 4 ms at n = 500, 0.63 by digits).
-constexpr int64_t kDenseLib = 1024;
-static bool dense_inverse(cbx_handle* h, const double* A, int64_t n, double* out, double* logdet) {
-  if (n > kDenseLib) return fx64_cholesky(h, A, n, true, out, logdet);
-  cudaStream_t s = h->stream;
-  Libs& L = libs(h);
-  if (A != out) CBX_CUDA(cudaMemcpyAsync(out, A, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  int l1 = 0, l2 = 0;
-  CBX_SOLVER(cusolverDnDpotrf_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, out, (int)n, &l1));
-  CBX_SOLVER(cusolverDnDpotri_bufferSize(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, out, (int)n, &l2));
-  DevBuf<double> work;
-  work.resize(std::max({l1, l2, 1}));
-  DevBuf<int> info;
-  info.resize(1);
-  CBX_SOLVER(cusolverDnDpotrf(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, out, (int)n, work.p, l1, info.p));
-  if (d2h(h, info.p, 1)[0] != 0) return false;
-  std::vector<double> d(n);
-  CBX_CUDA(cudaMemcpy2DAsync(d.data(), sizeof(double), out, (n + 1) * sizeof(double), sizeof(double), n,
-                             cudaMemcpyDeviceToHost, s));
-  CBX_CUDA(cudaStreamSynchronize(s));
-  *logdet = 0.0;
-  for (double v : d) *logdet += 2.0 * std::log(v);
-  CBX_SOLVER(cusolverDnDpotri(L.sol, CUBLAS_FILL_MODE_LOWER, (int)n, out, (int)n, work.p, l2, info.p));
-  if (d2h(h, info.p, 1)[0] != 0) return false;
-  k_dense_mirror<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out, n);
-  h->launched("k_dense_mirror");
-  CBX_CUDA(cudaStreamSynchronize(s));
-  return true;
-}
 struct DenseExact {
   bool init = false;
   int64_t n = 0, dim = 0;
@@ -868,7 +829,7 @@ static void dense_init(cbx_handle* h, DenseExact& D) {
   A.resize((size_t)q * q);
   CBX_CUDA(cudaMemcpy2DAsync(A.p, q * sizeof(double), m.Qd64.p, m.ld * sizeof(double), q * sizeof(double), q,
                              cudaMemcpyDeviceToDevice, s));
-  CBX_REQUIRE(dense_inverse(h, A.p, q, A.p, &D.log_det_A), CBX_ERR_FACTOR, "Qinv is not positive definite");
+  CBX_REQUIRE(fx64_cholesky(h, A.p, q, true, A.p, &D.log_det_A), CBX_ERR_FACTOR, "Qinv is not positive definite");
   D.log_det_A = -D.log_det_A;
   D.ZAZt.resize((size_t)n * n);
   k_build_zazt<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(n, q, m.aid.p, A.p, D.ZAZt.p);
@@ -939,7 +900,7 @@ static double dense_logL(cbx_handle* h, DenseExact& D, double vu, double ve) {
   build_lhs(h, ve / vu, D.C);
   D.Ci.resize((size_t)dim * dim);
   double ld_C = 0.0;
-  if (!dense_inverse(h, D.C.p, dim, D.Ci.p, &ld_C)) return -1e18;
+  if (!fx64_cholesky(h, D.C.p, dim, true, D.Ci.p, &ld_C)) return -1e18;
   if (!std::isfinite(ld_C)) return -1e18;
   solve_by_inverse(h, D.C.p, D.Ci.p, dim, m.rhs.p, D.sol);
   DevBuf<double> e;
