@@ -31,6 +31,20 @@ struct DevBuf {
     if (count) CBX_CUDA(cudaMalloc(&p, count * sizeof(T)));
     n = count;
   }
+  // resize, or false (and empty) where the memory does not hold it
+  bool try_resize(size_t count) {
+    if (count == n && p) return true;
+    release();
+    const cudaError_t e = count ? cudaMalloc(&p, count * sizeof(T)) : cudaSuccess;
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    CBX_CUDA(e);
+    n = count;
+    return true;
+  }
   void zero(cudaStream_t s) {
     if (n) CBX_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }

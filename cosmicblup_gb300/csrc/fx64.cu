@@ -558,14 +558,14 @@ __global__ void __launch_bounds__(256) k_slices(const double* __restrict__ part,
 // ---- Cholesky ------------------------------------------------------------------
 // The factorization runs on D A D, D_ii = 2^-k_i with 4^k_i <= A_ii < 4^(k_i + 1): its entries
 // are below 4, so that no 2 x 2 determinant over- or underflows, and the scaling is exact.
-__global__ void k_scales(const double* __restrict__ A, int64_t n, int64_t np, int32_t* __restrict__ sc) {
+__global__ void k_scales(const double* __restrict__ A, int64_t n, int64_t np, FxAdd add, int32_t* __restrict__ sc) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= np) return;
-  const double v = i < n ? A[i * n + i] : 1.0;
+  const double v = i < n ? A[i * n + i] + add.diag + add.all : 1.0;
   sc[i] = v > 0.0 && isfinite(v) ? ilogb(v) >> 1 : 0;
 }
 // W (np x np row-major) = lower triangle of D A D (A column-major), identity on the padding
-__global__ void __launch_bounds__(256) k_load_lower(const double* __restrict__ A, int64_t n, int64_t np,
+__global__ void __launch_bounds__(256) k_load_lower(const double* __restrict__ A, int64_t n, int64_t np, FxAdd add,
                                                     const int32_t* __restrict__ sc, double* __restrict__ W) {
   __shared__ double t[32][33];
   const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;
@@ -573,7 +573,9 @@ __global__ void __launch_bounds__(256) k_load_lower(const double* __restrict__ A
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   for (int c = y; c < 32; c += 8) {
     const int64_t i = i0 + x, j = j0 + c;
-    t[c][x] = (i < n && j < n) ? A[j * n + i] * pow2d(max(-1022, min(1023, -sc[i] - sc[j]))) : (i == j ? 1.0 : 0.0);
+    t[c][x] = (i < n && j < n)
+                  ? (A[j * n + i] + (i == j ? add.diag : 0.0) + add.all) * pow2d(max(-1022, min(1023, -sc[i] - sc[j])))
+                  : (i == j ? 1.0 : 0.0);
   }
   __syncthreads();
   for (int r = y; r < 32; r += 8) W[(i0 + r) * np + j0 + x] = t[x][r];
@@ -624,8 +626,8 @@ __device__ __forceinline__ double reciprocal(double d) {
 // condition where two adjacent rows are near-duplicates.  Measured with the pair's inverse
 // and X before, both this way now: factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81, now 2.84;
 // at 8,000 18.3, now 18.2, and 34.4, now 35.0 (a substitution issues 92 FP64 instructions a
-// warp and group, the product 80).  L L' - A at n = 96 with adjacent rows 1e-3 apart: 0.02 of 4 n u,
-// before above it 200 times, and at 1e-5 apart no pivot was found.
+// warp and group, the product 80).  L L' - A at n = 96 with adjacent rows 1e-3 apart: 0.01 of
+// 4 n u sqrt(A_ii A_jj), 1e5 times it before, when rows 1e-4 apart were found not positive definite.
 __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) {
   __shared__ double X[32][33], V[4][32][5], pa[16][32], pb[16][32], ra[16][32], rw[16][32];
   __shared__ double pv[32], lp[16], i1[16], l2[16], i2[16];
@@ -830,16 +832,18 @@ __global__ void __launch_bounds__(128) k_panel_digits(const __grid_constant__ Pa
     put_digits(v, e, blk, threadIdx.x, kg);
   }
 }
-// Digits of M' (row j = column j of M = L^-1, K steps from the row tile's own on)
-__global__ void __launch_bounds__(128) k_minv_digits(const double* __restrict__ W, const double* __restrict__ D, int64_t np, int n, int ks,
+// Digits of M' (row j = column j of M = L^-1): all row tiles, each from its own K step on
+// (group 0), or `group` row tiles from rt0 on, all of K step ks0 on (zeros left of the diagonal)
+__global__ void __launch_bounds__(128) k_minv_digits(const double* __restrict__ W, const double* __restrict__ D, int64_t np,
+                                                     int n, int ks, int rt0, int ks0, int group,
                                                      const int32_t* __restrict__ ex, const int32_t* __restrict__ sc,
                                                      int32_t* __restrict__ exd, uint8_t* __restrict__ dig) {
-  const int rt = blockIdx.x, k0 = blockIdx.y;
-  if (k0 < 4 * rt) return;
+  const int rt = rt0 + blockIdx.x, k0 = ks0 + blockIdx.y;
+  if (!group && k0 < 4 * rt) return;
   const int r = rt * 128 + threadIdx.x;
   // A^-1 = D (M'M) D: the scaling goes into the product's exponents
   if (k0 == 4 * rt) exd[r] = r < n ? ex[r] - sc[r] : EX_MIN;
-  uint8_t* blk = dig + blk_of(rt, k0, ks, 1) * BLK;
+  uint8_t* blk = dig + (group ? (size_t)blockIdx.x * (ks - ks0) + blockIdx.y : blk_of(rt, k0, ks, 1)) * BLK;
   const int e = r < n ? ex[r] : EX_MIN;
 #pragma unroll
   for (int kg = 0; kg < 4; ++kg) {
@@ -882,14 +886,25 @@ __global__ void k_store_factor(const double* __restrict__ W, const double* __res
 constexpr size_t kKeepBytes = (size_t)1 << 30;
 struct Scratch {
   DevBuf<double> W, P, D, piv;
-  DevBuf<uint8_t> din, dout, dm;
+  DevBuf<uint8_t> din, dout, dm, dm2;
   DevBuf<int32_t> ex, exo, exm, sc;
   DevBuf<int> bad;
-  size_t bytes() const { return W.n * 8 + P.n * 8 + din.n + dout.n + dm.n; }
+  size_t bytes() const { return W.n * 8 + P.n * 8 + din.n + dout.n + dm.n + dm2.n; }
 };
 template <typename T>
 static void at_least(DevBuf<T>& b, size_t n) {
   if (b.n < n) b.resize(n);
+}
+// at_least for digits, or false where they do not fit
+static bool try_at_least(cbx_handle* h, DevBuf<uint8_t>& b, size_t n) {
+  if (h->fx_limit && n > h->fx_limit) return false;
+  return b.n >= n || b.try_resize(n);
+}
+// Row tiles of a group, where digits go by groups: 16 (2,048 rows, 512 output tiles of 64 columns a pair of
+// groups, 3.4 waves), fewer under a limit
+static int group_tiles(cbx_handle* h, int rt, int ks) {
+  const size_t row = (size_t)ks * BLK;
+  return (int)std::min<size_t>(rt, h->fx_limit ? std::max<size_t>(1, std::min<size_t>(16, h->fx_limit / row)) : 16);
 }
 static Scratch& scratch(cbx_handle* h) {
   if (!h->fx_slot) h->fx_slot = std::make_shared<Scratch>();
@@ -1022,7 +1037,49 @@ void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& p
   h->launched("k_slices");
 }
 
-bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet) {
+// out = M'M by pairs of row groups: the digits of two groups at a time, from the first group's
+// first K step on.  Every total is the same integer as with all digits at once.
+static void minv_product_groups(cbx_handle* h, fx::Scratch& S, int64_t np, int64_t n, double* out) {
+  cudaStream_t s = h->stream;
+  const int rt = (int)(np / 128), ks = (int)(np / 32), gt = fx::group_tiles(h, rt, ks);
+  const size_t most = (size_t)gt * ks * fx::BLK;
+  S.dm.release();
+  S.dm2.release();
+  S.dm.resize(most);
+  if (gt < rt) S.dm2.resize(most);
+  for (int ra = 0; ra < rt; ra += gt) {
+    const int na = std::min(gt, rt - ra), ks0 = 4 * ra;
+    auto digits = [&](int r0, int cnt, uint8_t* dst) {
+      fx::k_minv_digits<<<dim3(cnt, ks - ks0), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, r0, ks0, cnt, S.exm.p, S.sc.p,
+                                                           S.ex.p, dst);
+      h->launched("k_minv_digits");
+    };
+    digits(ra, na, S.dm.p);
+    for (int ca = 0; ca <= ra; ca += gt) {
+      if (ca < ra) digits(ca, gt, S.dm2.p);
+      fx::Job M{};
+      // the kernel's block (row tile, K step) is at row tile x (ks - ks0) + K step
+      auto base = [&](const uint8_t* p, int r0) {
+        return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) -
+                                                ((uintptr_t)r0 * (ks - ks0) + ks0) * fx::BLK);
+      };
+      M.A = base(S.dm.p, ra);
+      M.B = ca < ra ? base(S.dm2.p, ca) : M.A;
+      M.ea = M.eb = S.ex.p;
+      M.ka = M.kb = ks - ks0;
+      M.ks0 = ks0;
+      M.ks1 = ks;
+      M.seg[0] = {ra, ra + na, 4 * ca, 4 * (ca + gt), ca == ra ? 1 : 0, 0};
+      M.mode = 2;
+      M.m = M.n = (int)n;
+      M.C = out;
+      M.ldc = n;
+      fx::launch(h, M);
+    }
+  }
+}
+
+bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet, FxAdd add) {
   CBX_REQUIRE(n > 0 && n <= 130000, CBX_ERR_ARG, "matrix order out of range");
   cudaStream_t s = h->stream;
   fx::Scratch& S = fx::scratch(h);
@@ -1041,9 +1098,9 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
   fx::at_least(S.sc, (size_t)np);
   fx::at_least(S.bad, 1);
   CBX_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), s));
-  fx::k_scales<<<(unsigned)(np / 128), 128, 0, s>>>(A, n, np, S.sc.p);
+  fx::k_scales<<<(unsigned)(np / 128), 128, 0, s>>>(A, n, np, add, S.sc.p);
   h->launched("k_scales");
-  fx::k_load_lower<<<dim3((unsigned)(np / 32), (unsigned)(np / 32)), 256, 0, s>>>(A, n, np, S.sc.p, S.W.p);
+  fx::k_load_lower<<<dim3((unsigned)(np / 32), (unsigned)(np / 32)), 256, 0, s>>>(A, n, np, add, S.sc.p, S.W.p);
   h->launched("k_load_lower");
   fx::Panel a{S.W.p, np, 0, 0, 0, B, inverse ? 1 : 0, S.din.p, S.ex.p, S.exo.p, S.exm.p, S.P.p, S.D.p, S.piv.p,
               S.bad.p};
@@ -1092,10 +1149,12 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
   CBX_CUDA(cudaMemcpyAsync(&bad, S.bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   CBX_CUDA(cudaStreamSynchronize(s));
   h->check_status("FP64 factorization");
-  if (!bad && inverse) {
-    const int ks = (int)(np / 32);
-    fx::at_least(S.dm, ((size_t)rt * ks - 2 * (size_t)rt * (rt - 1)) * fx::BLK);
-    fx::k_minv_digits<<<dim3(rt, ks), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, S.exm.p, S.sc.p, S.ex.p, S.dm.p);
+  const int ks = (int)(np / 32);
+  if (!bad && inverse && !fx::try_at_least(h, S.dm, ((size_t)rt * ks - 2 * (size_t)rt * (rt - 1)) * fx::BLK)) {
+    minv_product_groups(h, S, np, n, out);
+  } else if (!bad && inverse) {
+    fx::k_minv_digits<<<dim3(rt, ks), 128, 0, s>>>(S.W.p, S.D.p, np, (int)n, ks, 0, 0, 0, S.exm.p, S.sc.p, S.ex.p,
+                                                   S.dm.p);
     h->launched("k_minv_digits");
     fx::Job M{};
     M.A = M.B = S.dm.p;

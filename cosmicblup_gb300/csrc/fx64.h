@@ -28,11 +28,18 @@ void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int
 void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,
                   const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active);
 
+// diag I + all 11' is added to a matrix on reading it
+struct FxAdd {
+  double diag = 0.0, all = 0.0;
+};
+
 // Cholesky of the symmetric n x n matrix A (column-major, its lower triangle is
-// read).  Returns false when a pivot is not positive.  logdet (may be null) gets
+// read).  Needs 8 n^2 bytes beside A and out, and up to 8 n^2 more for an inverse where the
+// memory has them.  Returns false when a pivot is not positive.  logdet (may be null) gets
 // log det A.  With inverse, out (may be A) receives the full symmetric A^-1;
 // otherwise, when out is given, out gets the factor U = L' (column-major upper
 // triangle, zeros below).
-bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet);
+bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet,
+                   FxAdd add = {});
 
 }  // namespace cbx

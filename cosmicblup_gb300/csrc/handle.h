@@ -61,6 +61,9 @@ struct cbx_handle {
   std::shared_ptr<void> dense_slot;
   // scratch of the FP64 factorizations (fx64.cu)
   std::shared_ptr<void> fx_slot;
+  // largest digit buffer in bytes (0: what the memory holds); work whose digits do not fit
+  // goes by row groups
+  size_t fx_limit = 0;
   // scratch of the device W'W assembly (wtw.cu), kept between MMEs
   std::shared_ptr<void> wtw_slot;
   // genotypes kept on the device by cbx_geno_attach (matrix-free Z / Z^T products)

@@ -1511,21 +1511,21 @@ static void invert_psd_full(cbx_handle* h, const double* M_dev, int64_t n, doubl
                        &zero, out_dev, (int)n));
 }
 
-// R = N - u w' - w u' + g u u' + beta a a'
-__global__ void k_deflated(const double* __restrict__ N, int64_t n, const double* __restrict__ u,
-                           const double* __restrict__ w, double uw, double g, double beta, double* __restrict__ R) {
+// N - u w' - w u' + g u u' + beta a a' in N's place, a = w - uw u
+__global__ void k_deflated(double* __restrict__ N, int64_t n, const double* __restrict__ u, const double* __restrict__ w,
+                           double uw, double g, double beta) {
   const int64_t total = n * n;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = idx % n, c = idx / n;
     const double ur = u[r], uc = u[c], wr = w[r], wc = w[c];
-    // the two rank-1 terms are added first and a a' is symmetric, so R is too
-    R[idx] = (N[idx] - (ur * wc + wr * uc)) + (g * (ur * uc) + beta * ((wr - uw * ur) * (wc - uw * uc)));
+    // the two rank-1 terms are added first and a a' is symmetric, so the result is too
+    N[idx] = (N[idx] - (ur * wc + wr * uc)) + (g * (ur * uc) + beta * ((wr - uw * ur) * (wc - uw * uc)));
   }
 }
 
-// One eigenvalue of Mr (M + ridge I, in out_dev) below eps, along a direction
-// close to v = 1/sqrt(n) (v'Mr v < eps), from one inverse N = (Mr + c v v')^-1:
+// One eigenvalue of Mr = M + ridge I below eps, along a direction close to
+// v = 1/sqrt(n) (v'Mr v < eps), from one inverse N = (Mr + c v v')^-1:
 //  1. check: every eigenvalue of Mr + c v v' is above 100 eps -- 1 / ||N||_inf is a
 //     lower bound of them, and where that is too low a Cholesky factor of
 //     Mr + c v v' - 100 eps I decides.  A rank-1 term moves no eigenvalue past the next,
@@ -1538,36 +1538,29 @@ __global__ void k_deflated(const double* __restrict__ N, int64_t n, const double
 //     below a quarter of the bound of step 1, and the residual of what they give is checked;
 //  3. with P = I - u u', w = N u, a = P w: P N P + rho / (1 - rho u'w) a a' is the inverse
 //     of Mr on the complement of u, and u u' / eps is added.
-// Returns false, with out_dev untouched, when step 1 or 2 fails.  N's condition is that of
-// Mr off its null direction, so the result keeps the digits that inverting the raised
-// matrix (condition 1e6 and more) would lose.
-static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double* out_dev) {
+// Returns false, with out_dev (which holds N) no longer of use, when step 1 or 2 fails.  N's
+// condition is that of Mr off its null direction, so the result keeps the digits that
+// inverting the raised matrix (condition 1e6 and more) would lose.
+static bool deflate_ones(cbx_handle* h, const double* M_dev, int64_t n, double ridge, double eps, double c,
+                         double* out_dev) {
   cudaStream_t s = h->stream;
   Libs& L = libs(h);
   const int ni = (int)n;
   const unsigned grid = gridn(n * n, 256, 8 * h->num_sms);
-  DevBuf<double> T, N, u, v, y, w1;
-  T.resize((size_t)n * n);
-  N.resize((size_t)n * n);
+  DevBuf<double> u, v, y;
   u.resize(n);
   v.resize(n);
   y.resize(n);
-  w1.resize(1);
-  std::vector<double> x(n, 1.0 / std::sqrt((double)n));
+  const double v1 = 1.0 / std::sqrt((double)n), cvv = c * v1 * v1;
+  std::vector<double> x(n, v1);
   CBX_CUDA(cudaMemcpyAsync(v.p, x.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
-  CBX_CUDA(cudaMemcpyAsync(w1.p, &c, sizeof(double), cudaMemcpyHostToDevice, s));
-  CBX_CUDA(cudaMemcpyAsync(T.p, out_dev, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  k_add_lowrank<<<grid, 256, 0, s>>>(T.p, n, v.p, w1.p, 1);
-  h->launched("k_add_lowrank");
-  if (!fx64_cholesky(h, T.p, n, true, N.p, nullptr)) return false;
+  if (!fx64_cholesky(h, M_dev, n, true, out_dev, nullptr, {ridge, cvv})) return false;
   double ninf = 0.0;  // in the end a bound of 1 / lambda_2
-  k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(N.p, n, y.p);
+  k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(out_dev, n, y.p);
   h->launched("k_col_abs_sum");
   for (double t : d2h(h, y.p, n)) ninf = std::isfinite(t) ? std::max(ninf, t) : HUGE_VAL;
   if (!(ninf < 0.99 / (100.0 * eps))) {
-    k_add_ridge_copy<<<grid, 256, 0, s>>>(T.p, n, -100.0 * eps, T.p);
-    h->launched("k_add_ridge_copy");
-    if (!fx64_cholesky(h, T.p, n, false, nullptr, nullptr)) return false;
+    if (!fx64_cholesky(h, M_dev, n, false, nullptr, nullptr, {ridge - 100.0 * eps, cvv})) return false;
     ninf = 1.0 / (100.0 * eps);
   }
   auto dot = [&](const double* a, const double* b) {
@@ -1582,13 +1575,14 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
     const double vu = dot(v.p, u.p) * c;
     CBX_BLAS(cublasDscal(L.blas, ni, &rho, u.p, 1));
     CBX_BLAS(cublasDaxpy(L.blas, ni, &vu, v.p, 1, u.p, 1));
-    symv(h, N.p, n, u.p, nullptr, false, y.p);
+    symv(h, out_dev, n, u.p, nullptr, false, y.p);
     const double nrm = std::sqrt(dot(y.p, y.p));
     if (!(nrm > 0.0) || !std::isfinite(nrm)) return false;
     const double sc = 1.0 / nrm;
     CBX_BLAS(cublasDscal(L.blas, ni, &sc, y.p, 1));
     std::swap(u.p, y.p);
-    symv(h, out_dev, n, u.p, nullptr, false, y.p);
+    symv(h, M_dev, n, u.p, nullptr, false, y.p);
+    CBX_BLAS(cublasDaxpy(L.blas, ni, &ridge, u.p, 1, y.p, 1));
     rho = dot(u.p, y.p);
     const double q = std::abs(rho) * ninf;
     if (!(q < 0.25)) return false;
@@ -1600,11 +1594,11 @@ static bool deflate_ones(cbx_handle* h, int64_t n, double eps, double c, double*
   const double neg_rho = -rho;
   CBX_BLAS(cublasDaxpy(L.blas, ni, &neg_rho, u.p, 1, y.p, 1));
   if (!(std::sqrt(dot(y.p, y.p)) <= 32.0 * (double)n * 0x1p-53 * c)) return false;
-  symv(h, N.p, n, u.p, nullptr, false, y.p);
+  symv(h, out_dev, n, u.p, nullptr, false, y.p);
   const double uw = dot(u.p, y.p), beta = rho / (1.0 - rho * uw);
-  k_deflated<<<grid, 256, 0, s>>>(N.p, n, u.p, y.p, uw, uw + 1.0 / eps, beta, out_dev);
+  k_deflated<<<grid, 256, 0, s>>>(out_dev, n, u.p, y.p, uw, uw + 1.0 / eps, beta);
   h->launched("k_deflated");
-  CBX_CUDA(cudaStreamSynchronize(s));  // N and T go out of scope
+  CBX_CUDA(cudaStreamSynchronize(s));  // u, v and y go out of scope
   return true;
 }
 
@@ -1640,37 +1634,26 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
     CBX_BLAS(cublasDgemv(L.blas, CUBLAS_OP_N, ni, ni, &one, out_dev, ni, v.p, 1, &zero, y.p, 1));
     double rho0 = 0.0;
     CBX_BLAS(cublasDdot(L.blas, ni, v.p, 1, y.p, 1, &rho0));
-    if (rho0 < eps && deflate_ones(h, n, eps, rinf > 0.0 ? rinf : 1.0, out_dev)) return;
+    if (rho0 < eps && deflate_ones(h, M_dev, n, r, eps, rinf > 0.0 ? rinf : 1.0, out_dev)) return;
   }
-  DevBuf<double> T;
-  T.resize((size_t)n * n);
   // no eigenvalue below eps: 1 / ||M^-1||_inf, a lower bound of a positive definite M's
   // eigenvalues, is above it, or M - eps I is positive definite
-  if (fx64_cholesky(h, out_dev, n, true, T.p, nullptr)) {
+  if (fx64_cholesky(h, M_dev, n, true, out_dev, nullptr, {r, 0.0})) {
     DevBuf<double> cs;
     cs.resize(n);
-    k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(T.p, n, cs.p);
+    k_col_abs_sum<<<(unsigned)n, 256, 0, s>>>(out_dev, n, cs.p);
     h->launched("k_col_abs_sum");
     double ninf = 0.0;
     for (double v : d2h(h, cs.p, n)) ninf = std::isfinite(v) ? std::max(ninf, v) : HUGE_VAL;
-    bool all_above = ninf < 0.99 / eps;
-    if (!all_above) {
-      DevBuf<double> U;
-      U.resize((size_t)n * n);
-      k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, -eps, U.p);
-      h->launched("k_add_ridge_copy");
-      all_above = fx64_cholesky(h, U.p, n, false, nullptr, nullptr);
-    }
-    if (all_above) {
-      CBX_CUDA(cudaMemcpyAsync(out_dev, T.p, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      CBX_CUDA(cudaStreamSynchronize(s));  // T goes out of scope
-      return;
-    }
+    if (ninf < 0.99 / eps || fx64_cholesky(h, M_dev, n, false, nullptr, nullptr, {r - eps, 0.0})) return;
   }
+  k_add_ridge_copy<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(M_dev, n, r, out_dev);
+  h->launched("k_add_ridge_copy");
   // the eigenpairs below eps: lambda in (-||M||_inf - 1, eps)
   Libs& L = libs(h);
+  DevBuf<double> T, U, w;
+  T.resize((size_t)n * n);
   CBX_CUDA(cudaMemcpyAsync(T.p, out_dev, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  DevBuf<double> w;
   w.resize(n);
   const double vl = -rinf - 1.0, vu = std::nextafter(eps, 0.0), c = rinf > 0.0 ? rinf : 1.0;
   int meig = 0, lw = 0;
@@ -1698,7 +1681,10 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
     CBX_CUDA(cudaMemcpyAsync(w.p, wh.data(), meig * sizeof(double), cudaMemcpyHostToDevice, s));
     k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, T.p, w.p, meig);
     h->launched("k_add_lowrank");
+    U.resize((size_t)n * meig);
+    CBX_CUDA(cudaMemcpyAsync(U.p, T.p, (size_t)n * meig * sizeof(double), cudaMemcpyDeviceToDevice, s));
   }
+  T.release();
   if (!chol_inverse_device(h, out_dev, n)) {
     invert_psd_full(h, M_dev, n, ridge, out_dev);
     return;
@@ -1706,9 +1692,9 @@ void invert_psd_device(cbx_handle* h, const double* M_dev, int64_t n, double rid
   if (meig > 0) {
     std::vector<double> wh(meig, 1.0 / eps - 1.0 / c);
     CBX_CUDA(cudaMemcpyAsync(w.p, wh.data(), meig * sizeof(double), cudaMemcpyHostToDevice, s));
-    k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, T.p, w.p, meig);
+    k_add_lowrank<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(out_dev, n, U.p, w.p, meig);
     h->launched("k_add_lowrank");
-    CBX_CUDA(cudaStreamSynchronize(s));  // wh, w and T go out of scope
+    CBX_CUDA(cudaStreamSynchronize(s));  // wh, w and U go out of scope
   }
 }
 

@@ -384,3 +384,12 @@ extern "C" int cbx_selftest_fx64_chol(cbx_handle* h, const double* A, int64_t n,
     CBX_CUDA(cudaStreamSynchronize(h->stream));
   });
 }
+
+// Largest digit buffer in bytes from now on (0: what the memory holds): work whose digits do
+// not fit goes by row groups, or without digits.
+extern "C" int cbx_selftest_digit_limit(cbx_handle* h, int64_t bytes) {
+  return cbx_guard(h, [&] {
+    CBX_REQUIRE(bytes >= 0, CBX_ERR_ARG, "bad limit");
+    h->fx_limit = (size_t)bytes;
+  });
+}
