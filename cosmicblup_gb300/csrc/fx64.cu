@@ -948,11 +948,15 @@ static void launch(cbx_handle* h, const Job& J) {
 
 }  // namespace fx
 
-void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans) {
+static size_t panel_bytes(int64_t rows, int64_t k) {
   CBX_REQUIRE(rows > 0 && k > 0 && rows < (1 << 24) && k < (1 << 24), CBX_ERR_ARG, "bad operand shape");
+  return (size_t)((rows + 127) / 128) * ((k + 31) / 32) * fx::BLK;
+}
+
+void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans) {
+  fx::at_least(P.dig, panel_bytes(rows, k));
   P.rt = (int)((rows + 127) / 128);
   P.ks = (int)((k + 31) / 32);
-  fx::at_least(P.dig, (size_t)P.rt * P.ks * fx::BLK);
   fx::at_least(P.ex, (size_t)P.rt * 128);
   cudaStream_t s = h->stream;
   if (trans) fx::k_rowexp_t<<<P.rt * 4, 256, 0, s>>>(src, ld, rows, k, P.ex.p);
@@ -965,6 +969,12 @@ void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64
                                                  P.dig.p + (size_t)y * fx::BLK);
     h->launched("k_digits");
   }
+}
+
+bool fx64_try_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k) {
+  if (!fx::try_at_least(h, P.dig, panel_bytes(rows, k))) return false;
+  fx64_digits(h, P, src, ld, rows, k, false);
+  return true;
 }
 
 void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int64_t n, double* C, int64_t ldc) {
@@ -982,6 +992,27 @@ void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int
   J.C = C;
   J.ldc = ldc;
   fx::launch(h, J);
+}
+
+bool fx64_matmul(cbx_handle* h, const double* A, FxPanel& Ad, const double* B, FxPanel& Bd, bool has_b, int64_t n,
+                 double* C) {
+  if ((has_b || fx64_try_digits(h, Bd, B, n, n, n)) && fx64_try_digits(h, Ad, A, n, n, n)) {
+    fx64_gemm(h, Ad, Bd, n, n, C, n);
+    return true;
+  }
+  Ad = FxPanel{};
+  Bd = FxPanel{};
+  const int64_t rows = 128ll * fx::group_tiles(h, (int)((n + 127) / 128), (int)((n + 31) / 32));
+  for (int64_t i = 0; i < n; i += rows) {
+    const int64_t mi = std::min(rows, n - i);
+    fx64_digits(h, Ad, A + i * n, n, mi, n, false);
+    for (int64_t j = 0; j < n; j += rows) {
+      const int64_t mj = std::min(rows, n - j);
+      fx64_digits(h, Bd, B + j * n, n, mj, n, false);
+      fx64_gemm(h, Ad, Bd, mi, mj, C + i * n + j, n);
+    }
+  }
+  return false;
 }
 
 void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,

@@ -19,8 +19,16 @@ struct FxPanel {
 // Rows of P from src: element (r, k) is src[r * ld + k], or src[k * ld + r] when
 // trans.
 void fx64_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k, bool trans);
+// the same for rows of src as they lie, or false where the digits do not fit the memory
+bool fx64_try_digits(cbx_handle* h, FxPanel& P, const double* src, int64_t ld, int64_t rows, int64_t k);
 // C[i * ldc + j] = sum_k A(i, k) B(j, k) for i < m, j < n.
 void fx64_gemm(cbx_handle* h, const FxPanel& A, const FxPanel& B, int64_t m, int64_t n, double* C, int64_t ldc);
+
+// C = A B' for n x n row-major matrices.  Ad and Bd take the digits (B's are there already when
+// has_b); where they do not fit, the product goes by groups of rows, with the same bits.
+// Returns whether Bd holds the digits of B.
+bool fx64_matmul(cbx_handle* h, const double* A, FxPanel& Ad, const double* B, FxPanel& Bd, bool has_b, int64_t n,
+                 double* C);
 
 // out[i * os + c] = sum_k Q(i, k) X[(p + gmap[k]) * xs + c] for i < ng, c < ncols <= 64, zero
 // for ncols <= c < oc.  Q holds the digits of the ng x ng block; V and part are scratch.

@@ -785,10 +785,12 @@ struct DenseExact {
   int64_t n = 0, dim = 0;
   int64_t qinv_id = -1;  // the Qinv (Mme::qinv_id) this belongs to
   DevBuf<double> ZAZt;
-  FxPanel Vdig, Pdig;
-  // kept between steps up to order kKeepDense (0.5 GB each), where allocating them costs
-  // as much as the step: LHS, its inverse, P, P V
+  // kept between steps up to order kKeepDense (0.5 GB each, digits 1 GB), where allocating them
+  // costs as much as the step: LHS, its inverse, P, P V, the digits of V = Z A Z' (valid while
+  // V_ok) and of P
   DevBuf<double> C, Ci, P, Mu;
+  FxPanel Vdig, Pdig;
+  bool V_ok = false;
   double log_det_A = 0;
   // the point whose LHS, inverse and solution C, Ci and sol hold: cbx_reml_solve's steps
   // start where the one before ended, so each factors one LHS and not two
@@ -796,9 +798,16 @@ struct DenseExact {
   double at_vu = 0, at_ve = 0, at_logL = 0;
   DevBuf<double> sol;
   static constexpr int64_t kKeepDense = 8192;
+  void drop_digits() {
+    if (n <= kKeepDense && dim <= kKeepDense) return;
+    Vdig = FxPanel{};
+    Pdig = FxPanel{};
+    V_ok = false;
+  }
   struct Trim {
     DenseExact& d;
     ~Trim() {
+      d.drop_digits();
       if (d.n <= kKeepDense && d.dim <= kKeepDense) return;
       d.at = false;
       d.C.release();
@@ -834,8 +843,7 @@ static void dense_init(cbx_handle* h, DenseExact& D) {
   D.ZAZt.resize((size_t)n * n);
   k_build_zazt<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(n, q, m.aid.p, A.p, D.ZAZt.p);
   h->launched("k_build_zazt");
-  // V = Z A Z' is the second factor of every step's product P V: its digits are kept
-  fx64_digits(h, D.Vdig, D.ZAZt.p, n, n, n, false);
+  D.V_ok = false;
   CBX_CUDA(cudaStreamSynchronize(s));
   D.n = n;
   D.dim = dim;
@@ -966,8 +974,8 @@ static bool dense_exact_step(cbx_handle* h, double& vu_io, double& ve_io, IterIn
   k_build_P_ci<<<gridn(n * n, 256, 8 * h->num_sms), 256, 0, s>>>(n, m.p, m.q, dim, m.aid.p, m.x_ptr.p, m.x_col.p,
                                                                   m.x_val.p, D.Ci.p, ve, P.p);
   h->launched("k_build_P_ci");
-  fx64_digits(h, D.Pdig, P.p, n, n, n, false);
-  fx64_gemm(h, D.Pdig, D.Vdig, n, n, Mu.p, n);
+  D.V_ok = fx64_matmul(h, P.p, D.Pdig, D.ZAZt.p, D.Vdig, D.V_ok, n, Mu.p);
+  D.drop_digits();
   const unsigned g = gridn(n * n, 256, 4 * h->num_sms);
   DevBuf<double> part;
   part.resize((size_t)g * 5);
