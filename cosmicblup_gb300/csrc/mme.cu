@@ -445,11 +445,20 @@ __global__ void k_gather_cols(const double* __restrict__ X, int xs, int ncols, i
 // The FP64 solver's block product by digits (fx64.cu) from 2 columns and ng^2 columns =
 // kFx64From on: below, the CUDA-core product's FP64 issue (1.05 TFLOP/s) takes less than the
 // digit product's four launches (about 15 us).  Its digits take 16 bytes an entry: past
-// kFx64MaxNg (17 GB) the block stays on cuBLAS DGEMM.
+// kFx64MaxNg (17 GB) the block stays on cuBLAS DGEMM, and where they do not fit the memory
+// on the CUDA-core product.
 constexpr double kFx64From = 8e6;
 constexpr int64_t kFx64MaxNg = 32768;
 static bool use_fx64(int64_t ng, int ncols) {
   return ncols >= 2 && ng <= kFx64MaxNg && (double)ng * ng * ncols > kFx64From;
+}
+// The digits of the FP64 block, made at the first product; false where they do not fit.
+static bool block_digits(cbx_handle* h, Mme& m, const sv::OpView<double>& op) {
+  if (!m.fxQ_ok && !m.fxQ_no) {
+    m.fxQ_ok = fx64_try_digits(h, m.fxQ, op.Qd, op.ld, op.ng, op.ng);
+    m.fxQ_no = !m.fxQ_ok;
+  }
+  return m.fxQ_ok;
 }
 
 // Float-float block products are FP32-issue-bound, so they run on the
@@ -569,12 +578,8 @@ static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X
     return;
   }
   cudaStream_t s = h->stream;
-  if (use_fx64(op.ng, ncols)) {
-    Mme& mm = *h->mme;
-    if (!mm.fxQ_ok) {
-      fx64_digits(h, mm.fxQ, op.Qd, op.ld, op.ng, op.ng, false);
-      mm.fxQ_ok = true;
-    }
+  Mme& mm = *h->mme;
+  if (use_fx64(op.ng, ncols) && block_digits(h, mm, op)) {
     for (int c0 = 0; c0 < ncols; c0 += 64) {
       const int nc = std::min(64, ncols - c0);
       fx64_product(h, mm.fxQ, mm.fxV, mm.fxQ_part, X + c0, S, op.p, op.gmap, op.ng, nc, Tout + c0, S,
@@ -1733,6 +1738,7 @@ extern "C" int cbx_mme_create(cbx_handle* h, int64_t n_rec, int64_t p, int64_t q
       m->fxV = std::move(o.fxV);
       m->fxQ_part = std::move(o.fxQ_part);
       m->fxQ_ok = o.fxQ_ok;
+      m->fxQ_no = o.fxQ_no;
       m->planes_src = o.planes_src;
       m->planes_gen = o.planes_gen;
       if (o.dim == m->dim)
@@ -1777,6 +1783,7 @@ static void upload_dense(cbx_handle* h, Mme& m, const double* src, int64_t ng, i
     return;
   m.planes_src = nullptr;
   m.planes_gen = -1;
+  if (m.ng != ng) m.fxQ = FxPanel{};
   m.ng = ng;
   m.ld = (ng + 3) / 4 * 4;
   m.Qd64.resize((size_t)ng * m.ld);
@@ -1803,7 +1810,7 @@ static void upload_dense(cbx_handle* h, Mme& m, const double* src, int64_t ng, i
                                                                        m.Qlo32.p);
   h->launched("k_lowp_block");
   m.fx_rows_ok = false;
-  m.fxQ_ok = false;
+  m.fxQ_ok = m.fxQ_no = false;
   if (use_bf16() && m.ld % 8 == 0) {
     m.Qbf.resize((size_t)ng * m.ld);
     dense_bf_block(h, m.Qd64.p, ng, m.ld, m.qshift, m.Qbf.p);

@@ -70,9 +70,10 @@ struct Mme {
   // refinement product (valid while fx_rows_ok), and its scratch
   DevBuf<int32_t> fx_rowexp;
   bool fx_rows_ok = false;
-  // digits of Qd64 for the FP64 solver's block product (valid while fxQ_ok), and its scratch
+  // digits of Qd64 for the FP64 solver's block product (valid while fxQ_ok; fxQ_no: they do not
+  // fit the memory), and its scratch
   FxPanel fxQ, fxV;
-  bool fxQ_ok = false;
+  bool fxQ_ok = false, fxQ_no = false;
   DevBuf<double> fxQ_part;
   DevBuf<uint16_t> fx_bdig;
   DevBuf<int32_t> fx_cexp;
