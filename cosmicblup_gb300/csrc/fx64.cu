@@ -119,12 +119,13 @@ __device__ __noinline__ double from_totals_any(long long hi, long long lo, int n
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// digit planes of eight consecutive K elements of one row
-__device__ __forceinline__ void put_digits(const double (&v)[8], int ex, uint8_t* blk, int row, int kg) {
+// digit planes of N = 8 or 4 consecutive K elements of one row, from element N kg on
+template <int N>
+__device__ __forceinline__ void put_digits(const double (&v)[N], int ex, uint8_t* blk, int row, int kg) {
   const double sc = pow2d(61 - (ex == EX_BAD ? 0 : ex));
-  uint32_t lo[8], hi[8];
+  uint32_t lo[N], hi[N];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
+  for (int e = 0; e < N; ++e) {
     const unsigned long long G =
         BIAS + (ex == EX_BAD ? 0ull : (unsigned long long)__double2ll_rn(v[e] * sc));
     lo[e] = (uint32_t)G;
@@ -133,11 +134,13 @@ __device__ __forceinline__ void put_digits(const double (&v)[8], int ex, uint8_t
 #pragma unroll
   for (int pl = 0; pl < NPL; ++pl) {
     const int j = 7 - pl;
-    uint32_t w[4];
+    uint32_t w[N / 2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+    for (int e = 0; e < N / 2; ++e)
       w[e] = j < 4 ? digit_pair(lo[2 * e], lo[2 * e + 1], j) : digit_pair(hi[2 * e], hi[2 * e + 1], j - 4);
-    *reinterpret_cast<uint4*>(blk + pl * PLANE_A + cm_off(row, kg * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+    uint8_t* const dst = blk + pl * PLANE_A + cm_off(row, kg * N);
+    if constexpr (N == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
   }
 }
 
@@ -624,10 +627,11 @@ __device__ __forceinline__ double reciprocal(double d) {
 // first, and the condition of the pair enters twice.  The groups' rows are forward
 // substitutions by the same pairs and not products with X, which lose the root of L_kk's
 // condition where two adjacent rows are near-duplicates.  Measured with the pair's inverse
-// and X before, both this way now: factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81, now 2.84;
-// at 8,000 18.3, now 18.2, and 34.4, now 35.0 (a substitution issues 92 FP64 instructions a
-// warp and group, the product 80).  L L' - A at n = 96 with adjacent rows 1e-3 apart: 0.01 of
-// 4 n u sqrt(A_ii A_jj), 1e5 times it before, when rows 1e-4 apart were found not positive definite.
+// and X before, both this way now: factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81 both; at
+// 8,000 18.3, now 18.1, and 34.4, now 34.8 (a substitution issues 92 FP64 instructions a warp and group,
+// the product 80; the digits took 16 on half of the lanes, now 8).  L L' - A at n = 96 with adjacent
+// rows 1e-3 apart: 0.01 of 4 n u sqrt(A_ii A_jj), 1e5 times it before, when rows 1e-4 apart were
+// found not positive definite.
 __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) {
   __shared__ double X[32][33], V[4][32][5], pa[16][32], pb[16][32], ra[16][32], rw[16][32];
   __shared__ double pv[32], lp[16], i1[16], l2[16], i2[16];
@@ -788,12 +792,10 @@ __global__ void __launch_bounds__(128) k_panel(const __grid_constant__ Panel a) 
       if (a.inverse && !below) a.exm[r] = left ? max(e, a.exm[r]) : e;
     }
     __syncwarp();
-    if (c < 4) {  // K group c of the row
-      double v8[8];
+    double v4[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v8[i] = V[w][c * 8 + i][lane >> 3];
-      put_digits(v8, e, a.dig + (size_t)(r / 128) * BLK, r & 127, c);
-    }
+    for (int i = 0; i < 4; ++i) v4[i] = V[w][c * 4 + i][lane >> 3];
+    put_digits(v4, e, a.dig + (size_t)(r / 128) * BLK, r & 127, c);
     if (!below && !left) {
       for (int i = 0; i < 4; ++i) {
         const int l = g * 16 + 4 * w + i - a.k0, j = lane >> 1;
