@@ -157,7 +157,9 @@ static void ml_ordered(const std::vector<int64_t>& dam, const std::vector<int64_
   f.assign(n, 0.0);
   dii.assign(n, 1.0);
   const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-  const int nt = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(16, hw), n / 256));
+  // 16 bytes an animal and thread: at most 1 GB of them
+  const int64_t fit = std::max<int64_t>(1, (int64_t(1) << 26) / n);
+  const int nt = (int)std::max<int64_t>(1, std::min<int64_t>({16, hw, n / 256, fit}));
   Rendezvous meet;
   std::vector<std::atomic<int64_t>> next(nlev);
   for (int64_t l = 0; l < nlev; ++l) next[l].store(start[l]);
