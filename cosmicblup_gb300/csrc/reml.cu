@@ -866,9 +866,9 @@ static void build_lhs(cbx_handle* h, double lam, DevBuf<double>& C) {
 }
 // y = A x (+ y0 when given, minus A x when neg) for a symmetric n x n matrix: one warp
 // per row, 32 partial sums in a fixed order.  Bound by the read of A (HBM, or L2 below
-// n = 4,000).
+// n = 4,000).  y may be y0, whose elements the same threads read.
 __global__ void __launch_bounds__(256) k_symv(int64_t n, const double* __restrict__ A, const double* __restrict__ x,
-                                              const double* __restrict__ y0, int neg, double* __restrict__ y) {
+                                              const double* y0, int neg, double* y) {
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= n) return;
   const double* a = A + r * n;
