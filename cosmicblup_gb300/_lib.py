@@ -116,6 +116,8 @@ SIGNATURES = [
                                          C.c_int32, C.c_int32, C.c_void_p, C.POINTER(C.c_double)]),
     ("cbx_selftest_fx64_chol", C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p,
                                          C.POINTER(C.c_double), C.POINTER(C.c_int32), C.POINTER(C.c_double)]),
+    ("cbx_selftest_reciprocal", C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
+    ("cbx_selftest_from_totals", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     ("cbx_selftest_digit_limit", C.c_int, [C.c_void_p, C.c_int64]),
     ("cbx_selftest_wait_timeout", C.c_int, [C.c_void_p, C.c_int64, C.POINTER(C.c_double)]),
 ]

@@ -75,19 +75,17 @@ __device__ __forceinline__ int expo(double v) {
   const int e = (int)((__double_as_longlong(v) >> 52) & 0x7FF);
   return e == 0x7FF ? EX_BAD : max(EX_MIN, e - 1022);
 }
-// (hi 2^32 + lo) 2^n, rounded to nearest, for -900 < n < 900, in about 30 integer
+// (hi 2^32 + lo) 2^n, rounded to nearest (ties away from zero), for -900 < n < 900, in about 30 integer
 // instructions without a branch: on GB300 each FP64 instruction or int64 conversion of a
 // warp holds its quarter of the SM's FP64 pipe for 64 clocks.
-__host__ __device__ __forceinline__ unsigned long long from_totals(long long hi, long long lo, int n) {
+__device__ __forceinline__ unsigned long long from_totals(long long hi, long long lo, int n) {
   const long long h = hi + (lo >> 32);
   const uint32_t m = (uint32_t)(h >> 63);
   const unsigned long long l = (unsigned long long)((uint32_t)lo ^ m) + (m & 1u);
   const unsigned long long t = ((unsigned long long)h ^ ((unsigned long long)m << 32 | m)) + (l >> 32);
   uint32_t w2 = (uint32_t)(t >> 32), w1 = (uint32_t)t, w0 = (uint32_t)l;  // |x| in 96 bits
   int e = 1023 + 32 + 62 + n;  // biased exponent, less the leading bit the mantissa adds
-#ifdef __CUDA_ARCH__
 #pragma unroll
-#endif
   for (int i = 0; i < 2; ++i) {
     const bool z = w2 == 0;
     w2 = z ? w1 : w2;
@@ -95,14 +93,8 @@ __host__ __device__ __forceinline__ unsigned long long from_totals(long long hi,
     w0 = z ? 0u : w0;
     e -= z ? 32 : 0;
   }
-#ifdef __CUDA_ARCH__
   const int c = __clz((int)w2);
   const uint32_t b1 = __funnelshift_l(w1, w2, c), b0 = __funnelshift_l(w0, w1, c);
-#else
-  const int c = w2 ? __builtin_clz(w2) : 32;
-  const uint32_t b1 = c ? (c < 32 ? (w2 << c) | (w1 >> (32 - c)) : 0u) : w2;
-  const uint32_t b0 = c ? (c < 32 ? (w1 << c) | (w0 >> (32 - c)) : 0u) : w1;
-#endif
   const unsigned long long b = ((unsigned long long)b1 << 32) | b0;
   const unsigned long long v = ((unsigned long long)(uint32_t)(e - c) << 52) + (b >> 11) + ((b >> 10) & 1);
   return w2 ? v | ((unsigned long long)(m & 1u) << 63) : 0ull;
@@ -339,9 +331,10 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
       const int rb = rt * 128 + q * 32, row = rb + lane, col0 = ct * NT + j0;
       const int ea = J.ea[row] - 66;  // 56 - 2 * 61
       const int el = J.eb[col0 + (lane & 15)];
-      long long hi[16], lo[16];
+      // modulo 2^64: the offsets' sum leaves the range of an int64 from 432 chunks on
+      unsigned long long hi[16], lo[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) hi[j] = lo[j] = -(long long)MAGIC * 0x01010101ll * nch;
+      for (int j = 0; j < 16; ++j) hi[j] = lo[j] = 0ull - (unsigned long long)MAGIC * 0x01010101ull * (unsigned)nch;
       for (int ch = 0; ch < nch; ++ch, ++c) {
         if (!mbar_wait_idle(&bars->acc_full, c & 1, abort_flag, 20)) { ok = false; break; }
         tc_fence_after();
@@ -358,8 +351,8 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
             const float f = __uint_as_float(r[j]);
             big = fmaxf(big, fabsf(f));
             const long long v = (long long)__float_as_int(__fadd_rn(f, 12582912.0f)) * mul;
-            if (u < 4) hi[j] += v;
-            else lo[j] += v;
+            if (u < 4) hi[j] += (unsigned long long)v;
+            else lo[j] += (unsigned long long)v;
           }
         }
         // sums past 2^22 (possible over more than 32 K elements, and rare) do not fit the bits
@@ -376,8 +369,8 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
               const float f = __uint_as_float(r[j]);
               const long long v =
                   (long long)(__float2int_rn(f) + MAGIC - __float_as_int(__fadd_rn(f, 12582912.0f))) * mul;
-              if (u < 4) hi[j] += v;
-              else lo[j] += v;
+              if (u < 4) hi[j] += (unsigned long long)v;
+              else lo[j] += (unsigned long long)v;
             }
           }
         }
@@ -398,11 +391,11 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
           double2 x;
           const int e0 = ea + __shfl_sync(~0u, el, h + j), e1 = ea + __shfl_sync(~0u, el, h + j + 1);
           if (usual) {
-            x.x = __longlong_as_double((long long)from_totals(hi[h + j], lo[h + j], e0));
-            x.y = __longlong_as_double((long long)from_totals(hi[h + j + 1], lo[h + j + 1], e1));
+            x.x = __longlong_as_double((long long)from_totals((long long)hi[h + j], (long long)lo[h + j], e0));
+            x.y = __longlong_as_double((long long)from_totals((long long)hi[h + j + 1], (long long)lo[h + j + 1], e1));
           } else {
-            x.x = from_totals_any(hi[h + j], lo[h + j], e0);
-            x.y = from_totals_any(hi[h + j + 1], lo[h + j + 1], e1);
+            x.x = from_totals_any((long long)hi[h + j], (long long)lo[h + j], e0);
+            x.y = from_totals_any((long long)hi[h + j + 1], (long long)lo[h + j + 1], e1);
           }
           *reinterpret_cast<double2*>(out + lane * 64 + (((j >> 1) ^ ((lane >> 1) & 3)) << 4)) = x;
           if (J.mode == 2 && row < J.m) {
@@ -598,15 +591,6 @@ struct Panel {
   double* piv;
   int* bad;
 };
-
-// 1 / d from the hardware's 20-bit approximation by one third-order (Householder) step:
-// with e = 1 - d r, 1 / d = r (1 + e + e^2 + ...)
-__device__ __forceinline__ double reciprocal(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
 
 // One 32-wide step.  Every CTA factors the pivot block (it is small, and a separate
 // launch would cost more than the repeat), then takes 16-row groups: x L_kk' = v with v
@@ -948,7 +932,17 @@ static void launch(cbx_handle* h, const Job& J) {
   else launch_tiles<64>(h, J);
 }
 
+__global__ void k_selftest_totals(const int64_t* __restrict__ hi, const int64_t* __restrict__ lo,
+                                  const int32_t* __restrict__ e, int64_t n, double* __restrict__ y) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    y[i] = __longlong_as_double((long long)from_totals(hi[i], lo[i], e[i]));
+}
+
 }  // namespace fx
+
+void fx64_selftest_totals(cbx_handle* h, const int64_t* hi, const int64_t* lo, const int32_t* e, int64_t n, double* y) {
+  fx::k_selftest_totals<<<128, 256, 0, h->stream>>>(hi, lo, e, n, y);
+}
 
 static size_t panel_bytes(int64_t rows, int64_t k) {
   CBX_REQUIRE(rows > 0 && k > 0 && rows < (1 << 24) && k < (1 << 24), CBX_ERR_ARG, "bad operand shape");

@@ -50,4 +50,7 @@ struct FxAdd {
 bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, double* out, double* logdet,
                    FxAdd add = {});
 
+// y[i] = (hi[i] 2^32 + lo[i]) 2^e[i], |e[i]| < 900 (self-test of the products' conversion)
+void fx64_selftest_totals(cbx_handle* h, const int64_t* hi, const int64_t* lo, const int32_t* e, int64_t n, double* y);
+
 }  // namespace cbx

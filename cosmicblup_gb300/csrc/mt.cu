@@ -74,14 +74,6 @@ __global__ void k_half_cov(const double* __restrict__ Y, int64_t n, int t, doubl
     }
 }
 
-// 1 / d from the hardware's 20-bit approximation by one third-order (Householder) step
-__device__ __forceinline__ double reciprocal(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // In-register inverse of an SPD T x T matrix V = L D L' (unit lower L); false if not PD.
 // No square root and T reciprocals: FP64 issue bounds the EM loop.
 template <int T>

@@ -393,3 +393,43 @@ extern "C" int cbx_selftest_digit_limit(cbx_handle* h, int64_t bytes) {
     h->fx_limit = (size_t)bytes;
   });
 }
+
+__global__ void k_selftest_reciprocal(const double* __restrict__ x, int64_t n, double* __restrict__ y) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    y[i] = cbx::reciprocal(x[i]);
+}
+
+// y = 1 / x by the kernels' reciprocal
+extern "C" int cbx_selftest_reciprocal(cbx_handle* h, const double* x, int64_t n, double* y) {
+  return cbx_guard(h, [&] {
+    CBX_REQUIRE(n > 0 && x && y, CBX_ERR_ARG, "bad arguments");
+    CBX_CUDA(cudaSetDevice(h->device));
+    cbx::DevBuf<double> d;
+    d.resize(2 * n);
+    CBX_CUDA(cudaMemcpyAsync(d.p, x, n * 8, cudaMemcpyHostToDevice, h->stream));
+    k_selftest_reciprocal<<<128, 256, 0, h->stream>>>(d.p, n, d.p + n);
+    CBX_CUDA(cudaMemcpyAsync(y, d.p + n, n * 8, cudaMemcpyDeviceToHost, h->stream));
+    CBX_CUDA(cudaStreamSynchronize(h->stream));
+  });
+}
+
+// y[i] = (hi[i] 2^32 + lo[i]) 2^e[i] by the digit products' conversion
+extern "C" int cbx_selftest_from_totals(cbx_handle* h, const int64_t* hi, const int64_t* lo, const int32_t* e, int64_t n,
+                                        double* y) {
+  return cbx_guard(h, [&] {
+    CBX_REQUIRE(n > 0 && hi && lo && e && y, CBX_ERR_ARG, "bad arguments");
+    CBX_CUDA(cudaSetDevice(h->device));
+    cbx::DevBuf<int64_t> t;
+    cbx::DevBuf<int32_t> x;
+    cbx::DevBuf<double> d;
+    t.resize(2 * n);
+    x.resize(n);
+    d.resize(n);
+    CBX_CUDA(cudaMemcpyAsync(t.p, hi, n * 8, cudaMemcpyHostToDevice, h->stream));
+    CBX_CUDA(cudaMemcpyAsync(t.p + n, lo, n * 8, cudaMemcpyHostToDevice, h->stream));
+    CBX_CUDA(cudaMemcpyAsync(x.p, e, n * 4, cudaMemcpyHostToDevice, h->stream));
+    cbx::fx64_selftest_totals(h, t.p, t.p + n, x.p, n, d.p);
+    CBX_CUDA(cudaMemcpyAsync(y, d.p, n * 8, cudaMemcpyDeviceToHost, h->stream));
+    CBX_CUDA(cudaStreamSynchronize(h->stream));
+  });
+}
