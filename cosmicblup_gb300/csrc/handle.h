@@ -18,12 +18,13 @@ struct cbx_handle {
   int num_sms = 0;
   cudaStream_t stream = nullptr;
   // second stream of the PCG operator: the sparse part runs on it beside the
-  // dense block product on `stream` (fork / join events, captured into graphs)
+  // dense block product on `stream` (between fork / join events, not inside a capture)
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // third stream: the sums of the gathered vectors, beside the same product
   cudaStream_t stream3 = nullptr;
   cudaEvent_t ev_join3 = nullptr;
+  bool capturing = false;  // `stream` is being captured
   std::string last_error;
   int64_t launches = 0;
   cbx::DevBuf<int> status;  // device-side error word(s)

@@ -676,6 +676,36 @@ int product_from_vt(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, 
   return tsplit;
 }
 
+// Work beside the handle's stream, on a side stream between two events.  Inside a capture, and
+// with side == the handle's stream, it stays on that stream: with graphs that had branches,
+// batches of 32 and more problems on 16 host threads crashed in the driver, in an event's
+// record or in a context's synchronization; with unbranched graphs they do not.
+class Branch {
+ public:
+  Branch(cbx_handle* h, cudaStream_t side, cudaEvent_t done)
+      : h_(h), side_(h->capturing ? h->stream : side), done_(done) {}
+  // the stream that takes the branch's launches, up to end()
+  cudaStream_t begin() {
+    if (side_ != h_->stream) {
+      CBX_CUDA(cudaEventRecord(h_->ev_fork, h_->stream));
+      CBX_CUDA(cudaStreamWaitEvent(side_, h_->ev_fork, 0));
+    }
+    return side_;
+  }
+  void end() {
+    if (side_ != h_->stream) CBX_CUDA(cudaEventRecord(done_, side_));
+  }
+  // later launches of the handle's stream follow the branch too
+  void join() {
+    if (side_ != h_->stream) CBX_CUDA(cudaStreamWaitEvent(h_->stream, done_, 0));
+  }
+
+ private:
+  cbx_handle* h_;
+  cudaStream_t side_;
+  cudaEvent_t done_;
+};
+
 // Y = use_D * W'W X + lam [0; Qinv X_u] for an S-wide interleaved block whose
 // first ncols columns are populated (the rest are zero or ignored); optional
 // pq partials sum_i P[i] Y[i] for the PCG step.
@@ -696,21 +726,18 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   // stream under a launch trace, whose attribution assumes one)
   const Mme& mm = *h->mme;
   const bool segs = use_D && mm.nseg > 0;
-  cudaStream_t s2 = h->trace_on || !op.Qd ? s : h->stream2;
+  Branch side(h, h->trace_on || !op.Qd ? s : h->stream2, h->ev_join);
+  const cudaStream_t s2 = side.begin();
   auto segments = [&]() {
     if (!segs) return;
     sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s2>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p,
                                                     active, ncp);
     h->launched(sizeof(T) == 4 ? "k_fix_seg<f32>" : "k_fix_seg<f64>");
   };
-  if (op.Qd) {
-    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
-    CBX_CUDA(cudaStreamWaitEvent(s2, h->ev_fork, 0));
-  }
   segments();
   if (!op.Qd) {
   } else if constexpr (sizeof(T) == 8) {
-    CBX_CUDA(cudaEventRecord(h->ev_join, s2));
+    side.end();
     ff = ff && h->mme->Qlo32.p && h->mme->Qd32.p;
     if (!ff) colsum = nullptr;
     cbx_handle::ProfRec pr{};
@@ -730,12 +757,11 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       pr.bytes = 8.0 * (double)op.ng * op.ld + 8.0 * ncols * ((double)op.ld + (double)op.ng);
       h->prof.push_back(pr);
     }
-    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
+    side.join();
   } else {
     // FP32: gather the dense-block rows, their FP64 column sums, the product
     // (the populated 32-column groups only)
     const bool split = matvec_split(h, op);
-    cudaStream_t s3 = h->trace_on ? s : h->stream3;
     if (split) {
       // the rest of the sparse part beside the product too: k_spmv without the block
       // term writes every row and its pq partials
@@ -745,7 +771,7 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
                                                         w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
       h->launched("k_spmv<f32>");
     }
-    CBX_CUDA(cudaEventRecord(h->ev_join, s2));
+    side.end();
     if constexpr (S >= 32)
       sv::k_gather_tile<T, S><<<(unsigned)((op.ld + 31) / 32), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld, op.gmap,
                                                                             active, ncp);
@@ -754,14 +780,14 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
                                                                                    op.gmap, active, S, ncp);
     h->launched("k_gather_t<f32>");
     // the gathered vectors' sums, which only the last kernel reads, on the third
-    CBX_CUDA(cudaEventRecord(h->ev_fork, s));
-    CBX_CUDA(cudaStreamWaitEvent(s3, h->ev_fork, 0));
+    Branch sums(h, h->trace_on ? s : h->stream3, h->ev_join3);
+    const cudaStream_t s3 = sums.begin();
     sv::k_colsum_vt<T><<<ncp, 1024, 0, s3>>>(w.Vt.p, op.ld, op.ng, w.colsum.p);
     h->launched("k_colsum_vt<f32>");
-    CBX_CUDA(cudaEventRecord(h->ev_join3, s3));
+    sums.end();
     tsplit = product_from_vt<T, S>(h, op, w, active, ncols);
-    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join3, 0));
-    CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
+    sums.join();
+    side.join();
     if (split) {
       // the block term of the genotyped rows, once both are done
       sv::k_dense_add<T, S><<<w.nblk_dadd, sv::NT, 0, s>>>(op, w.Tout.p, tsplit, colsum, tshift, (T)lam, Y, P,
@@ -927,11 +953,13 @@ void run_pcg(cbx_handle* h, Mme& m, const sv::OpView<T>& op, Workspace<T, S>& w,
         const int64_t l0 = h->launches;
         bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
+          h->capturing = true;
           try {
             iterations(false);
           } catch (...) {
             ok = false;
           }
+          h->capturing = false;
           ok = (cudaStreamEndCapture(s, &g) == cudaSuccess) && ok && g;
         }
         if (ok) ok = cudaGraphInstantiate(&gexec, g, 0) == cudaSuccess;
