@@ -48,8 +48,6 @@ int cbx_create(int device, cbx_handle** out) {
     CBX_CUDA(cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking));
     CBX_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
     CBX_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
-    CBX_CUDA(cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking));
-    CBX_CUDA(cudaEventCreateWithFlags(&h->ev_join3, cudaEventDisableTiming));
     h->status.resize(4);
     h->status.zero(h->stream);
     CBX_CUDA(cudaStreamSynchronize(h->stream));
@@ -88,8 +86,6 @@ int cbx_destroy(cbx_handle* h) {
     if (tmp->ev_fork) cudaEventDestroy(tmp->ev_fork);
     if (tmp->ev_join) cudaEventDestroy(tmp->ev_join);
     if (tmp->stream2) cudaStreamDestroy(tmp->stream2);
-    if (tmp->ev_join3) cudaEventDestroy(tmp->ev_join3);
-    if (tmp->stream3) cudaStreamDestroy(tmp->stream3);
     if (tmp->stream) cudaStreamDestroy(tmp->stream);
   }
   delete h;

@@ -127,7 +127,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     k_dense_tf32(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int ng,
                  int ksteps, int total, int per, int nslot, float* __restrict__ Tpart, const int* active,
                  int* status, int nc) {
-  if (active && *active == 0) return;
+  if (active && *active == 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   using LY = Layout<S, NCM>;
   constexpr int NSTAGE = LY::NSTAGE;
   extern __shared__ uint8_t dsm_raw[];
@@ -316,6 +319,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem, TMEM_ALLOC);
+  // the sums that a block product may have started beside (release_successor in solver.cuh)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace dtc
@@ -350,8 +355,24 @@ int dense_tc_stream_k(int64_t ng, int64_t ld, int num_sms, int* grid, int* per) 
   return stream_k(ng, ld, num_sms, grid, per);
 }
 
+template <typename K, typename... A>
+static void launch_product(cbx_handle* h, K kern, int grid, int smem, bool beside, A... args) {
+  ensure_smem((const void*)kern, smem, h->device);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(dtc::THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = beside ? 1 : 0;
+  CBX_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+
 void dense_tc(cbx_handle* h, const float* Qd, int64_t ng, int64_t ld, const float* Vt, int S, int ksplit, float* Tpart,
-              const int* active, int ncols) {
+              const int* active, int ncols, bool beside) {
   CBX_REQUIRE(S == 16 || S == 32 || S == 64 || S == 128, CBX_ERR_ARG, "dense_tc supports 16, 32, 64 or 128 columns");
   // the MMAs and the lo conversion run on the populated columns, rounded up
   // to the MMA granularity of 16; the output's other columns are written as 0
@@ -366,27 +387,13 @@ void dense_tc(cbx_handle* h, const float* Qd, int64_t ng, int64_t ld, const floa
   int grid = 0, per = 0;
   const int nslot = stream_k(ng, ld, h->num_sms, &grid, &per);
   CBX_REQUIRE(nslot == ksplit, CBX_ERR_ARG, "partial slot count does not match dense_tc_ksplit");
-  if (S == 128) {
-    constexpr int SM = dtc::Layout<128, 80>::SMEM;
-    ensure_smem((const void*)dtc::k_dense_tf32<128, 80>, SM, h->device);
-    dtc::k_dense_tf32<128, 80><<<grid, dtc::THREADS, SM, h->stream>>>(ma, mb, (int)ng, ksteps, total, per, nslot,
-                                                                      Tpart, active, h->status.p, nc);
-  } else if (S == 64) {
-    constexpr int SM = dtc::Layout<64>::SMEM;
-    ensure_smem((const void*)dtc::k_dense_tf32<64>, SM, h->device);
-    dtc::k_dense_tf32<64><<<grid, dtc::THREADS, SM, h->stream>>>(ma, mb, (int)ng, ksteps, total, per, nslot, Tpart,
-                                                                 active, h->status.p, nc);
-  } else if (S == 32) {
-    constexpr int SM = dtc::Layout<32>::SMEM;
-    ensure_smem((const void*)dtc::k_dense_tf32<32>, SM, h->device);
-    dtc::k_dense_tf32<32><<<grid, dtc::THREADS, SM, h->stream>>>(ma, mb, (int)ng, ksteps, total, per, nslot, Tpart,
-                                                                 active, h->status.p, nc);
-  } else {
-    constexpr int SM = dtc::Layout<16>::SMEM;
-    ensure_smem((const void*)dtc::k_dense_tf32<16>, SM, h->device);
-    dtc::k_dense_tf32<16><<<grid, dtc::THREADS, SM, h->stream>>>(ma, mb, (int)ng, ksteps, total, per, nslot, Tpart,
-                                                                 active, h->status.p, nc);
-  }
+  auto run = [&](auto kern, int smem) {
+    launch_product(h, kern, grid, smem, beside, ma, mb, (int)ng, ksteps, total, per, nslot, Tpart, active, h->status.p, nc);
+  };
+  if (S == 128) run(dtc::k_dense_tf32<128, 80>, dtc::Layout<128, 80>::SMEM);
+  else if (S == 64) run(dtc::k_dense_tf32<64>, dtc::Layout<64>::SMEM);
+  else if (S == 32) run(dtc::k_dense_tf32<32>, dtc::Layout<32>::SMEM);
+  else run(dtc::k_dense_tf32<16>, dtc::Layout<16>::SMEM);
   h->launched("k_dense_tf32");
 }
 

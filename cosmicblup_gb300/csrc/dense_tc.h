@@ -7,9 +7,11 @@ namespace cbx {
 int dense_tc_ksplit(int64_t ng, int64_t ld, int num_sms);
 // The same split with its grid and the 32-element K steps per CTA.
 int dense_tc_stream_k(int64_t ng, int64_t ld, int num_sms, int* grid, int* per);
-// Tpart[ks][i][c] = sum over split ks of Qd[i][k] Vt[c][k]; S = 16 or 32.
+// Tpart[ks][i][c] = sum over split ks of Qd[i][k] Vt[c][k]; S = 16, 32, 64 or 128.  beside:
+// starts with the kernel before it on the stream, which lets it (release_successor) and
+// writes nothing that it reads; whatever follows the product normally finds both done.
 void dense_tc(cbx_handle* h, const float* Qd, int64_t ng, int64_t ld, const float* Vt, int S, int ksplit,
-              float* Tpart, const int* active, int ncols);
+              float* Tpart, const int* active, int ncols, bool beside = false);
 // The bf16 block product (dense_bf.cu): the same split over 64-element K steps,
 // the bf16 copy of Qd - shift, and Tpart as dense_tc for the first ncols of the
 // S gathered FP32 rows Vt (Vhl: 2 S ld bf16 scratch); returns the partial count.

@@ -163,6 +163,7 @@ struct Job {
   int nz, kper;
   int64_t cz;
   const int* active;  // nothing to do when it points to 0
+  int late;           // the kernel before writes nothing read here: wait for it at the end
 };
 struct Bars {
   uint64_t full[NSTAGE], empty[NSTAGE], acc_full, acc_empty, drain;
@@ -219,7 +220,10 @@ __device__ __forceinline__ size_t blk_of(int rt, int ks, int stride, int tri) {
 template <int NT>
 __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_constant__ Job J, int* status) {
   using T = Tile<NT>;
-  if (J.active && *J.active == 0) return;
+  if (J.active && *J.active == 0) {
+    pdl_wait();
+    return;
+  }
   extern __shared__ uint8_t dsm_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
   Bars* bars = reinterpret_cast<Bars*>(smem + T::OFF_BAR);
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
     bars->abort = 1;
     atomicExch(status, DEV_TIMEOUT);
   };
-  pdl_wait();
+  if (!J.late) pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -440,6 +444,7 @@ __global__ void __launch_bounds__(Tile<NT>::THREADS, 1) k_fx64(const __grid_cons
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem, 8 * NT);
+  if (J.late) pdl_wait();
 }
 
 // ---- digits of a matrix ------------------------------------------------------
@@ -1012,7 +1017,8 @@ bool fx64_matmul(cbx_handle* h, const double* A, FxPanel& Ad, const double* B, F
 }
 
 void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,
-                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active) {
+                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active,
+                  const std::function<bool()>& before) {
   CBX_REQUIRE(ncols >= 1 && ncols <= 64 && ng <= (int64_t)Q.rt * 128, CBX_ERR_ARG, "bad block product");
   cudaStream_t s = h->stream;
   const int nt = ncols <= 32 ? 32 : 64;
@@ -1057,6 +1063,7 @@ void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& p
   J.C = part.p;
   J.ldc = nt;
   J.active = active;
+  if (before) J.late = before() ? 1 : 0;
   if (nt == 32) fx::launch_tiles<32>(h, J);
   else fx::launch_tiles<64>(h, J);
   fx::k_slices<<<(unsigned)std::min<int64_t>((ng * oc + 255) / 256, 8 * h->num_sms), 256, 0, s>>>(

@@ -3,6 +3,7 @@
 // dense-AI paths.
 #pragma once
 #include <cstdint>
+#include <functional>
 #include "devbuf.h"
 
 struct cbx_handle;
@@ -32,9 +33,11 @@ bool fx64_matmul(cbx_handle* h, const double* A, FxPanel& Ad, const double* B, F
 
 // out[i * os + c] = sum_k Q(i, k) X[(p + gmap[k]) * xs + c] for i < ng, c < ncols <= 64, zero
 // for ncols <= c < oc.  Q holds the digits of the ng x ng block; V and part are scratch.
-// Does nothing while active (may be null) points to 0.
+// Does nothing while active (may be null) points to 0.  before (may be empty) is called ahead
+// of the MMAs: true if its last launch lets them start with it (release_successor).
 void fx64_product(cbx_handle* h, const FxPanel& Q, FxPanel& V, DevBuf<double>& part, const double* X, int xs, int64_t p,
-                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active);
+                  const int32_t* gmap, int64_t ng, int ncols, double* out, int os, int oc, const int* active,
+                  const std::function<bool()>& before = {});
 
 // diag I + all 11' is added to a matrix on reading it
 struct FxAdd {

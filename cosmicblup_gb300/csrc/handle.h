@@ -17,13 +17,10 @@ struct cbx_handle {
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
-  // second stream of the PCG operator: the sparse part runs on it beside the
-  // dense block product on `stream` (between fork / join events, not inside a capture)
+  // second stream: copies of G behind its tiles, and the opt-in overlap of the PCG operator's
+  // sparse part (fork / join events; never inside a capture)
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // third stream: the sums of the gathered vectors, beside the same product
-  cudaStream_t stream3 = nullptr;
-  cudaEvent_t ev_join3 = nullptr;
   bool capturing = false;  // `stream` is being captured
   std::string last_error;
   int64_t launches = 0;

@@ -11,6 +11,7 @@
 //    (src/core/pcg_solver.h:60-128, 436-536) and MatrixFreePCG's absolute stop
 //    (src/core/matrix_free_pcg.h:20-66).
 #include <algorithm>
+#include <functional>
 #include <cstdio>
 #include <cmath>
 #include <exception>
@@ -535,14 +536,37 @@ static void ff_plan(cbx_handle* h, const sv::OpView<double>& op, const double* X
   }
 }
 
+// A launch that, when dependent, may be set up while its predecessor on the stream still runs
+// (the kernel waits for its end with wait_predecessor).
+template <typename... KArgs, typename... Args>
+void launch_on(void (*kern)(KArgs...), int grid, int block, int smem, cudaStream_t s, bool dependent, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  CBX_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+}
+template <typename... KArgs, typename... Args>
+void launch_next(void (*kern)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
+  launch_on(kern, grid, block, 0, s, true, args...);
+}
+
 // Tout[:, 0:ncols] (rows S apart) of the dense block product in FP64
-// accuracy: float-float on the CUDA cores (ff), or cuBLAS DGEMM / DGEMV on the
-// gathered columns (the block is an ng x ng column-major matrix with leading
-// dimension ld; it is symmetric, so either orientation gives Qinv X).
+// accuracy: float-float on the CUDA cores (ff), or on the gathered columns by digits, the
+// CUDA cores or cuBLAS DGEMM (the block is an ng x ng column-major matrix with leading
+// dimension ld; it is symmetric, so either orientation gives Qinv X).  before is called once,
+// ahead of the product itself: true if its launch lets the product start with it.
 template <int S>
 static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X, int ncols, double* Vt, double* Tout,
-                    const int* active, bool ff, double* colsum) {
+                    const int* active, bool ff, double* colsum, const std::function<bool()>& before) {
   if (ff) {
+    before();
     // the compensated FP64 column sums that restore the block's shift
     sv::k_colsum_x<<<ncols, 256, 0, h->stream>>>(X, S, op.p, op.ng, op.gmap, colsum);
     h->launched("k_colsum_x<f64>");
@@ -583,15 +607,17 @@ static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X
     for (int c0 = 0; c0 < ncols; c0 += 64) {
       const int nc = std::min(64, ncols - c0);
       fx64_product(h, mm.fxQ, mm.fxV, mm.fxQ_part, X + c0, S, op.p, op.gmap, op.ng, nc, Tout + c0, S,
-                   c0 + nc < ncols ? nc : S - c0, active);
+                   c0 + nc < ncols ? nc : S - c0, active, c0 == 0 ? before : std::function<bool()>{});
     }
     return;
   }
   k_gather_cols<<<grid_for((int64_t)S * op.ld, 256, 4 * h->num_sms), 256, 0, s>>>(X, S, ncols, S, Vt, op.p, op.ng,
                                                                                  op.ld, op.gmap);
   h->launched("k_gather_cols<f64>");
+  const bool beside = before();
   if (ncols == 1 && S == 1) {
-    sv::k_gemv<double, 2, 4><<<(unsigned)((op.ng + 15) / 16), 256, 0, s>>>(op.Qd, op.ng, op.ld, Vt, Tout, active);
+    launch_on(sv::k_gemv<double, 2, 4>, (int)((op.ng + 15) / 16), 256, 0, s, beside, op.Qd, op.ng, op.ld, Vt, Tout, active,
+              1);
     h->launched("k_gemv<f64>");
     return;
   }
@@ -600,8 +626,8 @@ static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X
       constexpr int R = rpw<double, S>();
       constexpr int smem = S * 32 * 2 * 4 * (int)sizeof(double);
       ensure_smem((const void*)sv::k_dense<double, S, R>, smem, h->device);
-      sv::k_dense<double, S, R><<<(unsigned)((op.ng + 8 * R - 1) / (8 * R)), 256, smem, s>>>(op.Qd, op.ng, op.ld, Vt,
-                                                                                           Tout, active);
+      launch_on(sv::k_dense<double, S, R>, (int)((op.ng + 8 * R - 1) / (8 * R)), 256, smem, s, beside, op.Qd, op.ng, op.ld,
+                Vt, Tout, active, S);
       h->launched("k_dense<f64>");
       return;
     }
@@ -616,10 +642,11 @@ static void dense64(cbx_handle* h, const sv::OpView<double>& op, const double* X
 
 // FP32 dense block product Tout = Qd Vt^T from the gathered operand w.Vt (the
 // tcgen05 3xTF32 kernel for 16, 32 or 64 columns, the HBM-streaming GEMV for
-// one, the CUDA-core kernel otherwise); returns the number of K-split partials.
+// one, the CUDA-core kernel otherwise); returns the number of K-split partials.  beside: the
+// launch before lets the product start with it (release_successor).
 template <typename T, int S>
 int product_from_vt(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const int* active,
-                    int ncols = S) {
+                    int ncols = S, bool beside = false) {
   cudaStream_t s = h->stream;
   int tsplit = 1;
   cbx_handle::ProfRec pr{};
@@ -637,7 +664,7 @@ int product_from_vt(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, 
   } else if ((S == 16 || S == 32 || S == 64 || S == 128) && use_dense_tc()) {
     tsplit = dense_tc_ksplit(op.ng, op.ld, h->num_sms);
     dense_tc(h, reinterpret_cast<const float*>(op.Qd), op.ng, op.ld, reinterpret_cast<const float*>(w.Vt.p), S,
-             tsplit, reinterpret_cast<float*>(w.Tout.p), active, ncols);
+             tsplit, reinterpret_cast<float*>(w.Tout.p), active, ncols, beside);
   } else if constexpr (S == 128) {
     throw Error(CBX_ERR_UNSUPPORTED, "the 128-wide block needs the tensor-core product (CBX_DENSE_TC=1)");
   } else if (S == 1) {
@@ -676,36 +703,6 @@ int product_from_vt(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, 
   return tsplit;
 }
 
-// Work beside the handle's stream, on a side stream between two events.  Inside a capture, and
-// with side == the handle's stream, it stays on that stream: with graphs that had branches,
-// batches of 32 and more problems on 16 host threads crashed in the driver, in an event's
-// record or in a context's synchronization; with unbranched graphs they do not.
-class Branch {
- public:
-  Branch(cbx_handle* h, cudaStream_t side, cudaEvent_t done)
-      : h_(h), side_(h->capturing ? h->stream : side), done_(done) {}
-  // the stream that takes the branch's launches, up to end()
-  cudaStream_t begin() {
-    if (side_ != h_->stream) {
-      CBX_CUDA(cudaEventRecord(h_->ev_fork, h_->stream));
-      CBX_CUDA(cudaStreamWaitEvent(side_, h_->ev_fork, 0));
-    }
-    return side_;
-  }
-  void end() {
-    if (side_ != h_->stream) CBX_CUDA(cudaEventRecord(done_, side_));
-  }
-  // later launches of the handle's stream follow the branch too
-  void join() {
-    if (side_ != h_->stream) CBX_CUDA(cudaStreamWaitEvent(h_->stream, done_, 0));
-  }
-
- private:
-  cbx_handle* h_;
-  cudaStream_t side_;
-  cudaEvent_t done_;
-};
-
 // Y = use_D * W'W X + lam [0; Qinv X_u] for an S-wide interleaved block whose
 // first ncols columns are populated (the rest are zero or ignored); optional
 // pq partials sum_i P[i] Y[i] for the PCG step.
@@ -722,22 +719,23 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   // qshift * (column sums) back; the FP64 product uses the block itself.
   const double* colsum = op.Qd ? w.colsum.p : nullptr;
   const double tshift = h->mme->qshift;
-  // the fixed rows' segments run on the second stream beside the block product (one
-  // stream under a launch trace, whose attribution assumes one)
+  // The fixed rows' segments (and, in FP32, the gathered vectors' sums) run beside the block
+  // product, which starts with them once its operand is complete: on the same stream, so that the
+  // captured graph has no branches.  With side streams as branches of the graph, batches of 32
+  // and more problems on 16 host threads crashed in the driver (an event's record, a context's
+  // synchronization).  One after the other under a launch trace or a profile.
   const Mme& mm = *h->mme;
-  const bool segs = use_D && mm.nseg > 0;
-  Branch side(h, h->trace_on || !op.Qd ? s : h->stream2, h->ev_join);
-  const cudaStream_t s2 = side.begin();
-  auto segments = [&]() {
-    if (!segs) return;
-    sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, s2>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p,
-                                                    active, ncp);
+  const bool segs = use_D && mm.nseg > 0, overlap = !h->trace_on && !h->prof_on;
+  auto segments = [&](cudaStream_t st) {
+    if (!segs) return false;
+    sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, st>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p, active,
+                                                    ncp);
     h->launched(sizeof(T) == 4 ? "k_fix_seg<f32>" : "k_fix_seg<f64>");
+    return overlap;
   };
-  segments();
   if (!op.Qd) {
+    segments(s);
   } else if constexpr (sizeof(T) == 8) {
-    side.end();
     ff = ff && h->mme->Qlo32.p && h->mme->Qd32.p;
     if (!ff) colsum = nullptr;
     cbx_handle::ProfRec pr{};
@@ -750,19 +748,26 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       CBX_CUDA(cudaMemsetAsync(w.Tout.p, 0, (size_t)op.ng * S * sizeof(double), s));
       CBX_CUDA(cudaMemsetAsync(w.colsum.p, 0, S * sizeof(double), s));
     }
-    dense64<S>(h, op, X, ncols, w.Vt.p, w.Tout.p, active, ff, w.colsum.p);
+    dense64<S>(h, op, X, ncols, w.Vt.p, w.Tout.p, active, ff, w.colsum.p, [&] { return segments(s); });
     if (h->prof_on) {
       CBX_CUDA(cudaEventRecord(pr.b, s));
       pr.bucket = 1;
       pr.bytes = 8.0 * (double)op.ng * op.ld + 8.0 * ncols * ((double)op.ld + (double)op.ng);
       h->prof.push_back(pr);
     }
-    side.join();
   } else {
     // FP32: gather the dense-block rows, their FP64 column sums, the product
     // (the populated 32-column groups only)
     const bool split = matvec_split(h, op);
+    // opt-in: all of the sparse part on the second stream beside the product (inside a capture on
+    // the same stream)
+    cudaStream_t s2 = h->capturing ? s : h->stream2;
     if (split) {
+      if (s2 != s) {
+        CBX_CUDA(cudaEventRecord(h->ev_fork, s));
+        CBX_CUDA(cudaStreamWaitEvent(s2, h->ev_fork, 0));
+      }
+      segments(s2);
       // the rest of the sparse part beside the product too: k_spmv without the block
       // term writes every row and its pq partials
       sv::OpView<T> ops = op;
@@ -770,8 +775,8 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       sv::k_spmv<T, S><<<w.nblk_spmv, sv::NT, 0, s2>>>(ops, X, nullptr, 1, nullptr, 0.0, mm.fix_seg_ptr.p,
                                                         w.seg_part.p, (T)lam, use_D, Y, P, pq_part, active, ncp);
       h->launched("k_spmv<f32>");
+      if (s2 != s) CBX_CUDA(cudaEventRecord(h->ev_join, s2));
     }
-    side.end();
     if constexpr (S >= 32)
       sv::k_gather_tile<T, S><<<(unsigned)((op.ld + 31) / 32), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld, op.gmap,
                                                                             active, ncp);
@@ -779,16 +784,13 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
       sv::k_gather_t<T, S><<<grid_for(ncp * op.ld, 256, 16 * h->num_sms), 256, 0, s>>>(X, w.Vt.p, op.p, op.ng, op.ld,
                                                                                    op.gmap, active, S, ncp);
     h->launched("k_gather_t<f32>");
-    // the gathered vectors' sums, which only the last kernel reads, on the third
-    Branch sums(h, h->trace_on ? s : h->stream3, h->ev_join3);
-    const cudaStream_t s3 = sums.begin();
-    sv::k_colsum_vt<T><<<ncp, 1024, 0, s3>>>(w.Vt.p, op.ld, op.ng, w.colsum.p);
+    // the segments and the gathered vectors' sums, which only the last kernel reads
+    const bool with_segs = !split && segments(s);
+    launch_on(sv::k_colsum_vt<T>, ncp, 1024, 0, s, with_segs, w.Vt.p, op.ld, op.ng, w.colsum.p);
     h->launched("k_colsum_vt<f32>");
-    sums.end();
-    tsplit = product_from_vt<T, S>(h, op, w, active, ncols);
-    sums.join();
-    side.join();
+    tsplit = product_from_vt<T, S>(h, op, w, active, ncols, overlap);
     if (split) {
+      if (s2 != s) CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
       // the block term of the genotyped rows, once both are done
       sv::k_dense_add<T, S><<<w.nblk_dadd, sv::NT, 0, s>>>(op, w.Tout.p, tsplit, colsum, tshift, (T)lam, Y, P,
                                                            pq_part ? pq_part + (size_t)w.nblk_spmv * S : nullptr,
@@ -801,22 +803,6 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
                                                   w.seg_part.p,
                                                   (T)lam, use_D, Y, P, pq_part, active, ncp);
   h->launched(sizeof(T) == 4 ? "k_spmv<f32>" : "k_spmv<f64>");
-}
-
-// A launch that may be set up while its predecessor on the stream still runs; the kernel
-// begins with wait_predecessor.
-template <typename... KArgs, typename... Args>
-void launch_next(void (*kern)(KArgs...), int grid, int block, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  CBX_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
 }
 
 // Multi-RHS PCG in precision T on interleaved vectors; X receives the solution

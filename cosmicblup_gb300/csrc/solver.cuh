@@ -76,6 +76,13 @@ __device__ __forceinline__ double dot16(const double2& a, const double2& b) {
 __device__ __forceinline__ void wait_predecessor() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// The small sums beside a block product (k_fix_seg, k_colsum_vt) let the next kernel of the
+// stream start with them.  That one needs nothing of theirs, only what was complete before they
+// began, and waits for them at its end (wait_predecessor), so that whatever follows it normally
+// finds them done.  One stream and no branches.
+__device__ __forceinline__ void release_successor() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // Vt[c * ld + k] = X[(p + gmap[k]) * xs + c] for k < ng, 0 for ng <= k < ld
 // (S columns of a block whose rows are xs apart; xs = S for the whole block).
@@ -123,7 +130,10 @@ template <typename T, int S, int RPW>
 __global__ void __launch_bounds__(256) k_dense(const T* __restrict__ Qd, int64_t ng, int64_t ld,
                                                const T* __restrict__ Vt, T* __restrict__ Tout,
                                                const int* __restrict__ active, int os = S) {
-  if (active && *active == 0) return;
+  if (active && *active == 0) {
+    wait_predecessor();
+    return;
+  }
   using V = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::n;
   constexpr int KT = 32 * VEC * 4;
@@ -179,6 +189,7 @@ __global__ void __launch_bounds__(256) k_dense(const T* __restrict__ Qd, int64_t
       for (int c = 0; c < S; ++c) Tout[(row0 + r) * os + c] = acc[r][c];
     }
   }
+  wait_predecessor();
 }
 
 // Single right-hand side: Tout[i] = sum_k Qd[i * ld + k] v[k].  A pure HBM
@@ -188,7 +199,10 @@ template <typename T, int RPW, int U>
 __global__ void __launch_bounds__(256) k_gemv(const T* __restrict__ Qd, int64_t ng, int64_t ld,
                                               const T* __restrict__ v, T* __restrict__ Tout,
                                               const int* __restrict__ active, int os = 1) {
-  if (active && *active == 0) return;
+  if (active && *active == 0) {
+    wait_predecessor();
+    return;
+  }
   using V = typename Vec16<T>::type;
   constexpr int VEC = Vec16<T>::n;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -230,6 +244,7 @@ __global__ void __launch_bounds__(256) k_gemv(const T* __restrict__ Qd, int64_t 
     for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
     if (lane == 0 && row0 + r < ng) Tout[(row0 + r) * os] = t;
   }
+  wait_predecessor();
 }
 
 // ---------------------------------------------------------------------------
@@ -332,6 +347,7 @@ static __global__ void __launch_bounds__(256) k_colsum_x(const double* __restric
 template <typename T>
 __global__ void __launch_bounds__(1024) k_colsum_vt(const T* __restrict__ Vt, int64_t ld, int64_t ng,
                                                     double* __restrict__ out) {
+  release_successor();
   __shared__ double red[1024];
   const int c = blockIdx.x, tid = threadIdx.x;
   // per-thread sums compensated in the vectors' own precision (no FP64
@@ -351,6 +367,7 @@ __global__ void __launch_bounds__(1024) k_colsum_vt(const T* __restrict__ Vt, in
     __syncthreads();
   }
   if (tid == 0) out[c] = red[0];
+  wait_predecessor();
 }
 
 // Tout[i * S + c] = sum_k Qd[i][k] V[c][k] in float-float; Qh / Ql are the
@@ -657,6 +674,7 @@ __global__ void __launch_bounds__(NT) k_fix_seg(OpView<T> op, const int32_t* __r
                                                 const int32_t* __restrict__ seg_lo, const int32_t* __restrict__ seg_hi,
                                                 const T* __restrict__ X, T* __restrict__ seg_part,
                                                 const int* __restrict__ active, int ncp = S) {
+  release_successor();
   if (active && *active == 0) return;
   __shared__ T redT[NT];
   const int sg = blockIdx.x;
