@@ -441,8 +441,9 @@ __global__ void __launch_bounds__(256) k_geno_vdig(const long long* __restrict__
 
 // Z^T v: a warp takes 32 SNP rows and a chunk of samples, 256 at a time: each lane loads
 // 64 samples (16 bytes) of four rows, and 16 MMAs a row pair use them.  acc[row] += sum of
-// k V (64-bit atomics).  Bound by mma.sync, at its legacy rate of about 280 multiply-adds a clock
-// and SM: at n = 20,000, m = 50,000 0.10 ms (0.20 ms as two integer multiply-adds a code).
+// k V (64-bit atomics).  Bound by the latency of the loads at its few warps, with mma.sync busy a
+// quarter of the time (profiled): at n = 20,000, m = 50,000 0.097 ms (0.20 ms as two integer
+// multiply-adds a code).
 constexpr int ZT_ROWS = 32 * (ZT_THREADS / 32);
 __global__ void __launch_bounds__(ZT_THREADS) k_geno_zt(const uint8_t* __restrict__ bed, int64_t pitch, int64_t m,
                                                        int segs_per_cta, const uint2* __restrict__ B,
@@ -515,8 +516,9 @@ __global__ void __launch_bounds__(256) k_geno_zdig(const long long* __restrict__
 // at a time: lane (g, t) holds the words of SNPs 2t, 2t + 1, 2t + 8, 2t + 9, whose halves
 // pair up to samples 0-7 and 8-15 of two SNPs; MMA i multiplies samples i and i + 8 of
 // eight words.  A second MMA adds the term of codes with both bits set.  acc[i] += the
-// sum (64-bit atomics).  Bound by mma.sync's rate: at n = 20,000, m = 50,000
-// 0.20 ms (0.52 ms as integer multiply-adds).
+// sum (64-bit atomics).  Bound by the issue of the decoding, four instructions an MMA, and the
+// MMAs' latency (their pipe is busy a quarter of the time): at n = 20,000, m = 50,000 0.20 ms
+// (0.52 ms as integer multiply-adds).
 constexpr int Z_SAMPLES = 256 * (Z_THREADS / 32);
 __global__ void __launch_bounds__(Z_THREADS) k_geno_z(const uint8_t* __restrict__ bed, int64_t pitch, int64_t m,
                                                      int blks_per_cta, const uint4* __restrict__ B,
