@@ -723,9 +723,10 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   // product, which starts with them once its operand is complete: on the same stream, so that the
   // captured graph has no branches.  With side streams as branches of the graph, batches of 32
   // and more problems on 16 host threads crashed in the driver (an event's record, a context's
-  // synchronization).  One after the other under a launch trace or a profile.
+  // synchronization).  One after the other under a launch trace; a profile, whose events lie
+  // between, times the FP32 product by itself.
   const Mme& mm = *h->mme;
-  const bool segs = use_D && mm.nseg > 0, overlap = !h->trace_on && !h->prof_on;
+  const bool segs = use_D && mm.nseg > 0, overlap = !h->trace_on;
   auto segments = [&](cudaStream_t st) {
     if (!segs) return false;
     sv::k_fix_seg<T, S><<<mm.nseg, sv::NT, 0, st>>>(op, mm.seg_row.p, mm.seg_lo.p, mm.seg_hi.p, X, w.seg_part.p, active,
@@ -788,7 +789,7 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
     const bool with_segs = !split && segments(s);
     launch_on(sv::k_colsum_vt<T>, ncp, 1024, 0, s, with_segs, w.Vt.p, op.ld, op.ng, w.colsum.p);
     h->launched("k_colsum_vt<f32>");
-    tsplit = product_from_vt<T, S>(h, op, w, active, ncols, overlap);
+    tsplit = product_from_vt<T, S>(h, op, w, active, ncols, overlap && !h->prof_on);
     if (split) {
       if (s2 != s) CBX_CUDA(cudaStreamWaitEvent(s, h->ev_join, 0));
       // the block term of the genotyped rows, once both are done
