@@ -14,7 +14,7 @@
 // product is rounded to FP64 once.  The dropped pairs weigh below 2^-58 of the product
 // of the two row maxima per term, less than an FP64 multiply-add's rounding.
 //
-// Factorization.  Right-looking in blocks of 32 inside outer panels of 128 to 512
+// Factorization.  Right-looking in blocks of 32 inside outer panels of 256 or 512
 // columns, in a row-major lower triangle W.  Step k (k_panel) factors the 32 x 32
 // pivot block by FP64 elimination, giving X = L_kk^-1, and substitutes L_ik L_kk' = S_ik for
 // the rows below; for the inverse also row k of M = L^-1, L_kk M_kj = R_kj for j < k, where
@@ -26,7 +26,7 @@
 // Bound: below n = 3,000 the chain of 32-wide steps (a pivot factor and a K = 32 update,
 // 26 us); above it the digit MMAs (36 per FP64 multiply-add) and the L2 reads that feed
 // them (96 KB a step of 2,304 tensor clocks).  Measured, inverse with its factor, against
-// cuSOLVER potrf + potri: n = 500 0.63 ms (4.2), 2,000 2.8 (31), 8,000 35 (1,194), 20,000
+// cuSOLVER potrf + potri: n = 500 0.61 ms (4.2), 2,000 2.7 (31), 8,000 35 (1,194), 20,000
 // 322 (about 11,000).  The product at n = 2,000: 0.60 ms (15.3 by cuBLAS DGEMM).  128 x 64
 // tiles: eight classes of 64 columns fill the 512 TMEM columns, and a narrower tile reads
 // the A digits more often.
@@ -616,7 +616,7 @@ struct Panel {
 // first, and the condition of the pair enters twice.  The groups' rows are forward
 // substitutions by the same pairs and not products with X, which lose the root of L_kk's
 // condition where two adjacent rows are near-duplicates.  Measured with the pair's inverse
-// and X before, both this way now: factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81 both; at
+// and X before, both this way now (panels of 128): factor at n = 2,000 2.59 ms, now 2.47, inverse 2.81 both; at
 // 8,000 18.3, now 18.1, and 34.4, now 34.8 (a substitution issues 92 FP64 instructions a warp and group,
 // the product 80; the digits took 16 on half of the lanes, now 8).  L L' - A at n = 96 with adjacent
 // rows 1e-3 apart: 0.01 of 4 n u sqrt(A_ii A_jj), 1e5 times it before, when rows 1e-4 apart were
@@ -1118,7 +1118,11 @@ bool fx64_cholesky(cbx_handle* h, const double* A, int64_t n, bool inverse, doub
   cudaStream_t s = h->stream;
   fx::Scratch& S = fx::scratch(h);
   const int64_t np = (n + 127) / 128 * 128;
-  const int rt = (int)(np / 128), B0 = n < 3000 ? 128 : n < 10000 ? 256 : 512;
+  // panel width, inverse / factor in ms: n = 1,000 1.25 / 1.19 with 128, 1.22 / 1.16 with 256;
+  // 2,000 2.82 / 2.47, 2.67 / 2.35 (512: 2.88 / 2.36); 8,000 38.3 / 19.9, 34.8 / 18.1 (512: 35.4 /
+  // 18.0); 10,000 with 256 61.5 / 29.7, with 512 61.2 / 29.4 (1,024: 67.0 / 32.3); 14,000 132 / 61.9,
+  // 129 / 59.8.  A wider panel updates more by K = 32 inside it, a narrower one more often from outside
+  const int rt = (int)(np / 128), B0 = n < 10000 ? 256 : 512;
   const int B = (int)std::min<int64_t>(B0, np);
   fx::at_least(S.W, (size_t)np * np);
   fx::at_least(S.P, (size_t)np * B);

@@ -656,8 +656,9 @@ static int choose_parts(int64_t ntiles, int np, int sms) {
 
 // G is copied to pinned host memory behind the tiles, in groups of whole rounds of tiles:
 // the row blocks that a group completes are, with the entries below them, two rectangles.
-// From two rounds a group on: at n = 12,000 (59 rounds) the copy of 1.15 GB took 6 ms after
-// 42 ms of kernels, eight groups leave 0.8 of it.
+// From two rounds a group on.  The call at n = 12,000, m = 40,001 (59 rounds): 48.1 ms with one copy
+// after the tiles, 43.8 in four groups, 43.0 in eight, 42.9 in 16; at n = 6,000, m = 20,000 (14
+// rounds) 7.3, 6.4, 6.3 and 6.4.
 constexpr int COPY_GROUPS = 8;
 
 static bool is_pinned(const void* p) {
