@@ -722,7 +722,7 @@ void matvec(cbx_handle* h, const sv::OpView<T>& op, Workspace<T, S>& w, const T*
   // The fixed rows' segments (and, in FP32, the gathered vectors' sums) run beside the block
   // product, which starts with them once its operand is complete: on the same stream, so that the
   // captured graph has no branches.  With side streams as branches of the graph, batches of 32
-  // and more problems on 16 host threads crashed in the driver (an event's record, a context's
+  // and more problems on 16 host threads crashed in the CUDA driver (an event's record, a context's
   // synchronization).  One after the other under a launch trace; a profile, whose events lie
   // between, times the FP32 product by itself.
   const Mme& mm = *h->mme;
